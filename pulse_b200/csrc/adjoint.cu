@@ -34,6 +34,7 @@
 #include <atomic>
 
 #include "adjoint.h"
+#include "pt_wide.cuh"
 #include "wf_common.cuh"
 
 namespace pt {
@@ -313,6 +314,7 @@ cudaError_t launch_backward(const DevScene& S, const TraceCfg& tc, const PathCfg
   const size_t smem_t = (size_t)trace_smem_words(tc) * kAdjBlock * 4;
   const int light_blocks = sms * 16;
   const int trace_grid = sms * (int)(trace_blocks ? trace_blocks : kDefaultTraceBlocks);
+  const bool wide = wide_allowed(tc, S);
   uint32_t n = 0;
   e = cudaMemsetAsync(B.counts, 0, 8 * sizeof(uint32_t), st);
   if (e != cudaSuccess) return e;
@@ -321,9 +323,10 @@ cudaError_t launch_backward(const DevScene& S, const TraceCfg& tc, const PathCfg
   int qi = 0;
   for (uint32_t seg = 0; seg < pc.max_depth; ++seg) {
     if ((e = wf_reset_step(B, qi ^ 1, st)) != cudaSuccess) return e;
-    if ((e = wf_extend_step(tc, B, qi, trace_blocks, ctr, st)) != cudaSuccess) return e;
+    if ((e = wf_extend_step(tc, B, qi, trace_blocks, wide, ctr, st)) != cudaSuccess) return e;
     k_adj_shade<<<light_blocks, kAdjBlock, smem_g, st>>>(S, pc, B, rec, dimg, qi, grads, n_mat);
-    k_adj_shadow<<<trace_grid, kAdjBlock, smem_t, st>>>(S, tc, B, rec, ctr);
+    if (wide) wide_adj_shadow(tc, S, B, rec, kRec, kVisible, trace_blocks, ctr, st);
+    else k_adj_shadow<<<trace_grid, kAdjBlock, smem_t, st>>>(S, tc, B, rec, ctr);
     k_adj_resolve<<<light_blocks, kAdjBlock, smem_g, st>>>(S, pc, B, rec, dimg, qi, grads, n_mat);
     n += 5;
     qi ^= 1;

@@ -21,6 +21,8 @@
 #include "wavefront.h"
 #include "adjoint.h"
 #include "scene_prep.cuh"
+#include "pt_wide.cuh"
+#include "wide.cuh"
 
 namespace pt {
 namespace {
@@ -103,6 +105,12 @@ struct MeshRec {
   uint32_t id = 0, ntris = 0, node_count = 0, levels = 1;
   bool alive = false;
   DevBuf prims, tdata, nodes, idx;
+  // The eight-wide tree (wide.cuh): nodes, leaf node of every slot, and what a
+  // collapse reported.
+  DevBuf wide, leaf_of;
+  bool wide_ok = false;
+  uint32_t wide_count = 0, wide_root = 0, wide_levels = 0;
+  float wide_slack = 0.0f;
 };
 
 struct PulseScene {
@@ -114,6 +122,11 @@ struct PulseScene {
       materials, strength_cdf, tri_cdfs, mesh_areas, light_indices;
   // Derived layouts.
   DevBuf inst_light, tri_bvh;
+  DevBuf wide_blas, leaf_of;                      // of every mesh, concatenated
+  DevBuf wide_tlas, wide_thead, inst_wide;  // of the instances (pt_wide.cuh)
+  DevBuf wide_queue;                              // scratch of the instance tree's collapse
+  std::vector<uint32_t> mesh_wide;                // per mesh id: first wide node in wide_blas
+  uint64_t wide_nodes = 0;                        // rows of wide_blas
   bool tri_bvh_current = false;  // tri_bvh gathered from the current primitives and triangle_indices
   pt::DevScene dev{};
   // Scene-preparation path.
@@ -150,7 +163,7 @@ struct PulseScene {
   // which then becomes the back set was queued before it.
   struct FrameSet {
     DevBuf tlas_nodes, instance_indices, instances, strength_cdf, tri_cdfs, mesh_areas, light_indices, inst_light,
-        inst_bounds, prep_ii, prep_lights, tlas_min, tlas_max, tlas_cent, tlas_meta;
+        inst_bounds, prep_ii, prep_lights, tlas_min, tlas_max, tlas_cent, tlas_meta, wide_tlas, wide_thead, inst_wide;
     uint32_t* meta_host = nullptr;
     uint32_t* meta_mapped = nullptr;
   };
@@ -182,6 +195,9 @@ struct PulseScene {
     std::swap(tlas_max, b.tlas_max);
     std::swap(tlas_cent, b.tlas_cent);
     std::swap(tlas_meta, b.tlas_meta);
+    std::swap(wide_tlas, b.wide_tlas);
+    std::swap(wide_thead, b.wide_thead);
+    std::swap(inst_wide, b.inst_wide);
     std::swap(meta_host, b.meta_host);
     std::swap(meta_mapped, b.meta_mapped);
   }
@@ -189,7 +205,7 @@ struct PulseScene {
     FrameSet& b = back;
     for (DevBuf* x : {&b.tlas_nodes, &b.instance_indices, &b.instances, &b.strength_cdf, &b.tri_cdfs, &b.mesh_areas,
                       &b.light_indices, &b.inst_light, &b.inst_bounds, &b.prep_ii, &b.prep_lights, &b.tlas_min,
-                      &b.tlas_max, &b.tlas_cent, &b.tlas_meta})
+                      &b.tlas_max, &b.tlas_cent, &b.tlas_meta, &b.wide_tlas, &b.wide_thead, &b.inst_wide})
       free_buf(*x);
     if (b.meta_host) cudaFreeHost(b.meta_host);
     b.meta_host = b.meta_mapped = nullptr;
@@ -204,16 +220,20 @@ struct PulseScene {
   }
   void free_all() {
     for (DevBuf* b : bind_group()) free_buf(*b);
-    free_buf(inst_light);
-    free_buf(tri_bvh);
+    for (DevBuf* b : {&inst_light, &tri_bvh, &wide_blas, &leaf_of, &wide_tlas, &wide_thead, &inst_wide})
+      free_buf(*b);
+    dev.wide = 0u;
     tri_bvh_current = false;
     free_buf(inst_bounds);
     free_back();
     ready = false;
   }
   void free_meshes() {
-    for (MeshRec& m : meshes) { free_buf(m.prims); free_buf(m.tdata); free_buf(m.nodes); free_buf(m.idx); }
+    for (MeshRec& m : meshes) free_mesh(m);
     meshes.clear();
+  }
+  static void free_mesh(MeshRec& m) {
+    for (DevBuf* x : {&m.prims, &m.tdata, &m.nodes, &m.idx, &m.wide, &m.leaf_of}) free_buf(*x);
   }
   static void free_buf(DevBuf& b) {
     if (b.p) cudaFree(b.p);
@@ -418,7 +438,7 @@ pt::TraceCfg trace_cfg(const PulseRenderParams* p, const pt::DevScene& S) {
   pt::TraceCfg t;
   t.stack_depth = p->stack_depth;
   t.iter_cap = p->iter_cap;
-  pt::trace_stacks(t, S.tlas_levels, S.blas_levels);
+  pt::trace_stacks(t, S.tlas_levels, S.blas_levels, S.wide_stack, S.wide_top);
   t.eps_tri = p->eps_tri;
   t.eps_par = p->eps_par;
   t.quirks = p->quirks != 0;
@@ -610,7 +630,7 @@ int32_t pulse_scene_destroy(PulseScene* s) {
   s->free_meshes();
   s->bvh_scratch.release();
   for (DevBuf* x : {&s->tmp_a, &s->tmp_b, &s->tmp_c, &s->tmp_d, &s->prep_ii, &s->prep_lights, &s->prep_slot,
-                    &s->tlas_min, &s->tlas_max, &s->tlas_cent, &s->tlas_meta})
+                    &s->tlas_min, &s->tlas_max, &s->tlas_cent, &s->tlas_meta, &s->wide_queue})
     PulseScene::free_buf(*x);
   if (s->meta_host) cudaFreeHost(s->meta_host);
   if (s->upd_stream) cudaStreamDestroy(s->upd_stream);
@@ -618,6 +638,10 @@ int32_t pulse_scene_destroy(PulseScene* s) {
     if (ev) cudaEventDestroy(ev);
   delete s;
   return PULSE_OK;
+}
+
+static void set_wide_tlas(PulseScene* s) {
+  s->dev.wide_tlas = (const uint4*)s->wide_tlas.p;
 }
 
 // Derived layouts (tri_bvh per distinct mesh range, instance -> light map) and
@@ -634,7 +658,7 @@ static cudaError_t finalize_scene(PulseScene* s, const std::vector<std::array<ui
     for (const auto& r : ranges) {  // {triangle_offset, index_offset, count}
       if (e != cudaSuccess) break;
       e = pt::launch_gather_tri_bvh((const float4*)s->primitives.p, (const uint32_t*)s->triangle_indices.p,
-                                    (float4*)s->tri_bvh.p, r[0], r[1], r[2], st);
+                                    (const uint32_t*)s->leaf_of.p, (float4*)s->tri_bvh.p, r[0], r[1], r[2], st);
     }
     if (e != cudaSuccess) return e;
     s->tri_bvh_current = true;
@@ -658,6 +682,9 @@ static cudaError_t finalize_scene(PulseScene* s, const std::vector<std::array<ui
   d.inst_light = (const int32_t*)s->inst_light.p;
   d.instance_count = c.instance_count;
   d.light_count = c.light_count;
+  d.wide_blas = (const uint4*)s->wide_blas.p;
+  set_wide_tlas(s);
+  d.inst_wide = (const float4*)s->inst_wide.p;
   return cudaSuccess;
 }
 
@@ -822,6 +849,91 @@ int32_t pulse_build_tlas(PulseCtx* ctx, const float* bounds9, uint32_t n, const 
 }
 
 // ------------------------------------------------- scene-preparation path
+// The eight-wide tree of a mesh whose nodes and triangles are on the device.
+static cudaError_t collapse_mesh(MeshRec& m, cudaStream_t st) {
+  const size_t cap = wide::capacity(m.node_count);
+  DevBuf out, queue, head;
+  uint32_t h[wide::kHeadWords] = {};
+  cudaError_t e = ensure(m.leaf_of, (size_t)m.ntris * 4);
+  if (e == cudaSuccess) e = ensure(out, cap * pt::kWideNodeWords * 4);
+  if (e == cudaSuccess) e = ensure(queue, cap * 4);
+  if (e == cudaSuccess) e = ensure(head, sizeof(h));
+  if (e == cudaSuccess) e = cudaMemsetAsync(head.p, 0, sizeof(h), st);
+  if (e == cudaSuccess)
+    e = wide::collapse((const float4*)m.nodes.p, m.node_count, (uint4*)out.p, (uint32_t*)m.leaf_of.p,
+                       (uint32_t*)queue.p, (uint32_t*)head.p, st);
+  if (e == cudaSuccess) e = wide::extents((const float4*)m.prims.p, m.ntris, (uint32_t*)head.p, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h, head.p, sizeof(h), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess && !h[wide::kBad] && h[wide::kCount] <= cap) {
+    m.wide_count = h[wide::kCount];
+    m.wide_root = h[wide::kRoot];
+    m.wide_levels = h[wide::kLevels];
+    float area;
+    std::memcpy(&area, &h[wide::kArea], 4);
+    m.wide_slack = wide::slack(area);
+    const size_t bytes = (size_t)m.wide_count * pt::kWideNodeWords * 4;
+    e = ensure(m.wide, bytes);
+    if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(m.wide.p, out.p, bytes, cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    m.wide_ok = e == cudaSuccess;
+  }
+  for (DevBuf* x : {&out, &queue, &head}) PulseScene::free_buf(*x);
+  return e;
+}
+
+// Whether an instance's transform is affine and far enough from singular for the
+// wide traversal (its inverse's entries below 1e9): a missed mesh then converts to an
+// infinite distance, which replaces no record with the reference's quirks either.
+static bool wide_transform(const float* m) {
+  if (m[3] != 0.0f || m[7] != 0.0f || m[11] != 0.0f || m[15] != 1.0f) return false;
+  const double a = m[0], b = m[4], c = m[8], d = m[1], e = m[5], f = m[9], g = m[2], h = m[6], i = m[10];
+  const double cof[9] = {e * i - f * h, c * h - b * i, b * f - c * e, f * g - d * i, a * i - c * g,
+                         c * d - a * f, d * h - e * g, b * g - a * h, a * e - b * d};
+  const double det = a * cof[0] + b * cof[3] + c * cof[6];
+  double most = 0.0;
+  for (double x : cof) most = std::max(most, std::fabs(x));
+  for (int k = 0; k < 16; ++k)
+    if (!(std::fabs(m[k]) <= 1e9f)) return false;
+  return most <= 1e9 * std::fabs(det) && det != 0.0;
+}
+
+// What the collapse of the instance tree reported.
+struct WideTree {
+  bool ok = false;
+  uint32_t levels = 0, count = 0;
+  void read(const uint32_t* head) {
+    ok = !head[wide::kBad];
+    levels = head[wide::kLevels];
+    count = head[wide::kCount];
+  }
+};
+
+// After the instances and their tree are in place: whether the scene's rays may
+// take the wide traversal.
+static void decide_wide(PulseScene* s, const std::vector<prep::InstanceIn>& ii, const WideTree& tree) {
+  bool ok = tree.ok && !ii.empty();
+  float slack = pt::kLeastSlack;
+  uint32_t levels = 0;
+  for (const MeshRec& m : s->meshes)
+    if (m.alive) {
+      ok = ok && m.wide_ok;
+      slack = std::max(slack, m.wide_slack);
+      levels = std::max(levels, m.wide_levels);
+    }
+  // TLAS: every child hit, up to a fixed size (a ray that needs more is traced by
+  // the binary traversal); BLAS: a visit pushes the rest of its group and, with
+  // leaves hit, the interior children hit
+  const uint32_t top = std::min(7 * tree.levels + 1, tree.levels <= 3 ? pt::kTopStack : pt::kTopStackDeep);
+  s->dev.wide_top = top;
+  s->dev.wide_stack = top + levels + 1;
+  ok = ok && s->dev.wide_stack <= 96 && std::max((size_t)tree.count, ii.size()) < (1u << pt::kTopIndexBits) &&
+       s->wide_nodes < (1ull << pt::kWideIndexBits) && s->counts.triangle_index_count < (1u << pt::kWideFirstBits);
+  for (size_t i = 0; ok && i < ii.size(); ++i) ok = wide_transform(ii[i].object_world);
+  s->dev.wide_slack = slack;
+  s->dev.wide = ok ? 1u : 0u;
+}
+
 int32_t pulse_mesh_upload(PulseScene* s, const float* pos, const float* nrm, const float* uv, uint32_t nverts,
                           const uint32_t* idx, uint32_t nidx, const PulseBvhParams* params, uint32_t* mesh_id) {
   if (!s || !pos || !nrm || !uv || !idx || !params || !mesh_id) return PULSE_ERR_INVALID_ARG;
@@ -874,8 +986,13 @@ int32_t pulse_mesh_upload(PulseScene* s, const float* pos, const float* nrm, con
       ctx->stats.last_build_ms = ms;
   }
   for (DevBuf* x : {&dpos, &dnrm, &duv, &didx, &pmin, &pmax, &cent}) PulseScene::free_buf(*x);
+  if (rc == PULSE_OK) {
+    e = collapse_mesh(m, st);
+    if (e != cudaSuccess) rc = cuda_err(ctx, e, "mesh upload: eight-wide tree");
+    else ctx->stats.kernel_launches += 2;
+  }
   if (rc != PULSE_OK) {
-    for (DevBuf* x : {&m.prims, &m.tdata, &m.nodes, &m.idx}) PulseScene::free_buf(*x);
+    PulseScene::free_mesh(m);
     return rc;
   }
   m.alive = true;
@@ -891,7 +1008,7 @@ int32_t pulse_mesh_remove(PulseScene* s, uint32_t mesh_id) {
   quiesce(s->ctx);
   cudaStreamSynchronize(s->ctx->stream);
   MeshRec& m = s->meshes[mesh_id];
-  for (DevBuf* x : {&m.prims, &m.tdata, &m.nodes, &m.idx}) PulseScene::free_buf(*x);
+  PulseScene::free_mesh(m);
   m.alive = false;
   s->meshes_dirty = true;
   return PULSE_OK;
@@ -938,17 +1055,24 @@ static cudaError_t concat_meshes(PulseScene* s) {
   cudaStream_t st = s->ctx->stream;
   s->tri_bvh_current = false;
   uint64_t nt = 0, nn = 0;
+  uint64_t nw = 0;
   s->mesh_table.assign(s->meshes.size(), {~0u, 0u, ~0u, ~0u});
+  s->mesh_wide.assign(s->meshes.size(), 0u);
   for (const MeshRec& m : s->meshes) {
     if (!m.alive) continue;
     s->mesh_table[m.id] = {(uint32_t)nt, m.ntris, (uint32_t)nt, (uint32_t)nn};
+    s->mesh_wide[m.id] = (uint32_t)nw;
     nt += m.ntris;
     nn += m.node_count;
+    nw += m.wide_count;
   }
+  const size_t wide_bytes = pt::kWideNodeWords * 4;
   cudaError_t e = ensure(s->primitives, nt * 48);
   if (e == cudaSuccess) e = ensure(s->triangle_data, nt * 80);
   if (e == cudaSuccess) e = ensure(s->triangle_indices, nt * 4);
   if (e == cudaSuccess) e = ensure(s->blas_nodes, nn * 32);
+  if (e == cudaSuccess) e = ensure(s->wide_blas, nw * wide_bytes);
+  if (e == cudaSuccess) e = ensure(s->leaf_of, nt * 4);
   for (const MeshRec& m : s->meshes) {
     if (!m.alive || e != cudaSuccess) continue;
     const auto& t = s->mesh_table[m.id];
@@ -956,7 +1080,12 @@ static cudaError_t concat_meshes(PulseScene* s) {
     if (e == cudaSuccess) e = cudaMemcpyAsync((char*)s->triangle_data.p + (size_t)t[0] * 80, m.tdata.p, (size_t)m.ntris * 80, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync((char*)s->triangle_indices.p + (size_t)t[2] * 4, m.idx.p, (size_t)m.ntris * 4, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync((char*)s->blas_nodes.p + (size_t)t[3] * 32, m.nodes.p, (size_t)m.node_count * 32, cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync((char*)s->leaf_of.p + (size_t)t[2] * 4, m.leaf_of.p, (size_t)m.ntris * 4, cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess && m.wide_count)
+      e = wide::relocate((const uint32_t*)m.wide.p, m.wide_count, s->mesh_wide[m.id], t[2],
+                         (uint32_t*)s->wide_blas.p + (size_t)s->mesh_wide[m.id] * pt::kWideNodeWords, st);
   }
+  s->wide_nodes = nw;
   s->counts.primitive_count = (uint32_t)nt;
   s->counts.triangle_index_count = (uint32_t)nt;
   s->counts.blas_node_count = (uint32_t)nn;
@@ -964,16 +1093,33 @@ static cudaError_t concat_meshes(PulseScene* s) {
   return e;
 }
 
-// The TLAS over the n instance bounds in s->inst_bounds (src/scene/tlas.rs:29-65).
+// The TLAS over the n instance bounds in s->inst_bounds (src/scene/tlas.rs:29-65),
+// and its eight-wide form.
 // Up to bvh::direct_max() instances the build is one launch with no host
 // round trip: *pending is set and finish_tlas reads the node count and levels
 // once the caller has synchronized its stream.
-__global__ void k_meta_to_host(const uint32_t* __restrict__ meta, volatile uint32_t* host) {
+__global__ void k_meta_to_host(const uint32_t* __restrict__ meta, const uint32_t* __restrict__ head,
+                               volatile uint32_t* host) {
   if (threadIdx.x < 4) host[threadIdx.x] = meta[threadIdx.x];
+  else if (threadIdx.x < 4 + wide::kHeadWords) host[threadIdx.x] = head[threadIdx.x - 4];
+}
+
+// The eight-wide instance tree from the binary one of n instances just queued on st.
+static cudaError_t collapse_tlas(PulseScene* s, uint32_t n, const uint32_t* meta, cudaStream_t st) {
+  const uint32_t n_nodes = 2 * n - 1;
+  const size_t cap = wide::capacity(n_nodes);
+  cudaError_t e = ensure(s->wide_tlas, cap * pt::kWideNodeWords * 4);
+  if (e == cudaSuccess) e = ensure(s->wide_thead, wide::kHeadWords * 4);
+  if (e == cudaSuccess) e = ensure(s->wide_queue, cap * 4);
+  if (e != cudaSuccess) return e;
+  s->ctx->stats.kernel_launches += 1;
+  return wide::collapse_tlas((const float4*)s->tlas_nodes.p, n_nodes, meta, (const uint32_t*)s->instance_indices.p,
+                             (float4*)s->inst_wide.p, (uint4*)s->wide_tlas.p, (uint32_t*)s->wide_queue.p,
+                             (uint32_t*)s->wide_thead.p, st);
 }
 
 static int32_t rebuild_tlas(PulseScene* s, uint32_t n, const PulseBvhParams* tp, uint32_t* count, uint32_t* levels,
-                            bool* pending, cudaStream_t st) {
+                            WideTree* wt, bool* pending, cudaStream_t st) {
   PulseCtx* ctx = s->ctx;
   const uint64_t bvh_launches0 = s->bvh_scratch.launches;
   *count = 1;
@@ -1003,7 +1149,7 @@ static int32_t rebuild_tlas(PulseScene* s, uint32_t n, const PulseBvhParams* tp,
     bvh::Input in{(const float4*)pmin.p, (const float4*)pmax.p, (const float4*)cent.p, n};
     e = ensure(s->tlas_meta, 16);
     if (e == cudaSuccess && !s->meta_host) {
-      e = cudaHostAlloc((void**)&s->meta_host, 16, cudaHostAllocMapped);
+      e = cudaHostAlloc((void**)&s->meta_host, (4 + wide::kHeadWords) * 4, cudaHostAllocMapped);
       if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&s->meta_mapped, s->meta_host, 0);
       if (e != cudaSuccess && s->meta_host) {
         cudaFreeHost(s->meta_host);
@@ -1013,8 +1159,10 @@ static int32_t rebuild_tlas(PulseScene* s, uint32_t n, const PulseBvhParams* tp,
     if (e == cudaSuccess)
       e = bvh::build_direct(in, bvh::Params{tp->bins, tp->max_leaf, 1}, (uint32_t*)s->tlas_nodes.p,
                             (uint32_t*)s->instance_indices.p, (uint32_t*)s->tlas_meta.p, st);
+    if (e == cudaSuccess) e = collapse_tlas(s, n, (const uint32_t*)s->tlas_meta.p, st);
     if (e == cudaSuccess) {
-      k_meta_to_host<<<1, 32, 0, st>>>((const uint32_t*)s->tlas_meta.p, s->meta_mapped);
+      k_meta_to_host<<<1, 32, 0, st>>>((const uint32_t*)s->tlas_meta.p, (const uint32_t*)s->wide_thead.p,
+                                       s->meta_mapped);
       e = cudaGetLastError();
     }
     if (e != cudaSuccess) return cuda_err(ctx, e, "TLAS");
@@ -1032,21 +1180,30 @@ static int32_t rebuild_tlas(PulseScene* s, uint32_t n, const PulseBvhParams* tp,
     else if (r < 0) rc = set_err(ctx, PULSE_ERR_INVALID_ARG, why);
     else if (r > 0) rc = cuda_err(ctx, (cudaError_t)r, why.c_str());
   }
+  if (rc == PULSE_OK) {
+    uint32_t h[wide::kHeadWords] = {};
+    e = collapse_tlas(s, n, nullptr, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, s->wide_thead.p, sizeof(h), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) rc = cuda_err(ctx, e, "TLAS: eight-wide tree");
+    wt->read(h);
+  }
   ctx->stats.kernel_launches += 1 + (s->bvh_scratch.launches - bvh_launches0);
   return rc;
 }
 
 // Node count and levels of a TLAS built by rebuild_tlas with *pending set
 // (the context's stream must have been synchronized after the build).
-static int32_t finish_tlas(PulseScene* s, uint32_t* count, uint32_t* levels) {
-  uint32_t h[4];
-  for (int k = 0; k < 4; ++k) h[k] = reinterpret_cast<volatile uint32_t*>(s->meta_host)[k];
+static int32_t finish_tlas(PulseScene* s, uint32_t* count, uint32_t* levels, WideTree* wt) {
+  uint32_t h[4 + wide::kHeadWords];
+  for (uint32_t k = 0; k < 4 + wide::kHeadWords; ++k) h[k] = reinterpret_cast<volatile uint32_t*>(s->meta_host)[k];
   if ((int)h[2] == -7)
     return set_err(s->ctx, PULSE_ERR_DEGENERATE,
                    "TLAS: degenerate split, the reference's partition would underflow (src/scene/tlas.rs)");
   if (h[2] != 0 || h[0] == 0) return set_err(s->ctx, PULSE_ERR_CUDA, "TLAS: internal index check failed");
   *count = h[0];
   *levels = h[1];
+  wt->read(h + 4);
   return PULSE_OK;
 }
 
@@ -1111,6 +1268,10 @@ int32_t pulse_instances_set(PulseScene* s, const PulseInstanceDesc* inst, uint32
     ii[i].index_offset = t[2];
     ii[i].node_offset = t[3];
     ii[i].material_index = d.material_index;
+    const MeshRec& mesh = s->meshes[d.mesh_id];
+    ii[i].wide_root = mesh.wide_root ? 0u : s->mesh_wide[d.mesh_id] | (1u << 24);
+    ii[i].wide_slack = mesh.wide_slack;
+    ii[i].wide_leaf = mesh.wide_root ? mesh.wide_root + t[2] : 0u;
     const float* em = s->host_materials[d.material_index].emissive;
     const float len = std::sqrt(em[0] * em[0] + em[1] * em[1] + em[2] * em[2]);
     if (len > 0.0001f) {
@@ -1148,9 +1309,10 @@ int32_t pulse_instances_set(PulseScene* s, const PulseInstanceDesc* inst, uint32
   e = upload_keep(d_ii, ii.data(), (size_t)n * sizeof(prep::InstanceIn), st);
   if (e == cudaSuccess) e = ensure(s->instances, (size_t)n * 160);
   if (e == cudaSuccess) e = ensure(s->inst_bounds, (size_t)n * 36);
+  if (e == cudaSuccess) e = ensure(s->inst_wide, (size_t)n * pt::kWideInstRows * 16);
   if (e == cudaSuccess)
     e = prep::instances((const prep::InstanceIn*)d_ii.p, n, (const float4*)s->blas_nodes.p, (float4*)s->instances.p,
-                        (float*)s->inst_bounds.p, st);
+                        (float*)s->inst_bounds.p, (float4*)s->inst_wide.p, st);
   if (e == cudaSuccess) e = upload_keep(d_lights, lights.data(), (size_t)L * sizeof(prep::LightIn), st);
   if (e == cudaSuccess) e = ensure(s->tri_cdfs, (size_t)cdf_len * 4);
   if (e == cudaSuccess) e = ensure(s->mesh_areas, (size_t)L * 4);
@@ -1165,7 +1327,8 @@ int32_t pulse_instances_set(PulseScene* s, const PulseInstanceDesc* inst, uint32
   // TLAS (src/scene/tlas.rs:29-65).
   uint32_t tlas_count = 1, tlas_levels = 1;
   bool pending = false;
-  if (rc == PULSE_OK) rc = rebuild_tlas(s, n, tp, &tlas_count, &tlas_levels, &pending, st);
+  WideTree wt;
+  if (rc == PULSE_OK) rc = rebuild_tlas(s, n, tp, &tlas_count, &tlas_levels, &wt, &pending, st);
   if (rc == PULSE_OK) {
     std::vector<std::array<uint32_t, 3>> ranges;
     for (const MeshRec& m : s->meshes)
@@ -1181,7 +1344,9 @@ int32_t pulse_instances_set(PulseScene* s, const PulseInstanceDesc* inst, uint32
     // from now on starts after the update has completed.
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) rc = cuda_err(ctx, e, "scene finalize");
-    if (rc == PULSE_OK && pending) rc = finish_tlas(s, &tlas_count, &tlas_levels);
+    if (rc == PULSE_OK && pending) rc = finish_tlas(s, &tlas_count, &tlas_levels, &wt);
+    if (rc != PULSE_OK) wt.ok = false;
+    decide_wide(s, ii, wt);
     s->counts.tlas_node_count = tlas_count;
     s->dev.fast_slabs = 1u;  // trees built here nest by construction
     s->dev.tlas_levels = tlas_levels;
@@ -1237,19 +1402,21 @@ int32_t pulse_instances_update(PulseScene* s, const uint32_t* idx, const float* 
   if (e == cudaSuccess) e = upload_keep(d_slot, idx, (size_t)n * 4, st);
   if (e == cudaSuccess)
     e = prep::instances((const prep::InstanceIn*)d_ii.p, n, (const float4*)s->blas_nodes.p, (float4*)s->instances.p,
-                        (float*)s->inst_bounds.p, st, (const uint32_t*)d_slot.p);
+                        (float*)s->inst_bounds.p, (float4*)s->inst_wide.p, st, (const uint32_t*)d_slot.p);
   int32_t rc = e == cudaSuccess ? PULSE_OK : cuda_err(ctx, e, "instance update");
   ctx->stats.kernel_launches += n ? 1 : 0;
   uint32_t tlas_count = 1, tlas_levels = 1;
   bool pending = false;
-  if (rc == PULSE_OK) rc = rebuild_tlas(s, K, &tp, &tlas_count, &tlas_levels, &pending, st);
+  WideTree wt;
+  if (rc == PULSE_OK) rc = rebuild_tlas(s, K, &tp, &tlas_count, &tlas_levels, &wt, &pending, st);
   if (rc == PULSE_OK) {
     s->dev.tlas_nodes = (const float4*)s->tlas_nodes.p;
     s->dev.instance_indices = (const uint32_t*)s->instance_indices.p;
+    set_wide_tlas(s);
     cudaEventRecord(ctx->ev1, st);
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) rc = cuda_err(ctx, e, "instance update");
-    if (rc == PULSE_OK && pending) rc = finish_tlas(s, &tlas_count, &tlas_levels);
+    if (rc == PULSE_OK && pending) rc = finish_tlas(s, &tlas_count, &tlas_levels, &wt);
     s->counts.tlas_node_count = tlas_count;
     s->dev.tlas_levels = tlas_levels;
     float ms = 0.0f;
@@ -1264,6 +1431,7 @@ int32_t pulse_instances_update(PulseScene* s, const uint32_t* idx, const float* 
     std::memcpy(s->last_inst[idx[k]].object_world, object_world + 16 * (size_t)k, 64);
   }
   s->last_tlas = tp;
+  decide_wide(s, s->last_ii, wt);
   return PULSE_OK;
 }
 

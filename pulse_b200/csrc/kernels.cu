@@ -2,12 +2,14 @@
 #include <atomic>
 
 #include "kernels.h"
+#include "pt_wide.cuh"
+#include "wavefront.h"
 
 namespace pt {
 
 __global__ void k_gather_tri_bvh(const float4* __restrict__ primitives, const uint32_t* __restrict__ tri_idx,
-                                 float4* __restrict__ tri_bvh, uint32_t triangle_offset, uint32_t index_offset,
-                                 uint32_t count) {
+                                 const uint32_t* __restrict__ leaf_of, float4* __restrict__ tri_bvh,
+                                 uint32_t triangle_offset, uint32_t index_offset, uint32_t count) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const uint32_t slot = index_offset + i;
@@ -16,16 +18,16 @@ __global__ void k_gather_tri_bvh(const float4* __restrict__ primitives, const ui
   const float4 a = p[0], b = p[1], c = p[2];
   float4* o = tri_bvh + (size_t)slot * 3;
   o[0] = make_float4(a.x, a.y, a.z, __uint_as_float(tri));
-  o[1] = make_float4(b.x - a.x, b.y - a.y, b.z - a.z, 0.0f);
+  o[1] = make_float4(b.x - a.x, b.y - a.y, b.z - a.z, __uint_as_float(leaf_of ? leaf_of[slot] : 0u));
   o[2] = make_float4(c.x - a.x, c.y - a.y, c.z - a.z, 0.0f);
 }
 
-cudaError_t launch_gather_tri_bvh(const float4* primitives, const uint32_t* triangle_indices, float4* tri_bvh,
-                                  uint32_t triangle_offset, uint32_t index_offset, uint32_t count,
-                                  cudaStream_t st) {
+cudaError_t launch_gather_tri_bvh(const float4* primitives, const uint32_t* triangle_indices,
+                                  const uint32_t* leaf_of, float4* tri_bvh, uint32_t triangle_offset,
+                                  uint32_t index_offset, uint32_t count, cudaStream_t st) {
   if (count == 0) return cudaSuccess;
-  k_gather_tri_bvh<<<(count + 255) / 256, 256, 0, st>>>(primitives, triangle_indices, tri_bvh, triangle_offset,
-                                                         index_offset, count);
+  k_gather_tri_bvh<<<(count + 255) / 256, 256, 0, st>>>(primitives, triangle_indices, leaf_of, tri_bvh,
+                                                         triangle_offset, index_offset, count);
   return cudaGetLastError();
 }
 
@@ -164,6 +166,7 @@ cudaError_t launch_trace_rays(const DevScene& S, const TraceCfg& tc, const float
   static std::atomic<uint64_t> done{0};
   if (cudaError_t e = stack_limit(k_trace_rays, done)) return e;
   if (n == 0) return cudaSuccess;
+  if (wide_allowed(tc, S)) return wide_trace_rays(S, tc, rays, n, out, ctr, st);
   k_trace_rays<<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, stack_smem_bytes(tc, kTraceBlock), st>>>(
       S, tc, rays, n, out, ctr);
   return cudaGetLastError();

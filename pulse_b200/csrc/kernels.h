@@ -13,10 +13,11 @@ struct FrameCfg {
   uint32_t W, H, acc;
 };
 
-// One mesh's BVH-ordered triangle gather (see pt_trace.cuh, tri_bvh).
-cudaError_t launch_gather_tri_bvh(const float4* primitives, const uint32_t* triangle_indices, float4* tri_bvh,
-                                  uint32_t triangle_offset, uint32_t index_offset, uint32_t count,
-                                  cudaStream_t st);
+// One mesh's BVH-ordered triangle gather (see pt_trace.cuh, tri_bvh).  leaf_of: the
+// leaf node of every slot, or nullptr (then 0).
+cudaError_t launch_gather_tri_bvh(const float4* primitives, const uint32_t* triangle_indices,
+                                  const uint32_t* leaf_of, float4* tri_bvh, uint32_t triangle_offset,
+                                  uint32_t index_offset, uint32_t count, cudaStream_t st);
 
 // Per-pixel megakernel: every sample of a texel traced to termination by one
 // thread, then accumulated.  block = 128 threads over a 16 x 8 texel tile.

@@ -7,7 +7,7 @@
 //
 // Layout used on the device (built by the library at upload):
 //   nodes       float4 pairs (min.xyz | a) (max.xyz | count) -- the 32 B std430 node
-//   tri_bvh     three float4 per BVH slot of every mesh: (p0 | tri id), (p1 - p0), (p2 - p0)
+//   tri_bvh     three float4 per BVH slot of every mesh: (p0 | tri id), (p1 - p0 | leaf node), (p2 - p0)
 //               i.e. primitives[triangle_offset + triangle_indices[index_offset + slot]]
 //               pre-gathered into BVH order with the two Moller-Trumbore edges pre-subtracted
 //               (same IEEE subtraction, same bits); 48 B per test instead of 4 + 48 B.
@@ -37,6 +37,12 @@ struct DevScene {
   uint32_t instance_count, light_count;
   uint32_t fast_slabs;  // every child box lies inside its parent's: the slab guard is valid
   uint32_t tlas_levels, blas_levels;  // levels of the TLAS and of the deepest BLAS (root alone: 1)
+  // Eight-wide trees (pt_wide.cuh); valid when wide is set.
+  const uint4* __restrict__ wide_blas;       // 6 x uint4 per node, every mesh's tree
+  const uint4* __restrict__ wide_tlas;
+  const float4* __restrict__ inst_wide;      // 6 x float4 per instance (pt_wide.cuh)
+  float wide_slack;                          // the largest slack of the scene's meshes
+  uint32_t wide, wide_stack, wide_top;       // stack entries: in all, and for the TLAS
 };
 
 struct TraceCfg {
@@ -47,6 +53,9 @@ struct TraceCfg {
   // equal those of a stack_depth-entry stack; at stack_depth, pushes beyond
   // it are dropped and counted as in the reference.
   uint32_t stack_t, stack_b;
+  // Entries of the eight-wide traversal's stack (the launch's largest DevScene::wide_stack),
+  // and of its TLAS part (the largest wide_top).
+  uint32_t stack_w, stack_top;
   uint32_t iter_cap;
   float eps_tri, eps_par;
   bool quirks;
@@ -309,8 +318,11 @@ __host__ __device__ constexpr uint32_t trace_smem_words(const TraceCfg& tc) {
   return tc.stack_t + tc.stack_b + kColdWords;
 }
 
-// The per-level stack sizes for trees of the given levels.
-__host__ __device__ inline void trace_stacks(TraceCfg& tc, uint32_t tlas_levels, uint32_t blas_levels) {
+// The stack sizes for trees of the given levels and wide stack.
+__host__ __device__ inline void trace_stacks(TraceCfg& tc, uint32_t tlas_levels, uint32_t blas_levels,
+                                             uint32_t wide_stack, uint32_t wide_top) {
+  tc.stack_w = wide_stack;
+  tc.stack_top = wide_top;
   const uint32_t t = tlas_levels > 1 ? tlas_levels - 1 : 1, b = blas_levels > 1 ? blas_levels - 1 : 1;
   tc.stack_t = t < tc.stack_depth ? t : tc.stack_depth;
   tc.stack_b = b < tc.stack_depth ? b : tc.stack_depth;

@@ -2,6 +2,7 @@
 #include <cfloat>
 
 #include "pt_math.cuh"
+#include "pt_wide.cuh"
 #include "scene_prep.cuh"
 
 namespace prep {
@@ -66,7 +67,8 @@ __device__ void inverse4(const float* src, float* dst) {
 }
 
 __global__ void k_instances(const InstanceIn* __restrict__ in, uint32_t n, const float4* __restrict__ blas_nodes,
-                            float4* inst_out, float* bounds9, const uint32_t* __restrict__ slot) {
+                            float4* inst_out, float* bounds9, float4* wide_out,
+                            const uint32_t* __restrict__ slot) {
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   const InstanceIn x = in[j];
@@ -81,6 +83,12 @@ __global__ void k_instances(const InstanceIn* __restrict__ in, uint32_t n, const
   o[8] = make_float4(__uint_as_float(x.triangle_offset), __uint_as_float(x.triangle_count),
                      __uint_as_float(x.index_offset), __uint_as_float(x.node_offset));
   o[9] = make_float4(__uint_as_float(x.material_index), 0.0f, 0.0f, 0.0f);
+  // the wide traversal's record (pt_wide.cuh); its TLAS leaf comes with the tree
+  float4* wo = wide_out + (size_t)i * kWideInstRows;
+  for (int c = 0; c < 4; ++c) wo[c] = make_float4(inv[4 * c], inv[4 * c + 1], inv[4 * c + 2], inv[4 * c + 3]);
+  wo[4] = make_float4(__uint_as_float(x.wide_root), __uint_as_float(x.wide_leaf), x.wide_slack, 0.0f);
+  wo[5] = make_float4(__uint_as_float(x.index_offset), __uint_as_float(x.node_offset),
+                      __uint_as_float(kWideRootLeaf), 0.0f);
   // World bounds of the root box (src/scene/mod.rs:625-658).
   const float4 lo = blas_nodes[2 * (size_t)x.node_offset], hi = blas_nodes[2 * (size_t)x.node_offset + 1];
   const M4 m{o[0], o[1], o[2], o[3]};
@@ -152,9 +160,9 @@ cudaError_t soup(const float* pos, const float* nrm, const float* uv, const uint
 }
 
 cudaError_t instances(const InstanceIn* in, uint32_t n, const float4* blas_nodes, float4* inst_out, float* bounds9,
-                      cudaStream_t st, const uint32_t* slot) {
+                      float4* wide_out, cudaStream_t st, const uint32_t* slot) {
   if (!n) return cudaSuccess;
-  k_instances<<<(n + 127) / 128, 128, 0, st>>>(in, n, blas_nodes, inst_out, bounds9, slot);
+  k_instances<<<(n + 127) / 128, 128, 0, st>>>(in, n, blas_nodes, inst_out, bounds9, wide_out, slot);
   return cudaGetLastError();
 }
 

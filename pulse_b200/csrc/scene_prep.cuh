@@ -12,15 +12,18 @@ cudaError_t soup(const float* pos, const float* nrm, const float* uv, const uint
 
 struct InstanceIn {
   float object_world[16];
-  uint32_t triangle_offset, triangle_count, index_offset, node_offset, material_index, pad[3];
+  uint32_t triangle_offset, triangle_count, index_offset, node_offset, material_index;
+  uint32_t wide_root, wide_leaf;  // root group of the mesh's eight-wide tree, or 0 and its only leaf
+  float wide_slack;
 };
 
 // prepare_mesh_instances (src/scene/mod.rs:561-681) per instance: the 160 B
 // record with the inverse transform, and the world bounds of the BLAS root
-// (8 transformed corners) with their centre -> bounds9.  With `slot`, input i
-// writes record and bounds slot[i] (an incremental update of some instances).
+// (8 transformed corners) with their centre -> bounds9; the wide traversal's record
+// (pt_wide.cuh) -> wide_out.  With `slot`, input i writes records and bounds slot[i] (an
+// incremental update of some instances).
 cudaError_t instances(const InstanceIn* in, uint32_t n, const float4* blas_nodes, float4* inst_out, float* bounds9,
-                      cudaStream_t st, const uint32_t* slot = nullptr);
+                      float4* wide_out, cudaStream_t st, const uint32_t* slot = nullptr);
 
 struct LightIn { uint32_t instance, triangle_offset, triangle_count, cdf_offset, material; };
 

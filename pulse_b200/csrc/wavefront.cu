@@ -34,6 +34,7 @@
 #include <atomic>
 #include <cstring>
 
+#include "pt_wide.cuh"
 #include "wavefront.h"
 #include "wf_common.cuh"
 
@@ -43,30 +44,7 @@ namespace {
 
 using namespace wf;
 
-constexpr int kWfBlock = 128;
 constexpr uint32_t kTableChunk = 8;  // table entries per upload launch (kernel parameter)
-
-// The scene table in shared memory: [n entries of WfScene][traversal stacks].
-__device__ __forceinline__ const WfScene* load_table(const WfScene* g, uint32_t n, uint32_t* smem) {
-  WfScene* t = reinterpret_cast<WfScene*>(smem);
-  const uint4* src = reinterpret_cast<const uint4*>(g);
-  uint4* dst = reinterpret_cast<uint4*>(t);
-  const uint32_t words = n * (uint32_t)(sizeof(WfScene) / sizeof(uint4));
-  for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
-  __syncthreads();
-  return t;
-}
-__device__ __forceinline__ uint32_t* stacks_after(uint32_t* smem, uint32_t n) {
-  return smem + n * (uint32_t)(sizeof(WfScene) / 4);
-}
-__device__ __forceinline__ uint32_t scene_of(const WfScene* t, uint32_t n, uint32_t p) {
-  uint32_t lo = 0, hi = n;  // last scene with path_offset <= p
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (t[mid].path_offset <= p) lo = mid; else hi = mid;
-  }
-  return lo;
-}
 
 template <int MODE>
 __global__ void __launch_bounds__(kWfBlock) k_wf_generate(WfBuffers B, uint32_t n_scenes, uint32_t total) {
@@ -90,16 +68,6 @@ __global__ void __launch_bounds__(kWfBlock) k_wf_generate(WfBuffers B, uint32_t 
     const uint32_t slot = warp_append(alive, B.counts + 0);
     if (alive) B.q[0][slot] = p;
   }
-}
-
-// Shadow request slot ss of path p of scene sid.
-__device__ __forceinline__ void put_shadow(const WfBuffers& B, uint32_t ss, const ShadowReq& rq, uint32_t p,
-                                           uint32_t sid) {
-  float4* e = B.shadow + 4 * (size_t)ss;
-  e[0] = make_float4(rq.o.x, rq.o.y, rq.o.z, rq.limit);
-  e[1] = make_float4(rq.d.x, rq.d.y, rq.d.z, __uint_as_float(p));
-  e[2] = make_float4(rq.add_vis.x, rq.add_vis.y, rq.add_vis.z, __uint_as_float(sid));
-  e[3] = make_float4(rq.add_occ.x, rq.add_occ.y, rq.add_occ.z, 0.0f);
 }
 
 // Sample s of the realtime GI pass (src/pulse/gi.wgsl:56-83): one path per
@@ -194,22 +162,6 @@ __global__ void __launch_bounds__(kWfBlock) k_gi_resolve(WfBuffers B, float4* im
     const float3 out = add(prev, muls(c, spp_inv));
     image[p] = make_float4(out.x, out.y, out.z, 1.0f);
   }
-}
-
-template <int MODE>
-__device__ __forceinline__ void finish_shadow(const WfBuffers& B, uint32_t i, float hit_t) {
-  const float4* e = B.shadow + 4 * (size_t)i;
-  const float4 a = e[0], b = e[1], c = e[2], d = e[3];
-  const uint32_t p = __float_as_uint(b.w);
-  ShadowReq rq;
-  rq.limit = a.w;
-  rq.add_vis = xyz(c);
-  rq.add_occ = xyz(d);
-  const float4 col = B.s[4 * (size_t)p + 3];
-  PathState ps;
-  ps.color = xyz(col);
-  path_on_shadow<MODE>(ps, rq, hit_t);
-  B.s[4 * (size_t)p + 3] = make_float4(ps.color.x, ps.color.y, ps.color.z, col.w);
 }
 
 // Closest hit of every path of queue qi into h0/h1.  SHADOW >= 0 (estimator
@@ -649,6 +601,7 @@ cudaError_t raise_limits() {
     if (e == cudaSuccess) e = smem_attr(tail_kernel<MODE>(1, block));
     if (e == cudaSuccess) e = smem_attr(tail_kernel<MODE>(4, block));
   }
+  if (!COUNT && e == cudaSuccess) e = wide_prepare(MODE);
   if (e == cudaSuccess) e = smem_attr(k_wf_generate<MODE>);
   if (e == cudaSuccess) e = smem_attr(k_sort_count);
   if (e == cudaSuccess) e = smem_attr(k_sort_scatter);
@@ -699,11 +652,13 @@ uint32_t record_segments(const TraceCfg& tc, const WfBuffers& B, const WfLaunch&
   const ShadowK shadow = shadow_kernel<MODE, COUNT>(minb, tb);
   const TailK tail = tail_kernel<MODE>(g.tbps >= 4 ? 4 : 1, tb);
   const bool merge = MODE != 0 && !COUNT;
+  const bool wide = L.wide && !COUNT;
   uint32_t n = 0;
   const uint32_t wf = L.wf_segments < L.segments ? L.wf_segments : L.segments;
   int qi = 0;
   auto resolve = [&]() {
-    shadow<<<grid, tb, smem_tr, st>>>(tc, B, ns, ctr, work);
+    if (wide) wide_shadow(MODE, tc, B, L, ctr, st);
+    else shadow<<<grid, tb, smem_tr, st>>>(tc, B, ns, ctr, work);
     ++n;
     pending = false;
   };
@@ -720,7 +675,8 @@ uint32_t record_segments(const TraceCfg& tc, const WfBuffers& B, const WfLaunch&
       qi ^= 1;
     }
     k_wf_reset<<<1, 32, 0, st>>>(B.counts, qi ^ 1, pending ? 1 : 0);
-    (pending ? extend_sh : extend)<<<grid, tb, smem_tr, st>>>(tc, B, ns, qi, ctr, work);
+    if (wide) wide_extend(pending ? MODE : -1, tc, B, L, qi, ctr, st);
+    else (pending ? extend_sh : extend)<<<grid, tb, smem_tr, st>>>(tc, B, ns, qi, ctr, work);
     pending = false;
     k_wf_shade<MODE, COUNT><<<g.light_blocks, kWfBlock, g.tab, st>>>(B, ns, qi, work);
     n += 3;
@@ -733,7 +689,8 @@ uint32_t record_segments(const TraceCfg& tc, const WfBuffers& B, const WfLaunch&
   if (pending) resolve();  // no wavefront segment follows (no bounce, or tail only)
   if (!COUNT && wf < L.segments) {
     k_wf_reset<<<1, 32, 0, st>>>(B.counts, qi ^ 1, 0);
-    tail<<<grid, tb, smem_tr, st>>>(tc, B, ns, qi, ctr);
+    if (wide) wide_tail(MODE, tc, B, L, qi, ctr, st);
+    else tail<<<grid, tb, smem_tr, st>>>(tc, B, ns, qi, ctr);
     n += 2;
   }
   return n;
@@ -825,9 +782,17 @@ cudaError_t wf_upload_table(const WfScene* host, uint32_t n, WfScene* dev, cudaS
   return cudaGetLastError();
 }
 
-cudaError_t wf_extend_step(const TraceCfg& tc, const WfBuffers& B, int qi, uint32_t trace_blocks, Counters* ctr,
-                           cudaStream_t st) {
+cudaError_t wf_extend_step(const TraceCfg& tc, const WfBuffers& B, int qi, uint32_t trace_blocks, bool wide,
+                           Counters* ctr, cudaStream_t st) {
   if (cudaError_t e = wf_prepare(2)) return e;
+  if (wide) {
+    WfLaunch L{};
+    L.n_scenes = 1;
+    L.trace_blocks_per_sm = trace_blocks;
+    L.sms = device_sms();
+    wide_extend(-1, tc, B, L, qi, ctr, st);
+    return cudaGetLastError();
+  }
   const uint32_t tbps = trace_blocks ? trace_blocks : kDefaultTraceBlocks;
   const size_t smem = sizeof(WfScene) + (size_t)trace_smem_words(tc) * kWfBlock * 4;
   extend_kernel<false>(budget(tbps))<<<device_sms() * (int)tbps, kWfBlock, smem, st>>>(tc, B, 1, qi, ctr, nullptr);
@@ -847,7 +812,8 @@ cudaError_t wf_gbuffer_primary(const TraceCfg& tc, const WfScene& scene, float4*
   one.path_offset = 0;
   one.paths = one.fc.W * one.fc.H;
   TraceCfg tcs = tc;
-  trace_stacks(tcs, one.S.tlas_levels, one.S.blas_levels);
+  trace_stacks(tcs, one.S.tlas_levels, one.S.blas_levels, one.S.wide_stack,
+               one.S.wide_top);
   const uint32_t tbps = trace_blocks ? trace_blocks : kDefaultTraceBlocks;
   const int sms = device_sms();
   const size_t tab = sizeof(WfScene);
@@ -856,7 +822,15 @@ cudaError_t wf_gbuffer_primary(const TraceCfg& tc, const WfScene& scene, float4*
   if (e == cudaSuccess) e = cudaMemsetAsync(B.counts, 0, 8 * sizeof(uint32_t), st);
   if (e != cudaSuccess) return e;
   k_gbuf_generate<<<sms * 16, kWfBlock, tab, st>>>(B);
-  extend_kernel<false>(budget(tbps))<<<sms * (int)tbps, kWfBlock, smem, st>>>(tcs, B, 1, 0, ctr, nullptr);
+  if (wide_allowed(tcs, one.S)) {
+    WfLaunch L{};
+    L.n_scenes = 1;
+    L.trace_blocks_per_sm = trace_blocks;
+    L.sms = sms;
+    wide_extend(-1, tcs, B, L, 0, ctr, st);
+  } else {
+    extend_kernel<false>(budget(tbps))<<<sms * (int)tbps, kWfBlock, smem, st>>>(tcs, B, 1, 0, ctr, nullptr);
+  }
   k_gbuf_write<<<sms * 16, kWfBlock, tab, st>>>(B, gbuf);
   if (launches) *launches += 4;
   return cudaGetLastError();
@@ -879,7 +853,10 @@ cudaError_t wf_render_gi(const TraceCfg& tc, const WfScene& scene, const float4*
   L.trace_blocks_per_sm = trace_blocks;
   L.sms = device_sms();
   TraceCfg tcs = tc;
-  trace_stacks(tcs, one.S.tlas_levels, one.S.blas_levels);
+  trace_stacks(tcs, one.S.tlas_levels, one.S.blas_levels, one.S.wide_stack,
+               one.S.wide_top);
+  L.wide = wide_allowed(tcs, one.S);
+  if (L.wide && !wf_segments) L.wf_segments = kDefaultWideSegments;
   cudaError_t e = wf_upload_table(&one, 1, B.table, st);
   if (e != cudaSuccess) return e;
   if (launches) *launches += 1;
@@ -907,13 +884,20 @@ cudaError_t wf_render(int mode, const TraceCfg& tc, const WfScene* scenes, uint3
   L.trace_blocks_per_sm = trace_blocks;
   L.sms = device_sms();
   L.image_wait = image_wait;
-  uint32_t tl = 1, bl = 1;  // the deepest trees of the batch size the stacks
+  uint32_t tl = 1, bl = 1, wl = 0, wt = 0;  // the deepest trees of the batch size the stacks
   for (uint32_t i = 0; i < n; ++i) {
     tl = tab[i].S.tlas_levels > tl ? tab[i].S.tlas_levels : tl;
     bl = tab[i].S.blas_levels > bl ? tab[i].S.blas_levels : bl;
+    // (the TLAS part and the BLAS part above it can be largest in different scenes)
+    const uint32_t below = tab[i].S.wide_stack - tab[i].S.wide_top;
+    wl = below > wl ? below : wl;
+    wt = tab[i].S.wide_top > wt ? tab[i].S.wide_top : wt;
   }
   TraceCfg tcs = tc;
-  trace_stacks(tcs, tl, bl);
+  trace_stacks(tcs, tl, bl, wl + wt, wt);
+  L.wide = true;  // one scene that cannot keeps the batch on the binary traversal
+  for (uint32_t i = 0; i < n; ++i) L.wide = L.wide && wide_allowed(tcs, tab[i].S);
+  if (L.wide && !wf_segments) L.wf_segments = kDefaultWideSegments;
   cudaError_t e = wf_upload_table(tab, n, B.table, st);
   if (e != cudaSuccess) return e;
   if (launches) *launches += (n + kTableChunk - 1) / kTableChunk;

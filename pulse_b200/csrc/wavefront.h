@@ -15,6 +15,9 @@ constexpr uint32_t kWfTailOnly = 0xffffffffu;
 // from 2 to 3; the realtime GI frame is fastest at 2).
 constexpr uint32_t kDefaultWfSegments = 3;
 constexpr uint32_t kDefaultGiWfSegments = 2;
+// The same with the eight-wide traversal: its launches drain quickly, and the tail's
+// shading thrashes the instruction cache beside the traversal's code.
+constexpr uint32_t kDefaultWideSegments = 16;
 // Traversal blocks per SM when the parameter is 0: eight 128-thread blocks of
 // a 64-register budget fill the register file (1080p sphere frame: 5 blocks
 // 138.7, 6 blocks 140.9, 8 blocks 143.7 Mpaths/s; the spills of the 64-register
@@ -56,6 +59,7 @@ struct WfLaunch {
   uint32_t wf_segments;          // segments run as wavefront steps before the tail kernel
   uint32_t trace_blocks_per_sm;  // 0 = kDefaultTraceBlocks
   int sms;
+  bool wide = false;             // every scene's rays take the eight-wide traversal
   cudaEvent_t image_wait = nullptr;  // awaited before the accumulation writes the images
 };
 
@@ -128,9 +132,27 @@ cudaError_t wf_render_gi(const TraceCfg& tc, const WfScene& scene, const float4*
 // wf_render with B (its one-scene table): the closest hit of every path of
 // queue qi into B.h0/h1, and the reset of the counters before a segment whose
 // next queue is `next`.
-cudaError_t wf_extend_step(const TraceCfg& tc, const WfBuffers& B, int qi, uint32_t trace_blocks, Counters* ctr,
-                           cudaStream_t st);
+// wide: with the eight-wide traversal.
+cudaError_t wf_extend_step(const TraceCfg& tc, const WfBuffers& B, int qi, uint32_t trace_blocks, bool wide,
+                           Counters* ctr, cudaStream_t st);
 cudaError_t wf_reset_step(const WfBuffers& B, int next, cudaStream_t st);
+
+// The frame's traversal launches with the eight-wide trees (wavefront_wide.cu), for
+// launches whose scenes all allow it (pt_wide.cuh); errors are left for
+// cudaGetLastError.  shadow: the estimator mode whose previous segment's shadow requests
+// the extend also resolves, or -1.
+cudaError_t wide_prepare(int mode);
+void wide_extend(int shadow, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, int qi, Counters* ctr,
+                 cudaStream_t st);
+void wide_shadow(int mode, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, Counters* ctr, cudaStream_t st);
+void wide_tail(int mode, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, int qi, Counters* ctr,
+               cudaStream_t st);
+// The adjoint's shadow rays: visible ones set flag in word 3 (w) of their path's record.
+void wide_adj_shadow(const TraceCfg& tc, const DevScene& S, const WfBuffers& B, float4* rec, uint32_t rec_rows,
+                     uint32_t flag, uint32_t trace_blocks, Counters* ctr, cudaStream_t st);
+// Closest hits of n rays (6 floats each).
+cudaError_t wide_trace_rays(const DevScene& S, const TraceCfg& tc, const float* rays, uint32_t n, Hit* out,
+                            Counters* ctr, cudaStream_t st);
 
 // The table entry of one scene.
 inline WfScene wf_scene(const DevScene& S, const PathCfg& pc, const FrameCfg& fc, float4* image) {

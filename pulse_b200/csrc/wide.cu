@@ -1,0 +1,344 @@
+// wide.cu -- collapses binary BVHs into the eight-wide quantized nodes of
+// pt_wide.cuh.
+//
+// Children are found top-down: the interior child of the largest surface area is replaced by its
+// two children until there are eight.  One block walks the tree level by level
+// (a thread per wide node); a wide node takes a few microseconds of dependent loads,
+// so the blocks of a cooperative launch share the levels of large trees.
+#include <cooperative_groups.h>
+
+#include "pt_wide.cuh"
+#include "wide.cuh"
+
+namespace wide {
+
+namespace {
+
+constexpr int kBlock = 256;
+
+__device__ __forceinline__ float half_area(float4 lo, float4 hi) {
+  const float x = hi.x - lo.x, y = hi.y - lo.y, z = hi.z - lo.z;
+  return x * y + y * z + z * x;
+}
+
+// Where the leaf node of an element goes: an array by slot, or (instances) their records.
+struct LeafSink {
+  uint32_t* by_slot;
+  const uint32_t* instance_of;
+  float4* records;
+  __device__ __forceinline__ void put(uint32_t slot, uint32_t node) const {
+    if (by_slot) by_slot[slot] = node;
+    else records[(size_t)instance_of[slot] * pt::kWideInstRows + 5].z = __uint_as_float(node);
+  }
+  // A TLAS element's reference.
+  __device__ __forceinline__ uint32_t ref(uint32_t slot) const {
+    const uint32_t i = instance_of[slot];
+    return i | (records[(size_t)i * pt::kWideInstRows + 4].z > pt::kLeastSlack ? pt::kLooseRef : 0u);
+  }
+};
+
+// A BLAS leaf's reference.
+__device__ uint32_t leaf_ref(uint32_t first, uint32_t count, uint32_t* head) {
+  if (count > pt::kWideMaxCount || first + count > (1u << pt::kWideFirstBits)) {
+    head[kBad] = 1u;
+    return 0u;
+  }
+  return (count << pt::kWideFirstBits) | first;
+}
+
+// Up to eight children of one wide node.  A TLAS leaf of several instances is as many
+// children with the same box.
+struct Children {
+  float lo[8][3], hi[8][3];
+  uint32_t node[8], ref[8];  // binary node; a leaf's reference
+  bool leaf[8];
+  uint32_t n = 0;
+};
+
+__device__ void write_node(const Children& c, const float lo[3], const float hi[3], uint4* out, uint32_t* queue,
+                           uint32_t* head) {
+  // slots: interior children sorted along the axis of their centres' largest spread, leaves from 7 down
+  uint32_t inner[8], ni = 0, nl = 0, slot_of[8];
+  float cmin[3] = {3e38f, 3e38f, 3e38f}, cmax[3] = {-3e38f, -3e38f, -3e38f};
+  bool bad = false;
+  for (uint32_t k = 0; k < c.n; ++k) {
+    if (c.leaf[k]) {
+      slot_of[k] = 7u - nl++;
+      continue;
+    }
+    for (int j = 0; j < 3; ++j) {
+      cmin[j] = fminf(cmin[j], c.lo[k][j] + c.hi[k][j]);
+      cmax[j] = fmaxf(cmax[j], c.lo[k][j] + c.hi[k][j]);
+    }
+    inner[ni++] = k;
+  }
+  uint32_t axis = 0;
+  for (uint32_t j = 1; j < 3; ++j)
+    if (cmax[j] - cmin[j] > cmax[axis] - cmin[axis]) axis = j;
+  for (uint32_t i = 1; i < ni; ++i) {  // insertion sort
+    const uint32_t k = inner[i];
+    uint32_t j = i;
+    for (; j > 0 && c.lo[inner[j - 1]][axis] + c.hi[inner[j - 1]][axis] > c.lo[k][axis] + c.hi[k][axis]; --j)
+      inner[j] = inner[j - 1];
+    inner[j] = k;
+  }
+  uint32_t at = 0;
+  if (ni) {
+    at = atomicAdd(head + kCount, ni);
+    if (at + ni >= (1u << pt::kWideIndexBits)) bad = true;
+  }
+  for (uint32_t i = 0; i < ni; ++i) {
+    slot_of[inner[i]] = i;
+    queue[at + i] = c.node[inner[i]];
+  }
+  uint32_t words[pt::kWideNodeWords];
+  for (uint32_t k = 0; k < pt::kWideNodeWords; ++k) words[k] = 0u;
+  uint8_t* q8 = reinterpret_cast<uint8_t*>(words + 8);
+  words[3] = (ni << 24) | (nl << 28);
+  words[4] = at | (axis << pt::kWideIndexBits);
+  for (int j = 0; j < 3; ++j) {
+    // quanta: 2^e with the children's extent in 254 of them, and large enough
+    // against the coordinates for the origin to move by 1/32 of one
+    const double mag = fmax(fabs((double)lo[j]), fabs((double)hi[j]));
+    const double need = fmax(fmax(((double)hi[j] - lo[j]) / 254.0, mag * 7.63e-6), 1e-30);
+    int e;
+    frexp(need, &e);  // need <= 2^e
+    const double s = ldexp(1.0, e);
+    const float p = __double2float_rd((double)lo[j] - s / 32.0);
+    words[j] = __float_as_uint(p);
+    words[3] |= (uint32_t)(e + 127 + 15) << (8 * j);
+    for (uint32_t k = 0; k < c.n; ++k) {
+      const double ql = floor((c.lo[k][j] - (double)p) / s - 1.0 / 64.0), qh = ceil((c.hi[k][j] - (double)p) / s + 1.0 / 64.0);
+      if (!(ql >= 0.0) || !(qh <= 255.0)) bad = true;
+      q8[16 * j + slot_of[k]] = (uint8_t)ql;
+      q8[16 * j + 8 + slot_of[k]] = (uint8_t)qh;
+    }
+  }
+  for (uint32_t k = 0; k < c.n; ++k)
+    if (c.leaf[k]) words[pt::wide_ref_word(7u - slot_of[k])] = c.ref[k];
+  if (bad) head[kBad] = 1u;
+  uint32_t* w = reinterpret_cast<uint32_t*>(out);
+  for (uint32_t k = 0; k < pt::kWideNodeWords; ++k) w[k] = words[k];
+}
+
+// The wide node of binary node b (interior).
+__device__ void make_node(const float4* __restrict__ nodes, uint32_t b, uint4* out, const LeafSink& leaf_of,
+                          uint32_t* queue, uint32_t* head) {
+  uint32_t c[8], mult[8];  // children; places each takes
+  float area[8];           // below 0: not to be opened
+  uint32_t n = 0, places = 0;
+  const bool tlas = leaf_of.instance_of != nullptr;
+  auto places_of = [&](uint32_t node) {
+    const uint32_t count = __float_as_uint(nodes[2 * (size_t)node + 1].w);
+    return tlas && count ? count : 1u;
+  };
+  auto put = [&](uint32_t k, uint32_t node) {
+    const float4 lo = nodes[2 * (size_t)node], hi = nodes[2 * (size_t)node + 1];
+    c[k] = node;
+    mult[k] = places_of(node);
+    area[k] = __float_as_uint(hi.w) ? -1.0f : fmaxf(half_area(lo, hi), 0.0f);
+    places += mult[k];
+  };
+  const uint32_t first = __float_as_uint(nodes[2 * (size_t)b].w);
+  put(n++, first);
+  put(n++, first + 1);
+  if (places > 8) {
+    head[kBad] = 1u;
+    return;
+  }
+  while (places < 8) {
+    int best = -1;
+    float most = -0.5f;
+    for (uint32_t k = 0; k < n; ++k)
+      if (area[k] > most) { most = area[k]; best = (int)k; }
+    if (best < 0) break;
+    const uint32_t a = __float_as_uint(nodes[2 * (size_t)c[best]].w);
+    if (places - 1 + places_of(a) + places_of(a + 1) > 8) {
+      area[best] = -1.0f;
+      continue;
+    }
+    places -= 1;
+    put((uint32_t)best, a);
+    put(n++, a + 1);
+  }
+  Children ch;
+  float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
+  bool bad = false;
+  for (uint32_t k = 0; k < n; ++k) {
+    const float4 a = nodes[2 * (size_t)c[k]], z = nodes[2 * (size_t)c[k] + 1];
+    const float p[3] = {a.x, a.y, a.z}, q[3] = {z.x, z.y, z.z};
+    const uint32_t start = __float_as_uint(a.w), count = __float_as_uint(z.w);
+    for (uint32_t i = 0; i < count; ++i) leaf_of.put(start + i, c[k]);
+    for (uint32_t i = 0; i < mult[k]; ++i) {
+      const uint32_t at = ch.n++;
+      ch.node[at] = c[k];
+      ch.leaf[at] = count != 0u;
+      ch.ref[at] = !count ? 0u : tlas ? leaf_of.ref(start + i) : leaf_ref(start, count, head);
+      for (int j = 0; j < 3; ++j) {
+        if (!(fabsf(p[j]) <= 1e9f) || !(fabsf(q[j]) <= 1e9f) || !(p[j] <= q[j])) bad = true;
+        ch.lo[at][j] = p[j];
+        ch.hi[at][j] = q[j];
+      }
+    }
+    for (int j = 0; j < 3; ++j) {
+      lo[j] = fminf(lo[j], p[j]);
+      hi[j] = fmaxf(hi[j], q[j]);
+    }
+  }
+  if (bad) {
+    head[kBad] = 1u;
+    return;
+  }
+  write_node(ch, lo, hi, out, queue, head);
+}
+
+// A TLAS that is one leaf: a node of its instances with boxes around every ray (the
+// reference enters a root without testing its box).
+__device__ void make_root_leaf(uint32_t start, uint32_t count, uint4* out, const LeafSink& leaf_of, uint32_t* queue,
+                               uint32_t* head) {
+  if (count > 8) {
+    head[kBad] = 1u;
+    return;
+  }
+  Children ch;
+  const float lo[3] = {-1e12f, -1e12f, -1e12f}, hi[3] = {1e12f, 1e12f, 1e12f};
+  for (uint32_t i = 0; i < count; ++i) {
+    leaf_of.put(start + i, pt::kWideRootLeaf);
+    ch.leaf[i] = true;
+    ch.node[i] = 0u;
+    ch.ref[i] = leaf_of.ref(start + i);
+    for (int j = 0; j < 3; ++j) ch.lo[i][j] = lo[j], ch.hi[i][j] = hi[j];
+  }
+  ch.n = count;
+  write_node(ch, lo, hi, out, queue, head);
+}
+
+template <bool GRID>
+__global__ void __launch_bounds__(kBlock) k_collapse(const float4* __restrict__ nodes,
+                                                     const uint32_t* __restrict__ meta, uint4* out, LeafSink leaf_of,
+                                                     uint32_t* queue, uint32_t* head) {
+  auto sync = [] {
+    if (GRID) {
+      cooperative_groups::this_grid().sync();
+    } else {
+      __threadfence();
+      __syncthreads();
+    }
+  };
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  if (meta && (meta[2] != 0u || meta[0] == 0u)) {
+    if (tid == 0) head[kBad] = 1u;
+    return;
+  }
+  const float4 rlo = nodes[0], rhi = nodes[1];
+  const uint32_t count = __float_as_uint(rhi.w);
+  if (tid == 0) {
+    const uint32_t start = __float_as_uint(rlo.w);
+    const bool tlas = leaf_of.instance_of != nullptr;
+    head[kBad] = 0u;
+    head[kLevels] = count && tlas ? 1u : 0u;
+    head[kRoot] = count && !tlas ? leaf_ref(start, count, head) : 0u;
+    queue[0] = 0u;
+    *(volatile uint32_t*)(head + kCount) = count && !tlas ? 0u : 1u;
+    if (count && tlas) make_root_leaf(start, count, out, leaf_of, queue, head);
+    else
+      for (uint32_t i = 0; i < count; ++i) leaf_of.put(start + i, pt::kWideRootLeaf);
+  }
+  if (count) return;  // the tree is one leaf
+  sync();
+  uint32_t begin = 0, levels = 0;
+  while (true) {
+    const uint32_t end = *(volatile uint32_t*)(head + kCount);
+    if (begin == end) break;
+    ++levels;
+    sync();  // every thread has read the count
+    for (uint32_t i = begin + tid; i < end; i += stride)
+      make_node(nodes, *(volatile uint32_t*)(queue + i), out + (size_t)i * (pt::kWideNodeWords / 4), leaf_of, queue,
+                head);
+    sync();
+    begin = end;
+  }
+  if (tid == 0) head[kLevels] = levels;
+}
+
+__global__ void __launch_bounds__(kBlock) k_relocate(const uint32_t* __restrict__ in, uint32_t n, uint32_t node_add,
+                                                     uint32_t slot_add, uint32_t* __restrict__ out) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t* a = in + (size_t)i * pt::kWideNodeWords;
+  uint32_t* b = out + (size_t)i * pt::kWideNodeWords;
+  uint32_t w[pt::kWideNodeWords];
+  for (uint32_t k = 0; k < pt::kWideNodeWords; ++k) w[k] = a[k];
+  const uint32_t ni = (w[3] >> 24) & 15u, nl = w[3] >> 28;
+  if (ni) w[4] += node_add;
+  for (uint32_t r = 0; r < nl; ++r) w[pt::wide_ref_word(r)] += slot_add;
+  for (uint32_t k = 0; k < pt::kWideNodeWords; ++k) b[k] = w[k];
+}
+
+__global__ void __launch_bounds__(kBlock) k_extents(const float4* __restrict__ prims, uint32_t n, uint32_t* head) {
+  float area = 0.0f, edge = 0.0f;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const float3 p0 = pt::xyz(prims[3 * (size_t)i]), p1 = pt::xyz(prims[3 * (size_t)i + 1]),
+                 p2 = pt::xyz(prims[3 * (size_t)i + 2]);
+    const float a = pt::length(pt::sub(p1, p0)), b = pt::length(pt::sub(p2, p0));
+    area = fmaxf(area, a * b);  // a NaN vertex cannot be hit: its triangle does not count
+    edge = fmaxf(edge, fmaxf(a, b));
+  }
+  const uint32_t am = __reduce_max_sync(0xffffffffu, __float_as_uint(area));
+  const uint32_t em = __reduce_max_sync(0xffffffffu, __float_as_uint(edge));
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(head + kArea, am);
+    atomicMax(head + kEdge, em);
+  }
+}
+
+}  // namespace
+
+namespace {
+cudaError_t launch(const float4* nodes, uint32_t n_nodes, const uint32_t* meta, uint4* out, LeafSink leaf_of,
+                   uint32_t* queue, uint32_t* head, cudaStream_t st) {
+  // One block up to 16k nodes (every per-frame instance tree of the scenes here): its
+  // levels cost a block barrier, and it needs no co-residency with a frame's kernels.
+  if (n_nodes <= 16384u) {
+    k_collapse<false><<<1, kBlock, 0, st>>>(nodes, meta, out, leaf_of, queue, head);
+    return cudaGetLastError();
+  }
+  int dev = 0, sms = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  void* args[] = {&nodes, &meta, &out, &leaf_of, &queue, &head};
+  return cudaLaunchCooperativeKernel((const void*)k_collapse<true>, dim3((unsigned)sms), dim3(kBlock), args, 0, st);
+}
+}  // namespace
+
+cudaError_t collapse(const float4* nodes, uint32_t n_nodes, uint4* out, uint32_t* leaf_of, uint32_t* queue,
+                     uint32_t* head, cudaStream_t st) {
+  return launch(nodes, n_nodes, nullptr, out, LeafSink{leaf_of, nullptr, nullptr}, queue, head, st);
+}
+
+cudaError_t collapse_tlas(const float4* nodes, uint32_t n_nodes, const uint32_t* meta, const uint32_t* instance_of,
+                          float4* records, uint4* out, uint32_t* queue, uint32_t* head, cudaStream_t st) {
+  return launch(nodes, n_nodes, meta, out, LeafSink{nullptr, instance_of, records}, queue, head, st);
+}
+
+cudaError_t relocate(const uint32_t* nodes, uint32_t n, uint32_t node_add, uint32_t slot_add, uint32_t* out,
+                     cudaStream_t st) {
+  if (!n) return cudaSuccess;
+  k_relocate<<<(n + kBlock - 1) / kBlock, kBlock, 0, st>>>(nodes, n, node_add, slot_add, out);
+  return cudaGetLastError();
+}
+
+cudaError_t extents(const float4* prims, uint32_t n, uint32_t* head, cudaStream_t st) {
+  if (!n) return cudaSuccess;
+  const uint32_t blocks = (n + kBlock - 1) / kBlock;
+  k_extents<<<blocks < 1184u ? blocks : 1184u, kBlock, 0, st>>>(prims, n, head);
+  return cudaGetLastError();
+}
+
+float slack(float area) {
+  // 56 * 2^-24 * |e1||e2| / eps_par with the default eps_par of 1e-4
+  const float s = 56.0f * 5.9604645e-8f * area / 1e-4f;
+  return s < pt::kLeastSlack ? pt::kLeastSlack : s > 0.02f ? 0.02f : s;  // NaN: 0.02
+}
+
+}  // namespace wide

@@ -1,0 +1,151 @@
+"""The eight-wide traversal (scenes prepared by the library) against the CPU oracle:
+closest hits of every form a scene and a ray can take, bit for bit.
+
+Every other way through the library traces the same rays with the binary trees
+(kernel 1, step_policy 1, scenes set as raw buffers), so these cases are the ones that
+differ: leaves of one and of many elements, hits at equal distances, transforms far from
+the unit, rays that the wide boxes' arithmetic cannot take.
+"""
+import numpy as np
+import pytest
+
+import oracle
+from pulse_b200 import scenes
+from pulse_b200.layout import Instance, Material, Mesh
+from pulse_b200.tracer import Scene
+
+pytestmark = pytest.mark.gpu
+
+MAT = [Material((0.7, 0.7, 0.7, 1), (0, 0, 0, 1), 0.8, 0.5, 0.0)]
+
+
+def _triangle_mesh(n, seed, size=1.0, spread=0.0):
+    rng = np.random.default_rng(seed)
+    p = (rng.uniform(-spread, spread, (n, 1, 3)) + rng.normal(size=(n, 3, 3)) * size).reshape(-1, 3)
+    return Mesh(p, np.tile([0.0, 1.0, 0.0], (3 * n, 1)), np.zeros((3 * n, 2)), np.arange(3 * n, dtype=np.uint32))
+
+
+def _spheres(n, level, box, seed=0, scale=lambda rng: 1.0):
+    rng = np.random.default_rng(seed)
+    mesh = scenes.displaced_icosphere(level, 0.1, seed, radius=1.5)
+    inst = [Instance(0, 0, scenes.trs(rng.uniform(-box, box, 3), scenes.random_rotation(rng), scale(rng)))
+            for _ in range(n)]
+    return [mesh], inst
+
+
+def _scene(kind):
+    """(meshes, instances, BLAS leaf size, TLAS leaf size, half extent the rays start in)"""
+    eye = np.eye(4)
+    rng = np.random.default_rng(5)
+    if kind == "one_triangle":
+        return [_triangle_mesh(1, 1)], [Instance(0, 0)], 8, 1, 2.0
+    if kind == "one_leaf":
+        return [_triangle_mesh(8, 2, spread=2.0)], [Instance(0, 0)], 8, 1, 3.0
+    if kind == "nine_triangles":
+        return [_triangle_mesh(9, 3, spread=2.0)], [Instance(0, 0), Instance(0, 0, scenes.trs((3, 0, 0)))], 8, 1, 4.0
+    if kind.startswith("leaf"):  # leaf sizes within a reference's range and beyond it
+        return [_triangle_mesh(600, 4, 0.4, 4.0)], [Instance(0, 0)], int(kind[4:]), 1, 5.0
+    if kind == "cornell":
+        d = scenes.cornell()
+        return d.meshes, d.instances, 4, 1, 1.0
+    if kind == "cornell_leaf8":  # instances of several materials in TLAS leaves of up to 4
+        d = scenes.cornell()
+        return d.meshes, d.instances, 8, 4, 1.0
+    if kind == "overlapping":
+        return *_spheres(24, 3, 2.0), 8, 1, 3.0
+    if kind == "many":  # four levels of the wide instance tree
+        return *_spheres(700, 1, 12.0), 4, 1, 12.0
+    if kind == "same_centre":  # TLAS leaves that cannot be split
+        m = [scenes.displaced_icosphere(2, 0.1, 1)]
+        return m, [Instance(0, 0, scenes.trs(scale=(s, s, s))) for s in (1.0, 1.5, 2.0, 2.5)], 8, 1, 3.0
+    if kind == "same_centre_many":  # more than a wide node's eight
+        m = [scenes.displaced_icosphere(1, 0.1, 1)]
+        return m, [Instance(0, 0, scenes.trs(scale=(s, s, s))) for s in np.linspace(1, 3, 20)], 8, 1, 4.0
+    if kind == "duplicates":  # every hit at the same distance as another
+        m, i = _spheres(4, 2, 2.0)
+        m[0].indices = np.concatenate([m[0].indices, m[0].indices])
+        return m, i, 3, 1, 3.0
+    if kind == "coplanar":  # boxes standing on a floor and against each other
+        q = scenes.quad_mesh([(-4, 0, 4), (4, 0, 4), (4, 0, -4), (-4, 0, -4)], (0, 1, 0))
+        i = [Instance(0, 0)] + [Instance(1, 0, scenes.trs((x, 0.5, z))) for x in (-1, 0, 1) for z in (-1, 0, 1)]
+        return [q, scenes.unit_cube()], i, 4, 1, 2.0
+    if kind == "scaled":
+        return *_spheres(20, 2, 4.0, 1, lambda r: r.uniform(0.05, 3.0, 3)), 8, 1, 5.0
+    if kind == "mirrored_sheared":
+        m, i = _spheres(10, 2, 4.0, 2, lambda r: (-1.0, r.uniform(0.3, 2.0), 1.0))
+        for k, x in enumerate(i):
+            s = eye.copy()
+            s[0, 1] = 0.4 * k
+            x.object_world = np.asarray(x.object_world) @ s
+        return m, i, 8, 1, 5.0
+    if kind == "far_away":
+        m, i = _spheres(10, 3, 4.0, 3)
+        for x in i:
+            x.object_world = scenes.trs((2e4, -1e4, 3e4)) @ np.asarray(x.object_world)
+        return m, i, 8, 1, 5.0
+    if kind == "tiny":
+        return *_spheres(10, 2, 0.02, 4, lambda r: 0.01), 8, 1, 0.03
+    if kind == "huge":
+        return *_spheres(10, 2, 4e3, 5, lambda r: 1e3), 8, 1, 5e3
+    if kind == "large_triangles":  # the test's rounding exceeds a small slack
+        return [_triangle_mesh(300, 6, 30.0, 60.0), _triangle_mesh(300, 7, 0.3, 40.0)], \
+            [Instance(0, 0), Instance(1, 0)], 8, 1, 60.0
+    if kind == "singular":  # no inverse: the scene keeps the binary trees
+        return *_spheres(6, 2, 2.0, 6, lambda r: (1.0, 0.0, 1.0)), 8, 1, 3.0
+    if kind == "projective":
+        m, i = _spheres(6, 2, 2.0, 7)
+        for x in i:
+            x.object_world = np.asarray(x.object_world).copy()
+            x.object_world[3] = (0.01, 0.0, 0.02, 1.0)
+        return m, i, 8, 1, 3.0
+    if kind == "flat_grid":  # boxes without thickness, rays along their planes
+        v = scenes.fbm_grid(24, 8.0, 0.0, 1)
+        return [v], [Instance(0, 0), Instance(0, 0, scenes.trs((0, 1, 0), scenes.rot_y(rng.uniform())))], 2, 1, 4.0
+    raise ValueError(kind)
+
+
+def _rays(half, centre, seed):
+    rng = np.random.default_rng(seed)
+    n = 6000
+    o = centre + rng.uniform(-1.3, 1.3, (n, 3)) * half
+    d = rng.normal(size=(n, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    d[:900] = np.eye(3)[rng.integers(0, 3, 900)] * rng.choice([-1.0, 1.0], (900, 1))  # along axes
+    d[900:1500, 1] = 0.0                                                              # in a plane
+    d[900:1500] /= np.maximum(np.linalg.norm(d[900:1500], axis=1, keepdims=True), 1e-3)
+    o[1500:2100] = np.round(o[1500:2100] / half * 4) / 4 * half                       # on planes of the scene
+    o[2100:2300] += 50.0 * half                                                       # from far away
+    d[2100:2300] = centre - o[2100:2300] + rng.normal(size=(200, 3)) * half
+    d[2100:2300] /= np.linalg.norm(d[2100:2300], axis=1, keepdims=True)
+    d[2300:2400] *= rng.uniform(0.1, 10.0, (100, 1))                                  # not normalized
+    d[2400:2420] = 0.0
+    d[2420:2430, 0] = np.nan
+    o[2430:2440, 1] = np.inf
+    o[2440:2450] = 3e9
+    return np.concatenate([o, d], 1).astype(np.float32)
+
+
+KINDS = ["one_triangle", "one_leaf", "nine_triangles", "leaf1", "leaf2", "leaf63", "leaf64", "leaf100", "cornell",
+         "cornell_leaf8", "overlapping", "many", "same_centre", "same_centre_many", "duplicates", "coplanar", "scaled",
+         "mirrored_sheared", "far_away", "tiny", "huge", "large_triangles", "singular", "projective", "flat_grid"]
+
+
+@pytest.mark.parametrize("quirks", [1, 0])
+@pytest.mark.parametrize("kind", KINDS)
+def test_hits_equal_the_oracle(ctx, kind, quirks):
+    meshes, instances, leaf, tlas_leaf, half = _scene(kind)
+    sb = oracle.assemble(meshes, MAT * 8, instances, 20, leaf, 2, tlas_leaf)
+    centre = np.array([2e4, -1e4, 3e4]) if kind == "far_away" else np.zeros(3)
+    rays = _rays(half, centre, 11)
+    ref = oracle.trace(sb, rays, quirks=quirks)
+    sc = Scene(ctx)
+    ids = [sc.upload_mesh(m, 20, leaf) for m in meshes]
+    sc.set_materials(MAT * 8)
+    sc.set_instances(instances, ids, 2, tlas_leaf)
+    got = sc.trace(rays, quirks=quirks)
+    sc.close()
+    assert np.array_equal(got["t"].view(np.uint32), ref["t"].view(np.uint32))
+    for a, b in (("instance_index", "instance"), ("triangle_index", "triangle")):
+        assert np.array_equal(got[a], ref[b])
+    for k in "uv":
+        assert np.array_equal(got[k].view(np.uint32), ref[k].view(np.uint32))
