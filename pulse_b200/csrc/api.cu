@@ -107,7 +107,7 @@ struct MeshRec {
   DevBuf prims, tdata, nodes, idx;
   // The eight-wide tree (wide.cuh): nodes, leaf node of every slot, and what a
   // collapse reported.
-  DevBuf wide, leaf_of;
+  DevBuf wide, leaf_of, hull;
   bool wide_ok = false;
   uint32_t wide_count = 0, wide_root = 0, wide_levels = 0;
   float wide_slack = 0.0f;
@@ -122,9 +122,9 @@ struct PulseScene {
       materials, strength_cdf, tri_cdfs, mesh_areas, light_indices;
   // Derived layouts.
   DevBuf inst_light, tri_bvh;
-  DevBuf wide_blas, leaf_of;                      // of every mesh, concatenated
+  DevBuf wide_blas, leaf_of, hulls;               // of every mesh, concatenated
   DevBuf wide_tlas, wide_thead, inst_wide;  // of the instances (pt_wide.cuh)
-  DevBuf wide_queue;                              // scratch of the instance tree's collapse
+  DevBuf wide_queue, wide_box, wide_bounds;       // scratch of the instance tree's collapse
   std::vector<uint32_t> mesh_wide;                // per mesh id: first wide node in wide_blas
   uint64_t wide_nodes = 0;                        // rows of wide_blas
   bool tri_bvh_current = false;  // tri_bvh gathered from the current primitives and triangle_indices
@@ -220,7 +220,7 @@ struct PulseScene {
   }
   void free_all() {
     for (DevBuf* b : bind_group()) free_buf(*b);
-    for (DevBuf* b : {&inst_light, &tri_bvh, &wide_blas, &leaf_of, &wide_tlas, &wide_thead, &inst_wide})
+    for (DevBuf* b : {&inst_light, &tri_bvh, &wide_blas, &leaf_of, &hulls, &wide_tlas, &wide_thead, &inst_wide})
       free_buf(*b);
     dev.wide = 0u;
     tri_bvh_current = false;
@@ -233,7 +233,7 @@ struct PulseScene {
     meshes.clear();
   }
   static void free_mesh(MeshRec& m) {
-    for (DevBuf* x : {&m.prims, &m.tdata, &m.nodes, &m.idx, &m.wide, &m.leaf_of}) free_buf(*x);
+    for (DevBuf* x : {&m.prims, &m.tdata, &m.nodes, &m.idx, &m.wide, &m.leaf_of, &m.hull}) free_buf(*x);
   }
   static void free_buf(DevBuf& b) {
     if (b.p) cudaFree(b.p);
@@ -630,7 +630,7 @@ int32_t pulse_scene_destroy(PulseScene* s) {
   s->free_meshes();
   s->bvh_scratch.release();
   for (DevBuf* x : {&s->tmp_a, &s->tmp_b, &s->tmp_c, &s->tmp_d, &s->prep_ii, &s->prep_lights, &s->prep_slot,
-                    &s->tlas_min, &s->tlas_max, &s->tlas_cent, &s->tlas_meta, &s->wide_queue})
+                    &s->tlas_min, &s->tlas_max, &s->tlas_cent, &s->tlas_meta, &s->wide_queue, &s->wide_box, &s->wide_bounds})
     PulseScene::free_buf(*x);
   if (s->meta_host) cudaFreeHost(s->meta_host);
   if (s->upd_stream) cudaStreamDestroy(s->upd_stream);
@@ -875,6 +875,9 @@ static cudaError_t collapse_mesh(MeshRec& m, cudaStream_t st) {
     const size_t bytes = (size_t)m.wide_count * pt::kWideNodeWords * 4;
     e = ensure(m.wide, bytes);
     if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(m.wide.p, out.p, bytes, cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess) e = ensure(m.hull, wide::kHullBoxes * 32);
+    if (e == cudaSuccess)
+      e = wide::hull((const uint4*)m.wide.p, m.wide_count, (const float4*)m.nodes.p, (float4*)m.hull.p, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     m.wide_ok = e == cudaSuccess;
   }
@@ -1073,6 +1076,8 @@ static cudaError_t concat_meshes(PulseScene* s) {
   if (e == cudaSuccess) e = ensure(s->blas_nodes, nn * 32);
   if (e == cudaSuccess) e = ensure(s->wide_blas, nw * wide_bytes);
   if (e == cudaSuccess) e = ensure(s->leaf_of, nt * 4);
+  const size_t hull_bytes = wide::kHullBoxes * 32;
+  if (e == cudaSuccess) e = ensure(s->hulls, s->meshes.size() * hull_bytes);  // by mesh id
   for (const MeshRec& m : s->meshes) {
     if (!m.alive || e != cudaSuccess) continue;
     const auto& t = s->mesh_table[m.id];
@@ -1081,6 +1086,8 @@ static cudaError_t concat_meshes(PulseScene* s) {
     if (e == cudaSuccess) e = cudaMemcpyAsync((char*)s->triangle_indices.p + (size_t)t[2] * 4, m.idx.p, (size_t)m.ntris * 4, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync((char*)s->blas_nodes.p + (size_t)t[3] * 32, m.nodes.p, (size_t)m.node_count * 32, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync((char*)s->leaf_of.p + (size_t)t[2] * 4, m.leaf_of.p, (size_t)m.ntris * 4, cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess && m.wide_ok)
+      e = cudaMemcpyAsync((char*)s->hulls.p + m.id * hull_bytes, m.hull.p, hull_bytes, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess && m.wide_count)
       e = wide::relocate((const uint32_t*)m.wide.p, m.wide_count, s->mesh_wide[m.id], t[2],
                          (uint32_t*)s->wide_blas.p + (size_t)s->mesh_wide[m.id] * pt::kWideNodeWords, st);
@@ -1111,11 +1118,16 @@ static cudaError_t collapse_tlas(PulseScene* s, uint32_t n, const uint32_t* meta
   cudaError_t e = ensure(s->wide_tlas, cap * pt::kWideNodeWords * 4);
   if (e == cudaSuccess) e = ensure(s->wide_thead, wide::kHeadWords * 4);
   if (e == cudaSuccess) e = ensure(s->wide_queue, cap * 4);
+  if (e == cudaSuccess) e = ensure(s->wide_box, cap * 32);
+  if (e == cudaSuccess) e = ensure(s->wide_bounds, (size_t)n * 32);
+  if (e == cudaSuccess)
+    e = prep::tight_bounds(n, (const float4*)s->instances.p, (const float4*)s->inst_wide.p,
+                           (const float*)s->inst_bounds.p, (const float4*)s->hulls.p, (float4*)s->wide_bounds.p, st);
   if (e != cudaSuccess) return e;
-  s->ctx->stats.kernel_launches += 1;
+  s->ctx->stats.kernel_launches += 2;
   return wide::collapse_tlas((const float4*)s->tlas_nodes.p, n_nodes, meta, (const uint32_t*)s->instance_indices.p,
-                             (float4*)s->inst_wide.p, (uint4*)s->wide_tlas.p, (uint32_t*)s->wide_queue.p,
-                             (uint32_t*)s->wide_thead.p, st);
+                             (float4*)s->inst_wide.p, (const float4*)s->wide_bounds.p, (float4*)s->wide_box.p,
+                             (uint4*)s->wide_tlas.p, (uint32_t*)s->wide_queue.p, (uint32_t*)s->wide_thead.p, st);
 }
 
 static int32_t rebuild_tlas(PulseScene* s, uint32_t n, const PulseBvhParams* tp, uint32_t* count, uint32_t* levels,
@@ -1271,6 +1283,7 @@ int32_t pulse_instances_set(PulseScene* s, const PulseInstanceDesc* inst, uint32
     const MeshRec& mesh = s->meshes[d.mesh_id];
     ii[i].wide_root = mesh.wide_root ? 0u : s->mesh_wide[d.mesh_id] | (1u << 24);
     ii[i].wide_slack = mesh.wide_slack;
+    ii[i].hull = d.mesh_id;
     ii[i].wide_leaf = mesh.wide_root ? mesh.wide_root + t[2] : 0u;
     const float* em = s->host_materials[d.material_index].emissive;
     const float len = std::sqrt(em[0] * em[0] + em[1] * em[1] + em[2] * em[2]);

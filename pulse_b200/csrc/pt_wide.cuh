@@ -83,7 +83,7 @@ constexpr uint32_t kTopStack = 16, kTopStackDeep = 24;  // entries for trees of 
 // fullest one nearly always fills the warp, where one ray per lane in
 // registers left 11 to 15 lanes active per instruction (1080p sphere frame, first
 // extend: see k_wide_extend).
-constexpr uint32_t kPool = 64;
+constexpr uint32_t kPool = 64;  // slots laid out; kPool - 1 are used (six-bit counts)
 
 // An instance's record for entering it (DevScene::inst_wide), 96 bytes: its
 // world-to-object matrix, (root group of the mesh's tree, or 0 and its only leaf's reference,
@@ -108,7 +108,8 @@ enum WideWord : uint32_t {
 constexpr uint32_t kInstBits = 17, kInstMask = (1u << kInstBits) - 1u;
 // Action classes of a slot.  kwShade: the kernel's own step.
 enum WideAct : uint32_t {
-  kwNode = 0, kwTriangles = 1, kwInstance = 2, kwTop = 3, kwVerify = 4, kwRedo = 5, kwShade = 6, kwEmpty = 7, kwDone = 8
+  kwNode = 0, kwTriangles = 1, kwInstance = 2, kwTop = 3, kwVerify = 4, kwRedo = 5, kwShade = 6, kwEmpty = 7, kwDone = 8,
+  kwUnused = 9
 };
 
 // Words of a warp's pool: the rays with their stacks, the slots' classes and the step's list.
@@ -379,28 +380,44 @@ __device__ __forceinline__ float wide_candidate(float3 o, float3 d, float gate, 
   return may ? t : 1e30f;
 }
 
-// The next two triangles of the current leaf.
+// The next triangles of the current leaf: kTrisPerVisit, or two when no ray of the step has
+// more left.  Leaves hold 5.8 triangles on average (BLAS leaf size 8): the 1080p sphere
+// frame took 10.9 ms with two a step, 10.2 with three, 10.0 with four.
+constexpr uint32_t kTrisPerVisit = 4;
 __device__ __forceinline__ uint32_t wide_tri(const WideRay& R, const DevScene& S, const TraceCfg& cfg) {
   const uint32_t cur = R.u(kwCur);
   const uint32_t first = cur & kWideFirstMask, left = cur >> kWideFirstBits;
+  const bool more = __any_sync(__activemask(), left > 2u);
   const float4* tp = S.tri_bvh + (size_t)first * 3;
-  const float4* tq = left > 1u ? tp + 3 : tp;
-  const float4 g0 = __ldg(tp), g1 = __ldg(tp + 1), g2 = __ldg(tp + 2);
-  const float4 k0 = __ldg(tq), k1 = __ldg(tq + 1), k2 = __ldg(tq + 2);
+  float4 g[kTrisPerVisit][3];
+#pragma unroll
+  for (uint32_t k = 0; k < kTrisPerVisit; ++k)
+    if (k < 2u || more) {
+      const float4* tq = k < left ? tp + 3 * k : tp;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) g[k][j] = __ldg(tq + j);
+    }
   const float3 o = R.f3(kwOX), d = R.f3(kwDX);
   const float len = R.f(kwLen), best = R.f(kwRecT), eps = R.f(kwEps);
   const float gate = best < 1e30f ? wide_gate(best, eps) * len : 1e30f;
-  const float ta = wide_candidate(o, d, gate, g0, g1, g2, cfg);
-  float tb = wide_candidate(o, d, gate, k0, k1, k2, cfg);
-  if (left <= 1u) tb = 1e30f;
-  if (fminf(ta, tb) < 1e30f) {
+  float ta = 1e30f, tb = 1e30f;  // the nearest candidate and the second
+  uint32_t ka = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < kTrisPerVisit; ++k)
+    if (k < 2u || more) {
+      const float x = wide_candidate(o, d, gate, g[k][0], g[k][1], g[k][2], cfg);
+      const float t = k < left ? x : 1e30f;
+      tb = fminf(tb, fmaxf(ta, t));
+      ka = t < ta ? k : ka;
+      ta = fminf(ta, t);
+    }
+  if (ta < 1e30f) {
     const float scale = __fdividef(1.0f, len);
-    const float wa = ta < 1e30f ? ta * scale : 1e30f, wb = tb < 1e30f ? tb * scale : 1e30f;
-    const float w = fminf(wa, wb);
-    const uint32_t spx = R.u(kwSp), slot = first + (wa <= wb ? 0u : 1u);
+    const float w = ta * scale;
+    const uint32_t spx = R.u(kwSp), slot = first + ka;
     const bool decided = w < R.f(kwExit);  // an occlusion query's light is hidden, if this hit is verified
-    // the nearest of the three and the second: ambiguous within the nearest's gate
-    const float second = fminf(fmaxf(w, best), fmaxf(wa, wb)), M = wide_gate(fminf(w, best), eps);
+    // the nearest of all and the second: ambiguous within the nearest's gate
+    const float second = fminf(fmaxf(w, best), tb < 1e30f ? tb * scale : 1e30f), M = wide_gate(fminf(w, best), eps);
     if (!decided && second <= M) return kwRedo;
     if (w < best) {
       R.setf(kwRecT, w);
@@ -410,8 +427,9 @@ __device__ __forceinline__ uint32_t wide_tri(const WideRay& R, const DevScene& S
     }
     if (decided) return kwVerify;
   }
-  if (left > 2u) {
-    R.set(kwCur, cur + 2u - (2u << kWideFirstBits));
+  const uint32_t done = more ? kTrisPerVisit : 2u;
+  if (left > done) {
+    R.set(kwCur, cur + done - (done << kWideFirstBits));
     return kwTriangles;
   }
   uint32_t grp = R.u(kwGrp);
@@ -554,10 +572,10 @@ __device__ __forceinline__ void wide_run(Item& it, const TraceCfg& tc, uint32_t*
   const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
   uint8_t* cls = reinterpret_cast<uint8_t*>(pool + (kWideWords + tc.stack_w) * kPool);
   uint8_t* list = cls + kPool;
-  reinterpret_cast<uint16_t*>(cls)[lane] = (uint16_t)(kwEmpty | (kwEmpty << 8));
+  reinterpret_cast<uint16_t*>(cls)[lane] = (uint16_t)(kwEmpty | ((lane < 31u ? kwEmpty : kwUnused) << 8));
   __syncwarp();
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-  const uint32_t share = min(kPool, (n_items + warps - 1u) / warps);  // of the first, fixed items
+  const uint32_t share = min(kPool - 1u, (n_items + warps - 1u) / warps);  // of the first, fixed items
   uint32_t at = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * share;
   uint32_t end = min(at + share, n_items);
   at = min(at, end);
@@ -565,30 +583,26 @@ __device__ __forceinline__ void wide_run(Item& it, const TraceCfg& tc, uint32_t*
   while (true) {
     const uint32_t two = reinterpret_cast<const uint16_t*>(cls)[lane];
     const uint32_t c0 = two & 0xffu, c1 = two >> 8;
-    // slots per class, 7 bits each
+    // slots per class, six bits each for the first five
     const uint32_t packed =
-        __reduce_add_sync(0xffffffffu, (c0 < 4u ? 1u << (7u * c0) : 0u) + (c1 < 4u ? 1u << (7u * c1) : 0u));
-    const uint32_t nn = packed & 127u, nt = (packed >> 7) & 127u, ni = (packed >> 14) & 127u, nu = packed >> 21;
-    const uint32_t nv = __popc(__ballot_sync(0xffffffffu, c0 == kwVerify)) + __popc(__ballot_sync(0xffffffffu, c1 == kwVerify));
-    const uint32_t nr = __popc(__ballot_sync(0xffffffffu, c0 == kwRedo)) + __popc(__ballot_sync(0xffffffffu, c1 == kwRedo));
-    uint32_t empty = kPool - nn - nt - ni - nu - nv - nr;
-    uint32_t act = kwNode, most = min(nn, 32u);
-    if (min(nt, 32u) > most) { act = kwTriangles; most = min(nt, 32u); }
-    if (min(ni, 32u) > most) { act = kwInstance; most = min(ni, 32u); }
-    if (min(nu, 32u) > most) { act = kwTop; most = min(nu, 32u); }
-    if (min(nv, 32u) > most) { act = kwVerify; most = min(nv, 32u); }
-    if (Item::kShades) {
-      const uint32_t ns = __popc(__ballot_sync(0xffffffffu, c0 == kwShade)) + __popc(__ballot_sync(0xffffffffu, c1 == kwShade));
-      empty -= ns;
-      if (min(ns, 32u) > most) { act = kwShade; most = min(ns, 32u); }
+        __reduce_add_sync(0xffffffffu, (c0 < 5u ? 1u << (6u * c0) : 0u) + (c1 < 5u ? 1u << (6u * c1) : 0u));
+    // the fullest: count << 3 | class
+    const uint32_t kn = (packed & 63u) << 3, kt = ((packed >> 3) & 0x1f8u) | 1u, ki = ((packed >> 9) & 0x1f8u) | 2u;
+    const uint32_t ku = ((packed >> 15) & 0x1f8u) | 3u, kv = ((packed >> 21) & 0x1f8u) | 4u;
+    uint32_t key = max(max(max(kn, kt), max(ki, ku)), kv);
+    const uint32_t rest = kPool - 1u - (kn >> 3) - (kt >> 3) - (ki >> 3) - (ku >> 3) - (kv >> 3);
+    if (Item::kShades || rest >= kFetchAt || key < 8u) {
+      const uint32_t nr = __popc(__ballot_sync(0xffffffffu, c0 == kwRedo)) + __popc(__ballot_sync(0xffffffffu, c1 == kwRedo));
+      uint32_t ns = 0u;
+      if (Item::kShades) {
+        ns = __popc(__ballot_sync(0xffffffffu, c0 == kwShade)) + __popc(__ballot_sync(0xffffffffu, c1 == kwShade));
+        key = max(key, (ns << 3) | kwShade);
+      }
+      if (!drained && (rest - nr - ns >= kFetchAt || key < 8u)) key = kwEmpty;
+      else if (nr >= kRedoAt || (key < 8u && nr)) key = kwRedo;
+      else if (key < 8u) break;
     }
-    if (!drained && (empty >= kFetchAt || most == 0u)) {
-      act = kwEmpty;
-    } else if (nr >= kRedoAt || (most == 0u && nr)) {
-      act = kwRedo;
-    } else if (most == 0u) {
-      break;
-    }
+    const uint32_t act = key & 7u;
     const uint32_t b0 = __ballot_sync(0xffffffffu, c0 == act), b1 = __ballot_sync(0xffffffffu, c1 == act);
     const uint32_t n0 = __popc(b0);
     uint32_t n = min(n0 + __popc(b1), 32u);

@@ -86,7 +86,7 @@ __global__ void k_instances(const InstanceIn* __restrict__ in, uint32_t n, const
   // the wide traversal's record (pt_wide.cuh); its TLAS leaf comes with the tree
   float4* wo = wide_out + (size_t)i * kWideInstRows;
   for (int c = 0; c < 4; ++c) wo[c] = make_float4(inv[4 * c], inv[4 * c + 1], inv[4 * c + 2], inv[4 * c + 3]);
-  wo[4] = make_float4(__uint_as_float(x.wide_root), __uint_as_float(x.wide_leaf), x.wide_slack, 0.0f);
+  wo[4] = make_float4(__uint_as_float(x.wide_root), __uint_as_float(x.wide_leaf), x.wide_slack, __uint_as_float(x.hull));
   wo[5] = make_float4(__uint_as_float(x.index_offset), __uint_as_float(x.node_offset),
                       __uint_as_float(kWideRootLeaf), 0.0f);
   // World bounds of the root box (src/scene/mod.rs:625-658).
@@ -104,6 +104,55 @@ __global__ void k_instances(const InstanceIn* __restrict__ in, uint32_t n, const
   b[0] = wmin.x; b[1] = wmin.y; b[2] = wmin.z;
   b[3] = wmax.x; b[4] = wmax.y; b[5] = wmax.z;
   b[6] = center.x; b[7] = center.y; b[8] = center.z;
+}
+
+// One warp per instance, two hull boxes per lane.  A rotated mesh fills about half the
+// cross-section of the box around its root box's corners: the rays of the 1080p sphere
+// frame enter 4.5 instances instead of 6.9 (frame 11.9 -> 10.9 ms).
+// The bounds are widened by four roundings of the transform's and the ray's coordinates
+// times their amplification (the product of the matrix's and its inverse's largest
+// entries); where that exceeds 8 the reference's bounds stay.
+__global__ void __launch_bounds__(256) k_tight_bounds(uint32_t n, const float4* __restrict__ instances,
+                                                      const float4* __restrict__ inst_wide,
+                                                      const float* __restrict__ bounds9,
+                                                      const float4* __restrict__ hulls, float4* out) {
+  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+  if (i >= n) return;
+  const M4 m = load_m4(instances + (size_t)i * 10), w = load_m4(instances + (size_t)i * 10 + 4);
+  const float4* h = hulls + (size_t)__float_as_uint(__ldg(inst_wide + (size_t)i * kWideInstRows + 4).w) * 128;
+  float3 lo = v3(3e38f, 3e38f, 3e38f), hi = v3(-3e38f, -3e38f, -3e38f);
+  for (uint32_t k = lane; k < 64u; k += 32u) {
+    const float4 a = __ldg(h + 2 * k), z = __ldg(h + 2 * k + 1);
+    if (!(a.x <= z.x)) continue;
+    for (int c = 0; c < 8; ++c) {
+      const float3 p = transform_position(m, v3(c & 1 ? z.x : a.x, c & 2 ? z.y : a.y, c & 4 ? z.z : a.z));
+      lo = v3(fminf(lo.x, p.x), fminf(lo.y, p.y), fminf(lo.z, p.z));
+      hi = v3(fmaxf(hi.x, p.x), fmaxf(hi.y, p.y), fmaxf(hi.z, p.z));
+    }
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    lo = v3(fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, off)), fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, off)),
+            fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, off)));
+    hi = v3(fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, off)), fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, off)),
+            fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, off)));
+  }
+  if (lane != 0u) return;
+  const float* b = bounds9 + (size_t)i * 9;
+  float l[3] = {b[0], b[1], b[2]}, u[3] = {b[3], b[4], b[5]};
+  auto entry = [](const M4& x) {
+    return fmaxf(fmaxf(max_abs3(xyz(x.c0)), max_abs3(xyz(x.c1))), max_abs3(xyz(x.c2)));
+  };
+  const float amp = entry(m) * entry(w);
+  if (amp <= 8.0f) {
+    const float tl[3] = {lo.x, lo.y, lo.z}, tu[3] = {hi.x, hi.y, hi.z};
+    const float pad = 4e-6f * fmaxf(amp, 1.0f) * (fmaxf(max_abs3(lo), max_abs3(hi)) + max_abs3(sub(hi, lo)));
+    for (int k = 0; k < 3; ++k) {
+      const float x = fmaxf(l[k], tl[k] - pad), y = fminf(u[k], tu[k] + pad);
+      if (x <= y) l[k] = x, u[k] = y;
+    }
+  }
+  out[2 * (size_t)i] = make_float4(l[0], l[1], l[2], 0.0f);
+  out[2 * (size_t)i + 1] = make_float4(u[0], u[1], u[2], 0.0f);
 }
 
 __global__ void k_light_cdfs(const LightIn* __restrict__ lights, uint32_t n, const float4* __restrict__ prims,
@@ -163,6 +212,13 @@ cudaError_t instances(const InstanceIn* in, uint32_t n, const float4* blas_nodes
                       float4* wide_out, cudaStream_t st, const uint32_t* slot) {
   if (!n) return cudaSuccess;
   k_instances<<<(n + 127) / 128, 128, 0, st>>>(in, n, blas_nodes, inst_out, bounds9, wide_out, slot);
+  return cudaGetLastError();
+}
+
+cudaError_t tight_bounds(uint32_t n, const float4* instances, const float4* inst_wide, const float* bounds9,
+                         const float4* hulls, float4* out, cudaStream_t st) {
+  if (!n) return cudaSuccess;
+  k_tight_bounds<<<(n + 7) / 8, 256, 0, st>>>(n, instances, inst_wide, bounds9, hulls, out);
   return cudaGetLastError();
 }
 

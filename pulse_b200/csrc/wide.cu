@@ -22,10 +22,13 @@ __device__ __forceinline__ float half_area(float4 lo, float4 hi) {
 }
 
 // Where the leaf node of an element goes: an array by slot, or (instances) their records.
+// A TLAS also has the instances' bounds (two float4 each) and room for those of its nodes.
 struct LeafSink {
   uint32_t* by_slot;
   const uint32_t* instance_of;
   float4* records;
+  const float4* bounds;
+  float4* node_box;
   __device__ __forceinline__ void put(uint32_t slot, uint32_t node) const {
     if (by_slot) by_slot[slot] = node;
     else records[(size_t)instance_of[slot] * pt::kWideInstRows + 5].z = __uint_as_float(node);
@@ -46,83 +49,51 @@ __device__ uint32_t leaf_ref(uint32_t first, uint32_t count, uint32_t* head) {
   return (count << pt::kWideFirstBits) | first;
 }
 
-// Up to eight children of one wide node.  A TLAS leaf of several instances is as many
-// children with the same box.
-struct Children {
-  float lo[8][3], hi[8][3];
-  uint32_t node[8], ref[8];  // binary node; a leaf's reference
-  bool leaf[8];
-  uint32_t n = 0;
-};
+// The boxes of a wide node's children, by slot.
+struct Boxes { float lo[8][3], hi[8][3]; };
 
-__device__ void write_node(const Children& c, const float lo[3], const float hi[3], uint4* out, uint32_t* queue,
-                           uint32_t* head) {
-  // slots: interior children sorted along the axis of their centres' largest spread, leaves from 7 down
-  uint32_t inner[8], ni = 0, nl = 0, slot_of[8];
-  float cmin[3] = {3e38f, 3e38f, 3e38f}, cmax[3] = {-3e38f, -3e38f, -3e38f};
-  bool bad = false;
-  for (uint32_t k = 0; k < c.n; ++k) {
-    if (c.leaf[k]) {
-      slot_of[k] = 7u - nl++;
-      continue;
-    }
-    for (int j = 0; j < 3; ++j) {
-      cmin[j] = fminf(cmin[j], c.lo[k][j] + c.hi[k][j]);
-      cmax[j] = fmaxf(cmax[j], c.lo[k][j] + c.hi[k][j]);
-    }
-    inner[ni++] = k;
-  }
-  uint32_t axis = 0;
-  for (uint32_t j = 1; j < 3; ++j)
-    if (cmax[j] - cmin[j] > cmax[axis] - cmin[axis]) axis = j;
-  for (uint32_t i = 1; i < ni; ++i) {  // insertion sort
-    const uint32_t k = inner[i];
-    uint32_t j = i;
-    for (; j > 0 && c.lo[inner[j - 1]][axis] + c.hi[inner[j - 1]][axis] > c.lo[k][axis] + c.hi[k][axis]; --j)
-      inner[j] = inner[j - 1];
-    inner[j] = k;
-  }
-  uint32_t at = 0;
-  if (ni) {
-    at = atomicAdd(head + kCount, ni);
-    if (at + ni >= (1u << pt::kWideIndexBits)) bad = true;
-  }
-  for (uint32_t i = 0; i < ni; ++i) {
-    slot_of[inner[i]] = i;
-    queue[at + i] = c.node[inner[i]];
-  }
-  uint32_t words[pt::kWideNodeWords];
-  for (uint32_t k = 0; k < pt::kWideNodeWords; ++k) words[k] = 0u;
+// The planes of the slots in `used` into the node's words.
+__device__ void quantize(uint32_t* words, const Boxes& c, uint32_t used, uint32_t* head) {
   uint8_t* q8 = reinterpret_cast<uint8_t*>(words + 8);
-  words[3] = (ni << 24) | (nl << 28);
-  words[4] = at | (axis << pt::kWideIndexBits);
+  bool bad = false;
   for (int j = 0; j < 3; ++j) {
+    float lo = 3e38f, hi = -3e38f;
+    for (uint32_t k = 0; k < 8; ++k)
+      if (used & (1u << k)) {
+        if (!(fabsf(c.lo[k][j]) <= 1e9f) || !(fabsf(c.hi[k][j]) <= 1e9f) || !(c.lo[k][j] <= c.hi[k][j])) bad = true;
+        lo = fminf(lo, c.lo[k][j]);
+        hi = fmaxf(hi, c.hi[k][j]);
+      }
+    if (bad) break;
     // quanta: 2^e with the children's extent in 254 of them, and large enough
     // against the coordinates for the origin to move by 1/32 of one
-    const double mag = fmax(fabs((double)lo[j]), fabs((double)hi[j]));
-    const double need = fmax(fmax(((double)hi[j] - lo[j]) / 254.0, mag * 7.63e-6), 1e-30);
+    const double mag = fmax(fabs((double)lo), fabs((double)hi));
+    const double need = fmax(fmax(((double)hi - lo) / 254.0, mag * 7.63e-6), 1e-30);
     int e;
     frexp(need, &e);  // need <= 2^e
     const double s = ldexp(1.0, e);
-    const float p = __double2float_rd((double)lo[j] - s / 32.0);
+    const float p = __double2float_rd((double)lo - s / 32.0);
     words[j] = __float_as_uint(p);
     words[3] |= (uint32_t)(e + 127 + 15) << (8 * j);
-    for (uint32_t k = 0; k < c.n; ++k) {
-      const double ql = floor((c.lo[k][j] - (double)p) / s - 1.0 / 64.0), qh = ceil((c.hi[k][j] - (double)p) / s + 1.0 / 64.0);
+    for (uint32_t k = 0; k < 8; ++k) {
+      if (!(used & (1u << k))) continue;
+      const double ql = floor((c.lo[k][j] - (double)p) / s - 1.0 / 64.0);
+      const double qh = ceil((c.hi[k][j] - (double)p) / s + 1.0 / 64.0);
       if (!(ql >= 0.0) || !(qh <= 255.0)) bad = true;
-      q8[16 * j + slot_of[k]] = (uint8_t)ql;
-      q8[16 * j + 8 + slot_of[k]] = (uint8_t)qh;
+      q8[16 * j + k] = (uint8_t)ql;
+      q8[16 * j + 8 + k] = (uint8_t)qh;
     }
   }
-  for (uint32_t k = 0; k < c.n; ++k)
-    if (c.leaf[k]) words[pt::wide_ref_word(7u - slot_of[k])] = c.ref[k];
   if (bad) head[kBad] = 1u;
-  uint32_t* w = reinterpret_cast<uint32_t*>(out);
-  for (uint32_t k = 0; k < pt::kWideNodeWords; ++k) w[k] = words[k];
 }
 
-// The wide node of binary node b (interior).
-__device__ void make_node(const float4* __restrict__ nodes, uint32_t b, uint4* out, const LeafSink& leaf_of,
+__device__ __forceinline__ uint32_t used_slots(uint32_t ni, uint32_t nl) {
+  return ((1u << ni) - 1u) | ((0xff00u >> nl) & 0xffu);
+}
+
+// The wide node of binary node b (interior).  A TLAS leaf of several instances is as
+// many children, and the planes come later (fit_node).
+__device__ void make_node(const float4* __restrict__ nodes, uint32_t b, uint32_t* out, const LeafSink& leaf_of,
                           uint32_t* queue, uint32_t* head) {
   uint32_t c[8], mult[8];  // children; places each takes
   float area[8];           // below 0: not to be opened
@@ -161,57 +132,98 @@ __device__ void make_node(const float4* __restrict__ nodes, uint32_t b, uint4* o
     put((uint32_t)best, a);
     put(n++, a + 1);
   }
-  Children ch;
-  float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
-  bool bad = false;
+  uint32_t words[pt::kWideNodeWords];
+  for (uint32_t k = 0; k < pt::kWideNodeWords; ++k) words[k] = 0u;
+  // slots: interior children sorted along the axis of their centres' largest spread, leaves from 7 down
+  Boxes box;
+  uint32_t inner[8], ni = 0, nl = 0;
+  float mid[8][3], cmin[3] = {3e38f, 3e38f, 3e38f}, cmax[3] = {-3e38f, -3e38f, -3e38f};
+  auto set_box = [&](uint32_t slot, uint32_t node) {
+    const float4 a = nodes[2 * (size_t)node], z = nodes[2 * (size_t)node + 1];
+    box.lo[slot][0] = a.x, box.lo[slot][1] = a.y, box.lo[slot][2] = a.z;
+    box.hi[slot][0] = z.x, box.hi[slot][1] = z.y, box.hi[slot][2] = z.z;
+  };
   for (uint32_t k = 0; k < n; ++k) {
     const float4 a = nodes[2 * (size_t)c[k]], z = nodes[2 * (size_t)c[k] + 1];
-    const float p[3] = {a.x, a.y, a.z}, q[3] = {z.x, z.y, z.z};
     const uint32_t start = __float_as_uint(a.w), count = __float_as_uint(z.w);
-    for (uint32_t i = 0; i < count; ++i) leaf_of.put(start + i, c[k]);
-    for (uint32_t i = 0; i < mult[k]; ++i) {
-      const uint32_t at = ch.n++;
-      ch.node[at] = c[k];
-      ch.leaf[at] = count != 0u;
-      ch.ref[at] = !count ? 0u : tlas ? leaf_of.ref(start + i) : leaf_ref(start, count, head);
-      for (int j = 0; j < 3; ++j) {
-        if (!(fabsf(p[j]) <= 1e9f) || !(fabsf(q[j]) <= 1e9f) || !(p[j] <= q[j])) bad = true;
-        ch.lo[at][j] = p[j];
-        ch.hi[at][j] = q[j];
+    if (count) {
+      for (uint32_t i = 0; i < count; ++i) leaf_of.put(start + i, c[k]);
+      for (uint32_t i = 0; i < mult[k]; ++i) {
+        set_box(7u - nl, c[k]);
+        words[pt::wide_ref_word(nl++)] = tlas ? leaf_of.ref(start + i) : leaf_ref(start, count, head);
       }
+      continue;
     }
+    mid[k][0] = a.x + z.x, mid[k][1] = a.y + z.y, mid[k][2] = a.z + z.z;
     for (int j = 0; j < 3; ++j) {
-      lo[j] = fminf(lo[j], p[j]);
-      hi[j] = fmaxf(hi[j], q[j]);
+      cmin[j] = fminf(cmin[j], mid[k][j]);
+      cmax[j] = fmaxf(cmax[j], mid[k][j]);
+    }
+    inner[ni++] = k;
+  }
+  uint32_t axis = 0;
+  for (uint32_t j = 1; j < 3; ++j)
+    if (cmax[j] - cmin[j] > cmax[axis] - cmin[axis]) axis = j;
+  for (uint32_t i = 1; i < ni; ++i) {  // insertion sort
+    const uint32_t k = inner[i];
+    uint32_t j = i;
+    for (; j > 0 && mid[inner[j - 1]][axis] > mid[k][axis]; --j) inner[j] = inner[j - 1];
+    inner[j] = k;
+  }
+  words[3] = (ni << 24) | (nl << 28);
+  if (ni) {
+    const uint32_t at = atomicAdd(head + kCount, ni);
+    if (at + ni >= (1u << pt::kWideIndexBits)) head[kBad] = 1u;
+    words[4] = at | (axis << pt::kWideIndexBits);
+    for (uint32_t i = 0; i < ni; ++i) {
+      set_box(i, c[inner[i]]);
+      queue[at + i] = c[inner[i]];
     }
   }
-  if (bad) {
-    head[kBad] = 1u;
-    return;
-  }
-  write_node(ch, lo, hi, out, queue, head);
+  if (!tlas) quantize(words, box, used_slots(ni, nl), head);
+  for (uint32_t k = 0; k < pt::kWideNodeWords; ++k) out[k] = words[k];
 }
 
-// A TLAS that is one leaf: a node of its instances with boxes around every ray (the
-// reference enters a root without testing its box).
-__device__ void make_root_leaf(uint32_t start, uint32_t count, uint4* out, const LeafSink& leaf_of, uint32_t* queue,
+// A TLAS that is one leaf: a node of its instances.
+__device__ void make_root_leaf(uint32_t start, uint32_t count, uint32_t* out, const LeafSink& leaf_of,
                                uint32_t* head) {
   if (count > 8) {
     head[kBad] = 1u;
     return;
   }
-  Children ch;
-  const float lo[3] = {-1e12f, -1e12f, -1e12f}, hi[3] = {1e12f, 1e12f, 1e12f};
+  for (uint32_t k = 0; k < pt::kWideNodeWords; ++k) out[k] = 0u;
+  out[3] = count << 28;
   for (uint32_t i = 0; i < count; ++i) {
     leaf_of.put(start + i, pt::kWideRootLeaf);
-    ch.leaf[i] = true;
-    ch.node[i] = 0u;
-    ch.ref[i] = leaf_of.ref(start + i);
-    for (int j = 0; j < 3; ++j) ch.lo[i][j] = lo[j], ch.hi[i][j] = hi[j];
+    out[pt::wide_ref_word(i)] = leaf_of.ref(start + i);
   }
-  ch.n = count;
-  write_node(ch, lo, hi, out, queue, head);
 }
+
+// The planes of TLAS node i from its instances' bounds and its interior children's
+// boxes (made before it), and its own box.
+__device__ void fit_node(uint32_t i, uint32_t* out, const LeafSink& leaf_of, uint32_t* head) {
+  uint32_t* w = out + (size_t)i * pt::kWideNodeWords;
+  const uint32_t ni = (w[3] >> 24) & 15u, nl = w[3] >> 28, used = used_slots(ni, nl);
+  Boxes box;
+  float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
+  for (uint32_t k = 0; k < 8; ++k) {
+    if (!(used & (1u << k))) continue;
+    const float4* b = k < ni ? leaf_of.node_box + 2 * (size_t)((w[4] & pt::kWideIndexMask) + k)
+                             : leaf_of.bounds + 2 * (size_t)(w[pt::wide_ref_word(7u - k)] & ~pt::kLooseRef);
+    const float4 a = __ldcg(b), z = __ldcg(b + 1);
+    box.lo[k][0] = a.x, box.lo[k][1] = a.y, box.lo[k][2] = a.z;
+    box.hi[k][0] = z.x, box.hi[k][1] = z.y, box.hi[k][2] = z.z;
+    for (int j = 0; j < 3; ++j) {
+      lo[j] = fminf(lo[j], box.lo[k][j]);
+      hi[j] = fmaxf(hi[j], box.hi[k][j]);
+    }
+  }
+  leaf_of.node_box[2 * (size_t)i] = make_float4(lo[0], lo[1], lo[2], 0.0f);
+  leaf_of.node_box[2 * (size_t)i + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+  quantize(w, box, used, head);
+}
+
+constexpr uint32_t kMaxLevels = 64;  // of a TLAS whose nodes are fitted
 
 template <bool GRID>
 __global__ void __launch_bounds__(kBlock) k_collapse(const float4* __restrict__ nodes,
@@ -240,25 +252,74 @@ __global__ void __launch_bounds__(kBlock) k_collapse(const float4* __restrict__ 
     head[kRoot] = count && !tlas ? leaf_ref(start, count, head) : 0u;
     queue[0] = 0u;
     *(volatile uint32_t*)(head + kCount) = count && !tlas ? 0u : 1u;
-    if (count && tlas) make_root_leaf(start, count, out, leaf_of, queue, head);
-    else
+    if (count && tlas) {
+      make_root_leaf(start, count, reinterpret_cast<uint32_t*>(out), leaf_of, head);
+      if (count <= 8) fit_node(0u, reinterpret_cast<uint32_t*>(out), leaf_of, head);
+    } else {
       for (uint32_t i = 0; i < count; ++i) leaf_of.put(start + i, pt::kWideRootLeaf);
+    }
   }
   if (count) return;  // the tree is one leaf
+  __shared__ uint32_t level_at[kMaxLevels + 1];  // (each block its own: the same values)
   sync();
   uint32_t begin = 0, levels = 0;
   while (true) {
     const uint32_t end = *(volatile uint32_t*)(head + kCount);
     if (begin == end) break;
+    if (threadIdx.x == 0 && levels < kMaxLevels) level_at[levels] = begin;
     ++levels;
     sync();  // every thread has read the count
     for (uint32_t i = begin + tid; i < end; i += stride)
-      make_node(nodes, *(volatile uint32_t*)(queue + i), out + (size_t)i * (pt::kWideNodeWords / 4), leaf_of, queue,
-                head);
+      make_node(nodes, *(volatile uint32_t*)(queue + i), reinterpret_cast<uint32_t*>(out) + (size_t)i * pt::kWideNodeWords,
+                leaf_of, queue, head);
     sync();
     begin = end;
   }
   if (tid == 0) head[kLevels] = levels;
+  if (!leaf_of.instance_of) return;
+  // TLAS: bottom-up, the deepest level first
+  if (levels >= kMaxLevels || *(volatile uint32_t*)(head + kBad)) {
+    if (tid == 0) head[kBad] = 1u;
+    return;
+  }
+  for (uint32_t l = levels; l-- > 0;) {
+    const uint32_t from = level_at[l], to = l + 1 < levels ? level_at[l + 1] : begin;
+    for (uint32_t i = from + tid; i < to; i += stride) fit_node(i, reinterpret_cast<uint32_t*>(out), leaf_of, head);
+    sync();
+  }
+}
+
+// Boxes around a mesh for its instances' bounds: those of the root's children's
+// children (dequantized; kHullBoxes, unused ones inverted).  One block of 64 threads.
+__global__ void __launch_bounds__(64) k_hull(const uint32_t* __restrict__ wide_nodes, uint32_t n_wide,
+                                             const float4* __restrict__ nodes, float4* hull) {
+  const uint32_t t = threadIdx.x, k = t >> 3, j = t & 7u;
+  float4 lo = make_float4(3e38f, 3e38f, 3e38f, 0.0f), hi = make_float4(-3e38f, -3e38f, -3e38f, 0.0f);
+  auto box_of = [&](uint32_t node, uint32_t slot) {
+    const uint32_t* w = wide_nodes + (size_t)node * pt::kWideNodeWords;
+    const uint8_t* q = reinterpret_cast<const uint8_t*>(w + 8);
+    float l[3], h[3];
+    for (int a = 0; a < 3; ++a) {
+      const float p = __uint_as_float(w[a]), s = ldexpf(1.0f, (int)((w[3] >> (8 * a)) & 255u) - 127 - 15);
+      l[a] = p + q[16 * a + slot] * s;
+      h[a] = p + q[16 * a + 8 + slot] * s;
+    }
+    lo = make_float4(l[0], l[1], l[2], 0.0f);
+    hi = make_float4(h[0], h[1], h[2], 0.0f);
+  };
+  if (n_wide == 0u) {
+    if (t == 0u) lo = nodes[0], hi = nodes[1];
+  } else {
+    const uint32_t h = wide_nodes[3], ni = (h >> 24) & 15u, nl = h >> 28;
+    if (k < ni) {
+      const uint32_t child = (wide_nodes[4] & pt::kWideIndexMask) + k, c = wide_nodes[(size_t)child * pt::kWideNodeWords + 3];
+      if (used_slots((c >> 24) & 15u, c >> 28) & (1u << j)) box_of(child, j);
+    } else if (j == 0u && (used_slots(ni, nl) & (1u << k))) {
+      box_of(0u, k);
+    }
+  }
+  hull[2 * t] = lo;
+  hull[2 * t + 1] = hi;
 }
 
 __global__ void __launch_bounds__(kBlock) k_relocate(const uint32_t* __restrict__ in, uint32_t n, uint32_t node_add,
@@ -313,12 +374,18 @@ cudaError_t launch(const float4* nodes, uint32_t n_nodes, const uint32_t* meta, 
 
 cudaError_t collapse(const float4* nodes, uint32_t n_nodes, uint4* out, uint32_t* leaf_of, uint32_t* queue,
                      uint32_t* head, cudaStream_t st) {
-  return launch(nodes, n_nodes, nullptr, out, LeafSink{leaf_of, nullptr, nullptr}, queue, head, st);
+  return launch(nodes, n_nodes, nullptr, out, LeafSink{leaf_of, nullptr, nullptr, nullptr, nullptr}, queue, head, st);
 }
 
 cudaError_t collapse_tlas(const float4* nodes, uint32_t n_nodes, const uint32_t* meta, const uint32_t* instance_of,
-                          float4* records, uint4* out, uint32_t* queue, uint32_t* head, cudaStream_t st) {
-  return launch(nodes, n_nodes, meta, out, LeafSink{nullptr, instance_of, records}, queue, head, st);
+                          float4* records, const float4* bounds, float4* node_box, uint4* out, uint32_t* queue,
+                          uint32_t* head, cudaStream_t st) {
+  return launch(nodes, n_nodes, meta, out, LeafSink{nullptr, instance_of, records, bounds, node_box}, queue, head, st);
+}
+
+cudaError_t hull(const uint4* wide_nodes, uint32_t n_wide, const float4* nodes, float4* out, cudaStream_t st) {
+  k_hull<<<1, kHullBoxes, 0, st>>>(reinterpret_cast<const uint32_t*>(wide_nodes), n_wide, nodes, out);
+  return cudaGetLastError();
 }
 
 cudaError_t relocate(const uint32_t* nodes, uint32_t n, uint32_t node_add, uint32_t slot_add, uint32_t* out,

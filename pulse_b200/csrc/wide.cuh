@@ -26,10 +26,17 @@ cudaError_t collapse(const float4* nodes, uint32_t n_nodes, uint4* out, uint32_t
                      uint32_t* head, cudaStream_t st);
 
 // The same for an instance tree, whose elements' leaf nodes go into the instances'
-// records (pt_wide.cuh).  meta: the words of a bvh::build_direct queued before (kBad and
-// nothing read if it failed), or nullptr.
+// records (pt_wide.cuh) and whose boxes are those of the instances' own bounds (two float4
+// each; node_box: scratch of two float4 per node).  meta: the words of a
+// bvh::build_direct queued before (kBad and nothing read if it failed), or nullptr.
 cudaError_t collapse_tlas(const float4* nodes, uint32_t n_nodes, const uint32_t* meta, const uint32_t* instance_of,
-                          float4* records, uint4* out, uint32_t* queue, uint32_t* head, cudaStream_t st);
+                          float4* records, const float4* bounds, float4* node_box, uint4* out, uint32_t* queue,
+                          uint32_t* head, cudaStream_t st);
+
+// kHullBoxes boxes (two float4 each; unused ones inverted) that hold a mesh, from its
+// collapsed tree (n_wide 0: its only node's box).
+constexpr uint32_t kHullBoxes = 64;
+cudaError_t hull(const uint4* wide_nodes, uint32_t n_wide, const float4* nodes, float4* out, cudaStream_t st);
 
 // A mesh's n nodes with their indexes moved by node_add and their triangle slots by
 // slot_add, as they go into the scene's array.
