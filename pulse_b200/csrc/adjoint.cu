@@ -323,7 +323,7 @@ cudaError_t launch_backward(const DevScene& S, const TraceCfg& tc, const PathCfg
   int qi = 0;
   for (uint32_t seg = 0; seg < pc.max_depth; ++seg) {
     if ((e = wf_reset_step(B, qi ^ 1, st)) != cudaSuccess) return e;
-    if ((e = wf_extend_step(tc, B, qi, trace_blocks, wide, ctr, st)) != cudaSuccess) return e;
+    if ((e = wf_extend_step(tc, B, qi, trace_blocks, wide ? &one : nullptr, ctr, st)) != cudaSuccess) return e;
     k_adj_shade<<<light_blocks, kAdjBlock, smem_g, st>>>(S, pc, B, rec, dimg, qi, grads, n_mat);
     if (wide) wide_adj_shadow(tc, S, B, rec, kRec, kVisible, trace_blocks, ctr, st);
     else k_adj_shadow<<<trace_grid, kAdjBlock, smem_t, st>>>(S, tc, B, rec, ctr);

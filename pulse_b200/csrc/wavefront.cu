@@ -782,12 +782,13 @@ cudaError_t wf_upload_table(const WfScene* host, uint32_t n, WfScene* dev, cudaS
   return cudaGetLastError();
 }
 
-cudaError_t wf_extend_step(const TraceCfg& tc, const WfBuffers& B, int qi, uint32_t trace_blocks, bool wide,
+cudaError_t wf_extend_step(const TraceCfg& tc, const WfBuffers& B, int qi, uint32_t trace_blocks, const WfScene* wide,
                            Counters* ctr, cudaStream_t st) {
   if (cudaError_t e = wf_prepare(2)) return e;
   if (wide) {
     WfLaunch L{};
     L.n_scenes = 1;
+    L.one = wide;
     L.trace_blocks_per_sm = trace_blocks;
     L.sms = device_sms();
     wide_extend(-1, tc, B, L, qi, ctr, st);
@@ -825,6 +826,7 @@ cudaError_t wf_gbuffer_primary(const TraceCfg& tc, const WfScene& scene, float4*
   if (wide_allowed(tcs, one.S)) {
     WfLaunch L{};
     L.n_scenes = 1;
+    L.one = &one;
     L.trace_blocks_per_sm = trace_blocks;
     L.sms = sms;
     wide_extend(-1, tcs, B, L, 0, ctr, st);
@@ -856,6 +858,7 @@ cudaError_t wf_render_gi(const TraceCfg& tc, const WfScene& scene, const float4*
   trace_stacks(tcs, one.S.tlas_levels, one.S.blas_levels, one.S.wide_stack,
                one.S.wide_top);
   L.wide = wide_allowed(tcs, one.S);
+  L.one = &one;
   if (L.wide && !wf_segments) L.wf_segments = kDefaultWideSegments;
   cudaError_t e = wf_upload_table(&one, 1, B.table, st);
   if (e != cudaSuccess) return e;
@@ -895,6 +898,7 @@ cudaError_t wf_render(int mode, const TraceCfg& tc, const WfScene* scenes, uint3
   }
   TraceCfg tcs = tc;
   trace_stacks(tcs, tl, bl, wl + wt, wt);
+  if (n == 1) L.one = tab;
   L.wide = true;  // one scene that cannot keeps the batch on the binary traversal
   for (uint32_t i = 0; i < n; ++i) L.wide = L.wide && wide_allowed(tcs, tab[i].S);
   if (L.wide && !wf_segments) L.wf_segments = kDefaultWideSegments;

@@ -60,6 +60,7 @@ struct WfLaunch {
   uint32_t trace_blocks_per_sm;  // 0 = kDefaultTraceBlocks
   int sms;
   bool wide = false;             // every scene's rays take the eight-wide traversal
+  const WfScene* one = nullptr;  // the scene of a launch over one (host memory, while recording)
   cudaEvent_t image_wait = nullptr;  // awaited before the accumulation writes the images
 };
 
@@ -132,8 +133,8 @@ cudaError_t wf_render_gi(const TraceCfg& tc, const WfScene& scene, const float4*
 // wf_render with B (its one-scene table): the closest hit of every path of
 // queue qi into B.h0/h1, and the reset of the counters before a segment whose
 // next queue is `next`.
-// wide: with the eight-wide traversal.
-cudaError_t wf_extend_step(const TraceCfg& tc, const WfBuffers& B, int qi, uint32_t trace_blocks, bool wide,
+// wide: the scene, to take the eight-wide traversal, or nullptr.
+cudaError_t wf_extend_step(const TraceCfg& tc, const WfBuffers& B, int qi, uint32_t trace_blocks, const WfScene* wide,
                            Counters* ctr, cudaStream_t st);
 cudaError_t wf_reset_step(const WfBuffers& B, int next, cudaStream_t st);
 

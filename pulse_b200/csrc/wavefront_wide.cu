@@ -20,25 +20,37 @@ using namespace wf;
 // leave some 60 KB of L1.
 constexpr int kWideBlocks = 4;
 
+// The scenes of a launch: one, in the kernel's parameters (ONE: reading its pointers from
+// constant memory took 2% off the 1080p frames), or the table in shared memory.
+template <bool ONE>
+struct Scenes {
+  const WfScene& one;
+  const WfScene* tab;
+  uint32_t n;
+  __device__ __forceinline__ const WfScene& at(uint32_t i) const { return ONE ? one : tab[i]; }
+  __device__ __forceinline__ const WfScene& of(const WideRay& R) const { return ONE ? one : tab[R.u(kwRecInst) >> 20]; }
+  __device__ __forceinline__ uint32_t of_path(uint32_t p) const { return ONE ? 0u : scene_of(tab, n, p); }
+};
+
 // Paths of a queue and, with SHADOW >= 0 (the estimator mode), after them the previous
 // segment's shadow requests.
-template <int SHADOW>
+template <int SHADOW, bool ONE>
 struct ExtendItem {
-  const WfScene* tab;
+  Scenes<ONE> sc;
   const WfBuffers& B;
   const TraceCfg& tc;
   const uint32_t* q;
-  uint32_t n_scenes, n;
-  __device__ __forceinline__ const DevScene& scene(const WideRay& R) const { return tab[R.u(kwRecInst) >> 20].S; }
+  uint32_t n;
+  __device__ __forceinline__ const DevScene& scene(const WideRay& R) const { return sc.of(R).S; }
   __device__ __forceinline__ uint32_t fetch(const WideRay& R, uint32_t i) const {
     if (SHADOW >= 0 && i >= n) {
       const float4* e = B.shadow + 4 * (size_t)(i - n);
       const float4 a = e[0], b = e[1];
-      const uint32_t sid = __float_as_uint(e[2].w);
+      const uint32_t sid = ONE ? 0u : __float_as_uint(e[2].w);
       R.set(kwId, (i - n) | 0x80000000u);
         return wide_begin(R, sid, xyz(a), xyz(b), occ_limit(tc, a.w));
     }
-    const uint32_t p = q[i], sid = scene_of(tab, n_scenes, p);
+    const uint32_t p = q[i], sid = sc.of_path(p);
     const float4 a = B.s[4 * (size_t)p], b = B.s[4 * (size_t)p + 1];
     R.set(kwId, p);
     return wide_begin(R, sid, xyz(a), xyz(b), 3.0e38f);
@@ -67,44 +79,50 @@ struct ExtendItem {
   __device__ __forceinline__ uint32_t shade(const WideRay&) const { return kwEmpty; }
 };
 
-__device__ __forceinline__ uint32_t* warp_pool(uint32_t* smem, uint32_t n_scenes, const TraceCfg& tc) {
-  return stacks_after(smem, n_scenes) + (threadIdx.x >> 5) * wide_pool_words(tc.stack_w);
+__device__ __forceinline__ uint32_t* warp_pool(uint32_t* smem, uint32_t n_table, const TraceCfg& tc) {
+  return stacks_after(smem, n_table) + (threadIdx.x >> 5) * wide_pool_words(tc.stack_w);
 }
 
-template <int SHADOW, int BS>
-__global__ void __launch_bounds__(BS, kWideBlocks * kWfBlock / BS) k_wide_extend(TraceCfg tc, WfBuffers B,
-                                                                                 uint32_t n_scenes, int qi,
-                                                                                 Counters* ctr) {
+// The scenes of a block: the table goes to shared memory unless there is one scene.
+template <bool ONE>
+__device__ __forceinline__ Scenes<ONE> block_scenes(const WfScene& one, const WfBuffers& B, uint32_t n_table,
+                                                    uint32_t* smem) {
+  return Scenes<ONE>{one, ONE ? nullptr : load_table(B.table, n_table, smem), n_table};
+}
+
+// n_table: scenes of the table (0 with ONE, then `one` is the scene).
+template <int SHADOW, bool ONE, int BS>
+__global__ void __launch_bounds__(BS, kWideBlocks * kWfBlock / BS)
+    k_wide_extend(const __grid_constant__ TraceCfg tc, const __grid_constant__ WfBuffers B,
+                  const __grid_constant__ WfScene one, uint32_t n_table, int qi, Counters* ctr) {
   extern __shared__ uint32_t smem[];
-  const WfScene* tab = load_table(B.table, n_scenes, smem);
   const uint32_t n = B.counts[qi];
-  ExtendItem<SHADOW> it{tab, B, tc, B.q[qi], n_scenes, n};
-  wide_run(it, tc, warp_pool(smem, n_scenes, tc), B.counts + 4, SHADOW >= 0 ? n + B.counts[3] : n, ctr);
+  ExtendItem<SHADOW, ONE> it{block_scenes<ONE>(one, B, n_table, smem), B, tc, B.q[qi], n};
+  wide_run(it, tc, warp_pool(smem, n_table, tc), B.counts + 4, SHADOW >= 0 ? n + B.counts[3] : n, ctr);
 }
 
 // The last segment's shadow requests.
-template <int MODE, int BS>
-__global__ void __launch_bounds__(BS, kWideBlocks * kWfBlock / BS) k_wide_shadow(TraceCfg tc, WfBuffers B,
-                                                                                 uint32_t n_scenes, Counters* ctr) {
+template <int MODE, bool ONE, int BS>
+__global__ void __launch_bounds__(BS, kWideBlocks * kWfBlock / BS)
+    k_wide_shadow(const __grid_constant__ TraceCfg tc, const __grid_constant__ WfBuffers B,
+                  const __grid_constant__ WfScene one, uint32_t n_table, Counters* ctr) {
   extern __shared__ uint32_t smem[];
-  const WfScene* tab = load_table(B.table, n_scenes, smem);
-  ExtendItem<MODE> it{tab, B, tc, nullptr, n_scenes, 0u};
-  wide_run(it, tc, warp_pool(smem, n_scenes, tc), B.counts + 5, B.counts[2], ctr);
+  ExtendItem<MODE, ONE> it{block_scenes<ONE>(one, B, n_table, smem), B, tc, nullptr, 0u};
+  wide_run(it, tc, warp_pool(smem, n_table, tc), B.counts + 5, B.counts[2], ctr);
 }
 
 // Every path still alive, to its end: a finished ray's slot waits for its shading (or for
 // its shadow ray's contribution), which is one more action of the warp.  A path's
 // shadow request waits in the slot of the request array that its id names.
-template <int MODE>
+template <int MODE, bool ONE>
 struct TailItem {
-  const WfScene* tab;
+  Scenes<ONE> scs;
   const WfBuffers& B;
   const TraceCfg& tc;
   const uint32_t* q;
-  uint32_t n_scenes;
-  __device__ __forceinline__ const DevScene& scene(const WideRay& R) const { return tab[R.u(kwRecInst) >> 20].S; }
+  __device__ __forceinline__ const DevScene& scene(const WideRay& R) const { return scs.of(R).S; }
   __device__ __forceinline__ uint32_t fetch(const WideRay& R, uint32_t i) const {
-    const uint32_t p = q[i], sid = scene_of(tab, n_scenes, p);
+    const uint32_t p = q[i], sid = scs.of_path(p);
     const float4 a = B.s[4 * (size_t)p], b = B.s[4 * (size_t)p + 1];
     R.set(kwId, p);
     return wide_begin(R, sid, xyz(a), xyz(b), 3.0e38f);
@@ -124,7 +142,7 @@ struct TailItem {
   static constexpr bool kShades = true;
   __device__ __forceinline__ uint32_t shade(const WideRay& R) const {
     const uint32_t id = R.u(kwId), p = id & 0x7fffffffu, sid = R.u(kwRecInst) >> 20;
-    const WfScene& sc = tab[sid];
+    const WfScene& sc = scs.at(sid);
     PathState ps;
     load_state(B, p, ps);
     ShadowReq rq;
@@ -150,14 +168,13 @@ struct TailItem {
   }
 };
 
-template <int MODE, int BS>
-__global__ void __launch_bounds__(BS, kWideBlocks * kWfBlock / BS) k_wide_tail(TraceCfg tc, WfBuffers B,
-                                                                               uint32_t n_scenes, int qi,
-                                                                               Counters* ctr) {
+template <int MODE, bool ONE, int BS>
+__global__ void __launch_bounds__(BS, kWideBlocks * kWfBlock / BS)
+    k_wide_tail(const __grid_constant__ TraceCfg tc, const __grid_constant__ WfBuffers B,
+                const __grid_constant__ WfScene one, uint32_t n_table, int qi, Counters* ctr) {
   extern __shared__ uint32_t smem[];
-  const WfScene* tab = load_table(B.table, n_scenes, smem);
-  TailItem<MODE> it{tab, B, tc, B.q[qi], n_scenes};
-  wide_run(it, tc, warp_pool(smem, n_scenes, tc), B.counts + 6, B.counts[qi], ctr);
+  TailItem<MODE, ONE> it{block_scenes<ONE>(one, B, n_table, smem), B, tc, B.q[qi]};
+  wide_run(it, tc, warp_pool(smem, n_table, tc), B.counts + 6, B.counts[qi], ctr);
 }
 
 // The adjoint's shadow requests: visibility only.
@@ -192,8 +209,9 @@ struct AdjShadowItem {
   __device__ __forceinline__ uint32_t shade(const WideRay&) const { return kwEmpty; }
 };
 
-__global__ void __launch_bounds__(kWfBlock, kWideBlocks) k_wide_adj_shadow(DevScene S, TraceCfg tc, WfBuffers B,
-                                                                           float4* rec, uint32_t rows, uint32_t flag,
+__global__ void __launch_bounds__(kWfBlock, kWideBlocks) k_wide_adj_shadow(const __grid_constant__ DevScene S,
+                                                                           const __grid_constant__ TraceCfg tc,
+                                                                           const __grid_constant__ WfBuffers B, float4* rec, uint32_t rows, uint32_t flag,
                                                                            Counters* ctr) {
   extern __shared__ uint32_t smem[];
   AdjShadowItem it{S, B, tc, rec, rows, flag};
@@ -224,7 +242,8 @@ struct RayItem {
   __device__ __forceinline__ uint32_t shade(const WideRay&) const { return kwEmpty; }
 };
 
-__global__ void __launch_bounds__(kWfBlock, kWideBlocks) k_wide_trace_rays(DevScene S, TraceCfg tc,
+__global__ void __launch_bounds__(kWfBlock, kWideBlocks) k_wide_trace_rays(const __grid_constant__ DevScene S,
+                                                                           const __grid_constant__ TraceCfg tc,
                                                                            const float* __restrict__ rays, uint32_t n,
                                                                            Hit* __restrict__ out, Counters* ctr,
                                                                            uint32_t* cursor) {
@@ -248,7 +267,7 @@ Shape shape(const TraceCfg& tc, uint32_t n_scenes, uint32_t blocks_per_sm, int s
   return g;
 }
 Shape shape(const TraceCfg& tc, const WfLaunch& L) {
-  return shape(tc, L.n_scenes, L.trace_blocks_per_sm, L.sms, tc.block == 64 ? 64u : (uint32_t)kWfBlock);
+  return shape(tc, L.one ? 0u : L.n_scenes, L.trace_blocks_per_sm, L.sms, tc.block == 64 ? 64u : (uint32_t)kWfBlock);
 }
 
 template <typename K>
@@ -259,10 +278,11 @@ cudaError_t limit(K kernel) {
 template <int BS>
 using Blk = std::integral_constant<int, BS>;
 
+// f(block size, one scene) with both as types.
 template <typename F>
-void by_block(uint32_t block, F f) {
-  if (block == 64) f(Blk<64>{});
-  else f(Blk<kWfBlock>{});
+void by_shape(uint32_t block, bool one, F f) {
+  if (block == 64) one ? f(Blk<64>{}, std::true_type{}) : f(Blk<64>{}, std::false_type{});
+  else one ? f(Blk<kWfBlock>{}, std::true_type{}) : f(Blk<kWfBlock>{}, std::false_type{});
 }
 
 }  // namespace
@@ -273,13 +293,15 @@ cudaError_t wide_prepare(int mode) {
     if (e == cudaSuccess) e = limit(kernel);
   };
   for (uint32_t b : {64u, (uint32_t)kWfBlock})
-    by_block(b, [&](auto bs) {
-      constexpr int BS = decltype(bs)::value;
-      raise(k_wide_extend<-1, BS>);
-      if (mode == 1) raise(k_wide_extend<1, BS>), raise(k_wide_shadow<1, BS>), raise(k_wide_tail<1, BS>);
-      if (mode == 2) raise(k_wide_extend<2, BS>), raise(k_wide_shadow<2, BS>), raise(k_wide_tail<2, BS>);
-      if (mode == 0) raise(k_wide_tail<0, BS>);
-    });
+    for (bool one : {false, true})
+      by_shape(b, one, [&](auto bs, auto on) {
+        constexpr int BS = decltype(bs)::value;
+        constexpr bool ONE = decltype(on)::value;
+        raise(k_wide_extend<-1, ONE, BS>);
+        if (mode == 1) raise(k_wide_extend<1, ONE, BS>), raise(k_wide_shadow<1, ONE, BS>), raise(k_wide_tail<1, ONE, BS>);
+        if (mode == 2) raise(k_wide_extend<2, ONE, BS>), raise(k_wide_shadow<2, ONE, BS>), raise(k_wide_tail<2, ONE, BS>);
+        if (mode == 0) raise(k_wide_tail<0, ONE, BS>);
+      });
   if (mode == 2) raise(k_wide_adj_shadow);
   return e;
 }
@@ -287,29 +309,36 @@ cudaError_t wide_prepare(int mode) {
 void wide_extend(int shadow, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, int qi, Counters* ctr,
                  cudaStream_t st) {
   const Shape g = shape(tc, L);
-  by_block(g.block, [&](auto bs) {
+  by_shape(g.block, L.one != nullptr, [&](auto bs, auto on) {
     constexpr int BS = decltype(bs)::value;
-    const auto k = shadow == 1 ? k_wide_extend<1, BS> : shadow == 2 ? k_wide_extend<2, BS> : k_wide_extend<-1, BS>;
-    k<<<g.grid, g.block, g.smem, st>>>(tc, B, L.n_scenes, qi, ctr);
+    constexpr bool ONE = decltype(on)::value;
+    const auto k = shadow == 1   ? k_wide_extend<1, ONE, BS>
+                   : shadow == 2 ? k_wide_extend<2, ONE, BS>
+                                 : k_wide_extend<-1, ONE, BS>;
+    k<<<g.grid, g.block, g.smem, st>>>(tc, B, ONE ? *L.one : WfScene{}, ONE ? 0u : L.n_scenes, qi, ctr);
   });
 }
 
 void wide_shadow(int mode, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, Counters* ctr, cudaStream_t st) {
   const Shape g = shape(tc, L);
-  by_block(g.block, [&](auto bs) {
+  by_shape(g.block, L.one != nullptr, [&](auto bs, auto on) {
     constexpr int BS = decltype(bs)::value;
-    const auto k = mode == 1 ? k_wide_shadow<1, BS> : k_wide_shadow<2, BS>;
-    k<<<g.grid, g.block, g.smem, st>>>(tc, B, L.n_scenes, ctr);
+    constexpr bool ONE = decltype(on)::value;
+    const auto k = mode == 1 ? k_wide_shadow<1, ONE, BS> : k_wide_shadow<2, ONE, BS>;
+    k<<<g.grid, g.block, g.smem, st>>>(tc, B, ONE ? *L.one : WfScene{}, ONE ? 0u : L.n_scenes, ctr);
   });
 }
 
 void wide_tail(int mode, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, int qi, Counters* ctr,
                cudaStream_t st) {
   const Shape g = shape(tc, L);
-  by_block(g.block, [&](auto bs) {
+  by_shape(g.block, L.one != nullptr, [&](auto bs, auto on) {
     constexpr int BS = decltype(bs)::value;
-    const auto k = mode == 0 ? k_wide_tail<0, BS> : mode == 1 ? k_wide_tail<1, BS> : k_wide_tail<2, BS>;
-    k<<<g.grid, g.block, g.smem, st>>>(tc, B, L.n_scenes, qi, ctr);
+    constexpr bool ONE = decltype(on)::value;
+    const auto k = mode == 0   ? k_wide_tail<0, ONE, BS>
+                   : mode == 1 ? k_wide_tail<1, ONE, BS>
+                               : k_wide_tail<2, ONE, BS>;
+    k<<<g.grid, g.block, g.smem, st>>>(tc, B, ONE ? *L.one : WfScene{}, ONE ? 0u : L.n_scenes, qi, ctr);
   });
 }
 
