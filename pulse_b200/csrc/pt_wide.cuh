@@ -83,7 +83,7 @@ constexpr uint32_t kTopStack = 16, kTopStackDeep = 24;  // entries for trees of 
 // fullest one nearly always fills the warp, where one ray per lane in
 // registers left 11 to 15 lanes active per instruction (1080p sphere frame, first
 // extend: see k_wide_extend).
-constexpr uint32_t kPool = 64;  // slots laid out; kPool - 1 are used (six-bit counts)
+constexpr uint32_t kPool = 64;
 
 // An instance's record for entering it (DevScene::inst_wide), 96 bytes: its
 // world-to-object matrix, (root group of the mesh's tree, or 0 and its only leaf's reference,
@@ -91,8 +91,8 @@ constexpr uint32_t kPool = 64;  // slots laid out; kPool - 1 are used (six-bit c
 constexpr uint32_t kWideInstRows = 6;
 
 enum WideWord : uint32_t {
-  kwOX, kwOY, kwOZ, kwDX, kwDY, kwDZ,  // object ray
-  kwCull,                              // box entry bound in the BLAS
+  kwOX, kwOY, kwOZ, kwDX, kwDY, kwDZ,  // ray of the level
+  kwCull,                              // box entry bound of the level
   kwGrp,                               // current group
   kwCur,                               // current leaf: elements left << 26 | next element; TLAS: node or instance
   kwSp,                                // stack entries | those of the TLAS level << 7 | instance << 12 | in a BLAS << 31
@@ -108,8 +108,7 @@ enum WideWord : uint32_t {
 constexpr uint32_t kInstBits = 17, kInstMask = (1u << kInstBits) - 1u;
 // Action classes of a slot.  kwShade: the kernel's own step.
 enum WideAct : uint32_t {
-  kwNode = 0, kwTriangles = 1, kwInstance = 2, kwTop = 3, kwVerify = 4, kwRedo = 5, kwShade = 6, kwEmpty = 7, kwDone = 8,
-  kwUnused = 9
+  kwNode = 0, kwTriangles = 1, kwInstance = 2, kwVerify = 3, kwRedo = 4, kwShade = 5, kwEmpty = 6, kwDone = 7
 };
 
 // Words of a warp's pool: the rays with their stacks, the slots' classes and the step's list.
@@ -166,21 +165,33 @@ constexpr uint32_t kInBlas = 1u << 31;
 // transforms.
 __device__ __forceinline__ float wide_gate(float t, float eps) { return t * 1.0000025f + eps; }
 
+// The bound of boxes whose hits may be found up to the slack before them.
+__device__ __forceinline__ float wide_bound(float t, float slack) { return t * (1.0f + slack) + slack; }
+
+// The level becomes the TLAS.
+__device__ __forceinline__ void wide_world(const WideRay& R, const DevScene& S, float3 wo, float3 wd, float rec_t,
+                                           float far) {
+  R.setf3(kwOX, wo);
+  R.setf3(kwDX, wd);
+  R.setf(kwCull, fminf(wide_bound(rec_t, S.wide_slack), far));
+}
+
 // Begin a ray of a scene in a slot; its first class.  limit < 1e29 makes it an occlusion
 // query.
-__device__ __forceinline__ uint32_t wide_begin(const WideRay& R, uint32_t scene, float3 wo, float3 wd, float limit) {
+__device__ __forceinline__ uint32_t wide_begin(const WideRay& R, uint32_t scene, const DevScene& S, float3 wo,
+                                               float3 wd, float limit) {
+  const float far = world_cull(limit, wo);
+  wide_world(R, S, wo, wd, 1e30f, far);
   R.set(kwSp, 0u);
   R.setf(kwRecT, 1e30f);
   R.set(kwRecInst, scene << 20);
-  R.set(kwGrp, 0u);
   R.set(kwCur, 0u);  // the root node
-  R.setf(kwFar, world_cull(limit, wo));
+  R.setf(kwFar, far);
   R.setf(kwEps, 1e-6f * max_abs3(wo));
   const float x = limit * 0.9999f - 1e-3f * (1.0f + max_abs3(wo));
   R.setf(kwExit, limit < 1e29f && x < 3.0e38f ? x : -1.0f);
   if (!(limit > 0.0f)) return kwDone;
-  if (!wide_ray_ok(wo, wd)) return kwRedo;
-  return kwTop;
+  return wide_ray_ok(wo, wd) ? kwNode : kwRedo;
 }
 
 // The next leaf of a leaf group whose hit bits are not all zero, taken out of the group.
@@ -203,9 +214,6 @@ __device__ __forceinline__ uint32_t wide_pop(const WideRay& R, uint32_t spx) {
   return some ? kwNode : kwInstance;
 }
 
-// The bound of boxes whose hits may be found up to the slack before them.
-__device__ __forceinline__ float wide_bound(float t, float slack) { return t * (1.0f + slack) + slack; }
-
 // The next entry of the TLAS stack that is not beyond the bound, or the ray's end.
 __device__ __forceinline__ uint32_t wide_top_pop(const WideRay& R, uint32_t sp, float bound, float rec_t) {
   uint32_t next = kwDone;
@@ -213,7 +221,7 @@ __device__ __forceinline__ uint32_t wide_top_pop(const WideRay& R, uint32_t sp, 
     const uint32_t e = R.stack(--sp);
     if (__uint_as_float((e >> 18) << 17) > bound) continue;
     R.set(kwCur, (e >> 1) & ((1u << kTopIndexBits) - 1u));
-    next = e & 1u ? kwInstance : kwTop;
+    next = e & 1u ? kwInstance : kwNode;
     break;
   }
   R.set(kwSp, sp);
@@ -292,48 +300,46 @@ __device__ __forceinline__ WideTest wide_test(const uint4* np, float3 o, float3 
   return WideTest{miss, (e >> 24) & 15u, e >> 28, child};
 }
 
-// Visit the next child of the BLAS's current (interior) group.
-__device__ __forceinline__ uint32_t wide_node(const WideRay& R, const DevScene& S) {
-  const uint32_t grp = R.u(kwGrp);
+// Visit a node: in a BLAS the next child of the current (interior) group; in the TLAS
+// the current one, whose children hit go on the stack, the nearest on top.
+__device__ __forceinline__ uint32_t wide_node(const WideRay& R, const DevScene& S, const TraceCfg& cfg) {
   uint32_t spx = R.u(kwSp);
+  const bool blas = (spx & kInBlas) != 0u;
   const float3 rinv = v3(wide_rcp(R.f(kwDX)), wide_rcp(R.f(kwDY)), wide_rcp(R.f(kwDZ)));
-  const uint32_t axis = (grp >> kWideIndexBits) & 3u, hits = grp >> 24;
-  const float along = axis == 0u ? rinv.x : axis == 1u ? rinv.y : rinv.z;
-  const uint32_t k = along < 0.0f ? 31u - __clz(hits) : __ffs(hits) - 1u;
-  const uint32_t rest = grp & ~(0x1000000u << k);
-  const uint32_t at = (grp & kWideIndexMask) + k;
-  if (rest >> 24) R.stack(spx++ & 0x7fu) = rest;
-  const WideTest w = wide_test(S.wide_blas + (size_t)at * (kWideNodeWords / 4), R.f3(kwOX), rinv,
-                               R.f(kwCull), [](int, float) {});
-  const uint32_t ih = ~w.miss & ((1u << w.ni) - 1u), lh = ~w.miss & (0xff00u >> w.nl) & 0xffu;
-  const uint32_t inner = (w.child & (kWideIndexMask | (3u << kWideIndexBits))) | (ih << 24);
-  if (lh) {
-    if (ih) R.stack(spx++ & 0x7fu) = inner;
-    uint32_t leaves = at | (3u << kWideIndexBits) | (lh << 24);
-    R.set(kwCur, wide_leaf(S, leaves));
-    R.set(kwGrp, leaves);
-    R.set(kwSp, spx);
-    return kwTriangles;
+  uint32_t at = R.u(kwCur);
+  if (blas) {
+    const uint32_t grp = R.u(kwGrp), axis = (grp >> kWideIndexBits) & 3u, hits = grp >> 24;
+    const float along = axis == 0u ? rinv.x : axis == 1u ? rinv.y : rinv.z;
+    const uint32_t k = along < 0.0f ? 31u - __clz(hits) : __ffs(hits) - 1u;
+    const uint32_t rest = grp & ~(0x1000000u << k);
+    at = (grp & kWideIndexMask) + k;
+    if (rest >> 24) R.stack(spx++ & 0x7fu) = rest;
   }
-  if (ih) {
-    R.set(kwGrp, inner);
-    R.set(kwSp, spx);
-    return kwNode;
-  }
-  return wide_pop(R, spx);
-}
-
-// Visit a TLAS node: its children hit go on the stack, the nearest on top.
-__device__ __forceinline__ uint32_t wide_top(const WideRay& R, const DevScene& S, const TraceCfg& cfg, float3 wo,
-                                             float3 wd) {
-  uint32_t sp = R.u(kwSp);
-  const float rec_t = R.f(kwRecT), far = R.f(kwFar), slack = S.wide_slack;
-  const float bound = fminf(wide_bound(rec_t, kLeastSlack), far);
   float tn[8];
-  const uint4* np = S.wide_tlas + (size_t)R.u(kwCur) * (kWideNodeWords / 4);
-  const WideTest w = wide_test(np, wo, v3(wide_rcp(wd.x), wide_rcp(wd.y), wide_rcp(wd.z)),
-                               fminf(wide_bound(rec_t, slack), far), [&](int k, float t) { tn[k] = t; });
-  const uint32_t hit = ~w.miss & (((1u << w.ni) - 1u) | ((0xff00u >> w.nl) & 0xffu));
+  const uint4* np = (blas ? S.wide_blas : S.wide_tlas) + (size_t)at * (kWideNodeWords / 4);
+  const WideTest w = wide_test(np, R.f3(kwOX), rinv, R.f(kwCull), [&](int k, float t) { tn[k] = t; });
+  const uint32_t ih = ~w.miss & ((1u << w.ni) - 1u), lh = ~w.miss & (0xff00u >> w.nl) & 0xffu;
+  if (blas) {
+    const uint32_t inner = (w.child & (kWideIndexMask | (3u << kWideIndexBits))) | (ih << 24);
+    if (lh) {
+      if (ih) R.stack(spx++ & 0x7fu) = inner;
+      uint32_t leaves = at | (3u << kWideIndexBits) | (lh << 24);
+      R.set(kwCur, wide_leaf(S, leaves));
+      R.set(kwGrp, leaves);
+      R.set(kwSp, spx);
+      return kwTriangles;
+    }
+    if (ih) {
+      R.set(kwGrp, inner);
+      R.set(kwSp, spx);
+      return kwNode;
+    }
+    return wide_pop(R, spx);
+  }
+  const float rec_t = R.f(kwRecT), slack = S.wide_slack;
+  const float bound = fminf(wide_bound(rec_t, kLeastSlack), R.f(kwFar));
+  const uint32_t hit = ih | lh;
+  uint32_t sp = spx;
   if (hit) {
     if (sp + __popc(hit) > cfg.stack_top) return kwRedo;
     const uint4 ra = __ldg(np + 1), rb = __ldg(np + 5);  // references of the leaves
@@ -458,6 +464,7 @@ __device__ __forceinline__ uint32_t wide_instance(const WideRay& R, const DevSce
   if (sp & kInBlas) {
     const uint32_t next =
         wide_top_pop(R, (sp >> 7) & 0x1fu, fminf(wide_bound(rec_t, kLeastSlack), far), rec_t);
+    if (next == kwNode) wide_world(R, S, wo, wd, rec_t, far);
     if (next != kwInstance) return next;
     sp = R.u(kwSp);
   }
@@ -572,25 +579,25 @@ __device__ __forceinline__ void wide_run(Item& it, const TraceCfg& tc, uint32_t*
   const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
   uint8_t* cls = reinterpret_cast<uint8_t*>(pool + (kWideWords + tc.stack_w) * kPool);
   uint8_t* list = cls + kPool;
-  reinterpret_cast<uint16_t*>(cls)[lane] = (uint16_t)(kwEmpty | ((lane < 31u ? kwEmpty : kwUnused) << 8));
+  reinterpret_cast<uint16_t*>(cls)[lane] = (uint16_t)(kwEmpty | (kwEmpty << 8));
   __syncwarp();
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-  const uint32_t share = min(kPool - 1u, (n_items + warps - 1u) / warps);  // of the first, fixed items
-  uint32_t at = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * share;
+  const uint32_t share = min(kPool, (n_items + warps - 1u) / warps);  // of the first, fixed items
+  uint32_t at = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * share;
   uint32_t end = min(at + share, n_items);
   at = min(at, end);
   bool drained = false;  // nothing left to fetch
   while (true) {
     const uint32_t two = reinterpret_cast<const uint16_t*>(cls)[lane];
     const uint32_t c0 = two & 0xffu, c1 = two >> 8;
-    // slots per class, six bits each for the first five
+    // slots per class, seven bits each for the first four
     const uint32_t packed =
-        __reduce_add_sync(0xffffffffu, (c0 < 5u ? 1u << (6u * c0) : 0u) + (c1 < 5u ? 1u << (6u * c1) : 0u));
+        __reduce_add_sync(0xffffffffu, (c0 < 4u ? 1u << (7u * c0) : 0u) + (c1 < 4u ? 1u << (7u * c1) : 0u));
     // the fullest: count << 3 | class
-    const uint32_t kn = (packed & 63u) << 3, kt = ((packed >> 3) & 0x1f8u) | 1u, ki = ((packed >> 9) & 0x1f8u) | 2u;
-    const uint32_t ku = ((packed >> 15) & 0x1f8u) | 3u, kv = ((packed >> 21) & 0x1f8u) | 4u;
-    uint32_t key = max(max(max(kn, kt), max(ki, ku)), kv);
-    const uint32_t rest = kPool - 1u - (kn >> 3) - (kt >> 3) - (ki >> 3) - (ku >> 3) - (kv >> 3);
+    const uint32_t kn = (packed & 127u) << 3, kt = ((packed >> 4) & 0x3f8u) | 1u;
+    const uint32_t ki = ((packed >> 11) & 0x3f8u) | 2u, kv = ((packed >> 18) & 0x3f8u) | 3u;
+    uint32_t key = max(max(kn, kt), max(ki, kv));
+    const uint32_t rest = kPool - (kn >> 3) - (kt >> 3) - (ki >> 3) - (kv >> 3);
     if (Item::kShades || rest >= kFetchAt || key < 8u) {
       const uint32_t nr = __popc(__ballot_sync(0xffffffffu, c0 == kwRedo)) + __popc(__ballot_sync(0xffffffffu, c1 == kwRedo));
       uint32_t ns = 0u;
@@ -630,7 +637,7 @@ __device__ __forceinline__ void wide_run(Item& it, const TraceCfg& tc, uint32_t*
       const WideRay R{pool + slot};
       uint32_t next;
       if (act == kwNode) {
-        next = wide_node(R, it.scene(R));
+        next = wide_node(R, it.scene(R), tc);
       } else if (act == kwTriangles) {
         next = wide_tri(R, it.scene(R), tc);
       } else if (act == kwEmpty) {
@@ -641,9 +648,7 @@ __device__ __forceinline__ void wide_run(Item& it, const TraceCfg& tc, uint32_t*
         float3 wo, wd;
         float limit;
         it.ray(R, wo, wd, limit);
-        if (act == kwTop) {
-          next = wide_top(R, it.scene(R), tc, wo, wd);
-        } else if (act == kwInstance) {
+        if (act == kwInstance) {
           next = wide_instance(R, it.scene(R), wo, wd);
         } else if (act == kwVerify) {
           next = wide_verify(R, it.scene(R), tc, wo, wd);

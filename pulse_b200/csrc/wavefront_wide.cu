@@ -48,12 +48,12 @@ struct ExtendItem {
       const float4 a = e[0], b = e[1];
       const uint32_t sid = ONE ? 0u : __float_as_uint(e[2].w);
       R.set(kwId, (i - n) | 0x80000000u);
-        return wide_begin(R, sid, xyz(a), xyz(b), occ_limit(tc, a.w));
+        return wide_begin(R, sid, sc.at(sid).S, xyz(a), xyz(b), occ_limit(tc, a.w));
     }
     const uint32_t p = q[i], sid = sc.of_path(p);
     const float4 a = B.s[4 * (size_t)p], b = B.s[4 * (size_t)p + 1];
     R.set(kwId, p);
-    return wide_begin(R, sid, xyz(a), xyz(b), 3.0e38f);
+    return wide_begin(R, sid, sc.at(sid).S, xyz(a), xyz(b), 3.0e38f);
   }
   __device__ __forceinline__ void ray(const WideRay& R, float3& o, float3& d, float& limit) const {
     const uint32_t id = R.u(kwId);
@@ -125,7 +125,7 @@ struct TailItem {
     const uint32_t p = q[i], sid = scs.of_path(p);
     const float4 a = B.s[4 * (size_t)p], b = B.s[4 * (size_t)p + 1];
     R.set(kwId, p);
-    return wide_begin(R, sid, xyz(a), xyz(b), 3.0e38f);
+    return wide_begin(R, sid, scs.at(sid).S, xyz(a), xyz(b), 3.0e38f);
   }
   __device__ __forceinline__ void ray(const WideRay& R, float3& o, float3& d, float& limit) const {
     const uint32_t id = R.u(kwId);
@@ -160,11 +160,11 @@ struct TailItem {
     if (rq.active) {
       put_shadow(B, p, rq, p, sid);
       R.set(kwId, p | 0x80000000u);
-      return wide_begin(R, sid, rq.o, rq.d, occ_limit(tc, rq.limit));
+      return wide_begin(R, sid, sc.S, rq.o, rq.d, occ_limit(tc, rq.limit));
     }
     if (!(ps.flags & kAlive)) return kwEmpty;
     R.set(kwId, p);
-    return wide_begin(R, sid, ps.o, ps.d, 3.0e38f);
+    return wide_begin(R, sid, sc.S, ps.o, ps.d, 3.0e38f);
   }
 };
 
@@ -188,7 +188,7 @@ struct AdjShadowItem {
   __device__ __forceinline__ uint32_t fetch(const WideRay& R, uint32_t i) const {
     const float4 a = B.shadow[4 * (size_t)i], b = B.shadow[4 * (size_t)i + 1];
     R.set(kwId, i);
-    return wide_begin(R, 0u, xyz(a), xyz(b), occ_limit(tc, a.w));
+    return wide_begin(R, 0u, S, xyz(a), xyz(b), occ_limit(tc, a.w));
   }
   __device__ __forceinline__ void ray(const WideRay& R, float3& o, float3& d, float& limit) const {
     const float4* e = B.shadow + 4 * (size_t)R.u(kwId);
@@ -226,7 +226,7 @@ struct RayItem {
   __device__ __forceinline__ uint32_t fetch(const WideRay& R, uint32_t i) const {
     const float* r = rays + 6 * (size_t)i;
     R.set(kwId, i);
-    return wide_begin(R, 0u, v3(r[0], r[1], r[2]), v3(r[3], r[4], r[5]), 3.0e38f);
+    return wide_begin(R, 0u, S, v3(r[0], r[1], r[2]), v3(r[3], r[4], r[5]), 3.0e38f);
   }
   __device__ __forceinline__ void ray(const WideRay& R, float3& o, float3& d, float& limit) const {
     const float* r = rays + 6 * (size_t)R.u(kwId);
