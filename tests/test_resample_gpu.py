@@ -1,7 +1,10 @@
 """The upscaling hand-off (pulse_target_resample) against a NumPy restatement
 of the same float32 arithmetic and float16 rounding, bit for bit."""
+import ctypes as C
+
 import numpy as np
 import pytest
+import torch
 
 from pulse_b200 import scenes
 from pulse_b200.tracer import Scene, Target, render_forward
@@ -58,6 +61,26 @@ def test_resample_bit_exact(rendered, filt, size):
     got = tg.resample(size[0], size[1], filt)
     ref = resample_ref(img, size[0], size[1], filt)
     assert np.array_equal(got.view(np.uint16), ref.view(np.uint16))
+
+
+@pytest.mark.parametrize("filt", [0, 1])
+@pytest.mark.parametrize("offset", [0, 8])
+@pytest.mark.parametrize("size", [(2, 5), (511, 3), (512, 4), (513, 4), (514, 9)])
+def test_resample_to_device_memory(ctx, rendered, filt, offset, size):
+    """Widths and rows around a block's 512 columns (256 one texel at a time) and
+    4 rows, into a destination on and 8 bytes off a 16-byte boundary; nothing is
+    written outside it."""
+    tg, img = rendered
+    w, h = size
+    guard = 16
+    buf = torch.full((offset + w * h * 8 + guard,), 0xAB, dtype=torch.uint8, device="cuda")
+    assert buf.data_ptr() % 16 == 0
+    ctx.check(ctx.lib.pulse_target_resample(tg.h, w, h, filt, C.c_void_p(buf.data_ptr() + offset), 0), "resample")
+    ctx.sync()
+    raw = buf.cpu().numpy()
+    assert (raw[:offset] == 0xAB).all() and (raw[offset + w * h * 8:] == 0xAB).all()
+    got = raw[offset:offset + w * h * 8].view(np.uint16).reshape(h, w, 4)
+    assert np.array_equal(got, resample_ref(img, w, h, filt).view(np.uint16))
 
 
 def test_resample_identity_nearest(rendered):
