@@ -98,6 +98,22 @@ def test_batch_launch_shapes(ctx, trio, trace_blocks, wf_segments, block_size, r
     _close(scs, tgs)
 
 
+@pytest.mark.parametrize("spp", [1, 3, 4, 5, 9])
+def test_batch_samples_per_texel(ctx, trio, spp):
+    """Samples below, at and past the four a texel's thread fetches at a time, over
+    texel counts that are no multiple of a block's threads, in two frames."""
+    items = [(2, 2, 7), (0, 1, 8), (1, 2, 9)]
+    params = dict(max_depth=2, nee_mode=2, light_pick=1, quirks=0, spp=spp)
+    scs, tgs = _setup(ctx, trio, items)
+    for acc in range(2):
+        render_batch(ctx, [BatchItem(scs[i], trio[i][0].view, tgs[k], acc, md, seed)
+                           for k, (i, md, seed) in enumerate(items)], **params)
+    refs = _oracle_frames(trio, items, 2, params)
+    for k, ref in enumerate(refs):
+        _assert_same(tgs[k].download(), ref, f"item {k}")
+    _close(scs, tgs)
+
+
 def test_batch_equals_forward_and_composition_changes(ctx, trio):
     """Batches of 1, 5, 2 and 5 items in a row (graph re-instantiated or
     updated in place) each equal the per-scene forward render."""
