@@ -250,14 +250,17 @@ __global__ void __launch_bounds__(kAdjBlock, 8) k_adj_resolve(DevScene S, PathCf
     const float3 nn = xyz(a0), wo = xyz(a1), Tv = xyz(a3);
     const uint32_t mi = __float_as_uint(a1.w);
     const Material m = load_material(S, mi);
+    const Lobe lobe = lobe_at(nn, wo, m);
     const float3 d = path_delta(dimg, p, pc.spp, inv_n);
     float3 L_rem = xyz(r[5]);
+    float pb;
     if ((flags & kNee) && (flags & kVisible)) {
       const float4 a2 = r[2];
       const float3 wl = xyz(a2);
       const uint32_t ml = __float_as_uint(a2.w);
       const float sc = a0.w;
-      const float3 gl = eval_g(nn, wo, wl, m);
+      float3 gl;
+      eval_lobe(nn, wo, wl, m, lobe, gl, pb);
       const float3 Le = load_material(S, ml).emissive;
       G.add(ml, 3, d.x * Tv.x * gl.x * sc);
       G.add(ml, 4, d.y * Tv.y * gl.y * sc);
@@ -270,7 +273,8 @@ __global__ void __launch_bounds__(kAdjBlock, 8) k_adj_resolve(DevScene S, PathCf
     }
     if (flags & kCont) {
       const float3 wi = xyz(r[4]);
-      const float3 gv = eval_g(nn, wo, wi, m);
+      float3 gv;
+      eval_lobe(nn, wo, wi, m, lobe, gv, pb);
       float3 db, dr;
       eval_g_grad(nn, wo, wi, m, db, dr);
       const float3 coef = v3(gv.x != 0.0f ? d.x * L_rem.x / gv.x : 0.0f, gv.y != 0.0f ? d.y * L_rem.y / gv.y : 0.0f,

@@ -188,30 +188,39 @@ __device__ __forceinline__ void world_tri(const DevScene& S, const float4* ip, u
   ng = divs(cr, len);
 }
 
-__device__ __forceinline__ float3 eval_g(float3 n, float3 wo, float3 wi, const Material& m) {
-  const float NI = dot(n, wi), NO = dot(n, wo);
-  if (!(NI > 0.0f) || !(NO > 0.0f)) return v3(0.0f, 0.0f, 0.0f);
+// What the BRDF's value and its sampling pdf share for every incoming direction of a vertex.
+struct Lobe { float3 f0; float NO, F0max, g1o; };
+
+__device__ __forceinline__ Lobe lobe_at(float3 n, float3 wo, const Material& m) {
+  Lobe l;
+  l.f0 = material_f0(m);
+  l.NO = dot(n, wo);
+  l.F0max = max3(fresnel(l.NO, l.f0, false));
+  l.g1o = G1(l.NO, m.rough);
+  return l;
+}
+
+// gv: the BRDF times the cosine; pb: the pdf of the mixture that samples it.  One branch
+// and one half vector for both.
+__device__ __forceinline__ void eval_lobe(float3 n, float3 wo, float3 wi, const Material& m, const Lobe& l, float3& gv,
+                                          float& pb) {
+  gv = v3(0.0f, 0.0f, 0.0f);
+  pb = 0.0f;
+  const float NI = dot(n, wi);
+  if (!(NI > 0.0f) || !(l.NO > 0.0f)) return;
   const float3 h = normalize(add(wo, wi));
   const float NM = dot(n, h), OM = dot(wo, h);
-  const float3 F = fresnel(OM, material_f0(m), false);
+  const float3 F = fresnel(OM, l.f0, false);
   const float D = D_GGX(NM, m.rough);
-  const float G = G_smith(NO, NI, m.rough);
-  const float den = 4.0f * NO * NI;
+  const float G = G1(NI, m.rough) * l.g1o;
+  const float den = 4.0f * l.NO * NI;
   const float dg = D * G;
   const float3 spec = v3(F.x * dg / den, F.y * dg / den, F.z * dg / den);
   const float3 diff = muls(m.base, kINV_PI);
-  return muls(add(diff, spec), NI);
-}
-__device__ __forceinline__ float mix_pdf(float3 n, float3 wo, float3 wi, const Material& m) {
-  const float NI = dot(n, wi), NO = dot(n, wo);
-  if (!(NI > 0.0f) || !(NO > 0.0f)) return 0.0f;
-  const float F0max = max3(fresnel(NO, material_f0(m), false));
-  const float3 h = normalize(add(wo, wi));
-  const float NM = dot(n, h), OM = dot(wo, h);
-  const float D = D_GGX(NM, m.rough);
+  gv = muls(add(diff, spec), NI);
   const float ps = OM > 0.0f ? D * NM / (4.0f * OM) : 0.0f;
   const float pd = NI * kINV_PI;
-  return (1.0f - F0max) * pd + F0max * ps;
+  pb = (1.0f - l.F0max) * pd + l.F0max * ps;
 }
 // Power-heuristic weight a^2 / (a^2 + b^2).  When a square overflows (a pdf
 // above ~1.8e19: a light sampled or hit at a grazing angle, a GGX lobe of a
@@ -489,6 +498,7 @@ __device__ __forceinline__ void path_on_hit(const DevScene& S, const PathCfg& c,
     ps.color = add(ps.color, muls(mul(ps.thr, Le), w));
     if (REC) vr->w_le = w;
   }
+  const Lobe lobe = lobe_at(g.n, wo, g.m);  // (of both directions evaluated below)
   if (S.light_count > 0) {
     float lpick;
     const uint32_t li = pick_light(S, c, ps.rng, lpick);
@@ -515,9 +525,10 @@ __device__ __forceinline__ void path_on_hit(const DevScene& S, const PathCfg& c,
       req.d = normalize(to);
       req.limit = length(sub(pl, req.o)) - c.eps_shadow;
       req.active = true;
-      const float3 gv = eval_g(g.n, wo, wi, g.m);
+      float3 gv;
+      float pb;
+      eval_lobe(g.n, wo, wi, g.m, lobe, gv, pb);
       const float plw = pa * dist2 / ce;
-      const float pb = mix_pdf(g.n, wo, wi, g.m);
       const float wl = mis2(plw, pb);
       const Material lm = load_material(S, __float_as_uint(__ldg(mi + 9).x));
       const float sc = wl / plw;
@@ -534,14 +545,14 @@ __device__ __forceinline__ void path_on_hit(const DevScene& S, const PathCfg& c,
       }
     }
   }
-  const float F0max = max3(fresnel(dot(g.n, wo), material_f0(g.m), false));
   const float e0 = rand_f(ps.rng), e1 = rand_f(ps.rng), e2 = rand_f(ps.rng);
   float3 wi;
-  if (e0 <= F0max) wi = reflect(wo, ggx_half(g.n, g.m.rough, e1, e2));
+  if (e0 <= lobe.F0max) wi = reflect(wo, ggx_half(g.n, g.m.rough, e1, e2));
   else wi = sample_cosine_hemisphere(g.n, e1, e2);
   wi = normalize(wi);
-  const float3 gv = eval_g(g.n, wo, wi, g.m);
-  const float pb = mix_pdf(g.n, wo, wi, g.m);
+  float3 gv;
+  float pb;
+  eval_lobe(g.n, wo, wi, g.m, lobe, gv, pb);
   ps.depth += 1;
   if (!(pb > 0.0f)) { ps.flags = 0; return; }
   // An overflowed GGX peak makes gv and pb infinite together; their ratio is
@@ -567,7 +578,7 @@ __device__ __forceinline__ void path_on_hit(const DevScene& S, const PathCfg& c,
   }
 }
 
-// Derivatives of eval_g (the BRDF times the cosine) with respect to the
+// Derivatives of eval_lobe's gv (the BRDF times the cosine) with respect to the
 // material's base color (per channel: d gv_c / d base_c; the other channels
 // do not depend on base_c) and its perceptual roughness r (alpha = r^2):
 //   gv_c = NI (base_c / pi + F_c D G / (4 NO NI)),  F_c = f0_c + (1 - f0_c) (1 - OM)^5,

@@ -245,12 +245,12 @@ __global__ void __launch_bounds__(BS, MINB * kWfBlock / BS) k_wf_extend(TraceCfg
   }
 }
 
-// Six blocks per SM (80 registers, 60 / 96 bytes of spill) rather than the
-// four that 102 spill-free registers allow: the shading waits on dependent
-// loads (light CDF search, triangle and material records) and gains from the
-// warps.  1080p sphere frame 145.6 -> 146.2 Mpaths/s; eight blocks (64
-// registers) 146.1.
-constexpr int kShadeBlocks = 6;
+// Bound by issue and its latencies (48% of the issue slots; waiting on dependent loads,
+// on the serial arithmetic and on instruction fetch), so eight blocks per SM (64
+// registers, some spill) in one resident wave: the shading of 512^2 x 16 spp, 4.2 M
+// paths, took 1.66 ms of a 5.91 ms frame at six blocks per SM and sixteen launched; the
+// frame takes 5.65 ms with eight (six 5.72, ten 5.72, three times the blocks 5.70).
+constexpr int kShadeBlocks = 8;
 
 template <int MODE, bool COUNT>
 __global__ void __launch_bounds__(kWfBlock, kShadeBlocks) k_wf_shade(WfBuffers B, uint32_t n_scenes, int qi,
@@ -692,7 +692,7 @@ uint32_t record_segments(const TraceCfg& tc, const WfBuffers& B, const WfLaunch&
     if (wide) wide_extend(pending ? MODE : -1, tc, B, L, qi, ctr, st);
     else (pending ? extend_sh : extend)<<<grid, tb, smem_tr, st>>>(tc, B, ns, qi, ctr, work);
     pending = false;
-    k_wf_shade<MODE, COUNT><<<g.light_blocks, kWfBlock, g.tab, st>>>(B, ns, qi, work);
+    k_wf_shade<MODE, COUNT><<<L.sms * kShadeBlocks, kWfBlock, g.tab, st>>>(B, ns, qi, work);
     n += 3;
     if (MODE != 0) {
       if (merge && seg + 1 < wf) pending = true;
