@@ -958,12 +958,15 @@ static void decide_wide(PulseScene* s, const std::vector<prep::InstanceIn>& ii, 
       slack = std::max(slack, m.wide_slack);
       levels = std::max(levels, m.wide_levels);
     }
-  // TLAS: every child hit, up to a fixed size (a ray that needs more is traced by
-  // the binary traversal); BLAS: a visit pushes the rest of its group and, with
-  // leaves hit, the interior children hit
-  const uint32_t top = std::min(7 * tree.levels + 1, tree.levels <= 3 ? pt::kTopStack : pt::kTopStackDeep);
-  s->dev.wide_top = top;
-  s->dev.wide_stack = top + levels + 1;
+  // TLAS: every child hit, up to a fixed size, and beyond it an entry a level and the
+  // child gone on with; BLAS: a visit pushes the rest of its group and, with leaves hit,
+  // the interior children hit
+  const uint32_t all = 7 * tree.levels + 1, again = tree.levels + 1, below = levels + 1;
+  const uint32_t left = pt::kWideStack - std::min(pt::kWideStack, again + below);
+  const uint32_t some = std::min(std::max(left, pt::kTopLeast), tree.levels <= 3 ? pt::kTopShallow : pt::kTopMost);
+  const bool fits = all <= some + again;
+  s->dev.wide_top = fits ? all : some;
+  s->dev.wide_stack = (fits ? all : some + again) + below;
   ok = ok && s->dev.wide_stack <= 96 && std::max((size_t)tree.count, ii.size()) < (1u << pt::kTopIndexBits) &&
        s->wide_nodes < (1ull << pt::kWideIndexBits) && s->counts.triangle_index_count < (1u << pt::kWideFirstBits);
   for (size_t i = 0; ok && i < ii.size(); ++i) ok = wide_transform(ii[i].object_world);

@@ -71,10 +71,23 @@ constexpr uint32_t kWideIndexMask = (1u << kWideIndexBits) - 1u;
 // bits (rounded down: entries beyond the record are dropped when popped), then
 // interior: child index << 1; leaf: instance << 1 | 1.  The distance of a child that may
 // hold a mesh of more than the least slack is lowered by the largest slack of the scene.
-constexpr uint32_t kTopIndexBits = 17;
+// Where the children hit do not fit, one is gone on with and the node itself is the
+// entry of the rest, to be visited again without the children that were missed or are done:
+// kTopAgain | those << 17 | node (distances stay below 2^97, boxes lying within 1e9, so no
+// entry's upper three bits are all ones).  That takes one entry a level at most, beyond
+// the cfg.stack_top entries up to which children are pushed.
+constexpr uint32_t kTopIndexBits = 17, kTopIndexMask = (1u << kTopIndexBits) - 1u;
+constexpr uint32_t kTopAgain = 0xe0000000u;
 constexpr uint32_t kLooseRef = 0x80000000u;
 constexpr float kLeastSlack = 1e-4f;
-constexpr uint32_t kTopStack = 16, kTopStackDeep = 24;  // entries for trees of up to 3 levels, and of more
+// Entries up to which children are pushed: 16 for trees of up to 3 levels (the 1080p
+// sphere frame: 9.3 ms, with 24 and the less L1 they leave 9.45), 24 for deeper ones as far as
+// the stack of both levels stays within 36 words, the most with which four blocks fit an SM
+// (the 4K terrain frame 23.9 ms, with 38 words 26.8), and 12 at least.  640 x 360 frames of
+// 4,000 / 30,000 / 100,000 instances with 24: 4.1 / 6.9 / 11.7 ms; 12: 4.0 / 7.3 / 14.1
+// (the binary traversal 6.7 / 12.0 / 23.7).  Before kTopAgain, rays that overflowed were
+// traced again by the binary traversal: 4.1 / 14.3 / 39.7 ms.
+constexpr uint32_t kWideStack = 36, kTopLeast = 12, kTopShallow = 16, kTopMost = 24;
 
 // ------------------------------------------------------------- ray pools
 // A warp keeps kPool rays in shared memory (word k of slot s at [k * kPool + s]), two
@@ -94,8 +107,9 @@ enum WideWord : uint32_t {
   kwOX, kwOY, kwOZ, kwDX, kwDY, kwDZ,  // ray of the level
   kwCull,                              // box entry bound of the level
   kwGrp,                               // current group
-  kwCur,                               // current leaf: elements left << 26 | next element; TLAS: node or instance
-  kwSp,                                // stack entries | those of the TLAS level << 7 | instance << 12 | in a BLAS << 31
+  kwCur,                               // current leaf: elements left << 26 | next element; TLAS: node (children
+                                       // not to visit << 17) or instance
+  kwSp,                                // stack entries | those of the TLAS level << 7 | instance << 14 | in a BLAS << 31
   kwLen, kwSlack,                      // object distance per world distance; slack of the mesh
   kwExit,                              // an occlusion query is decided by a hit before it (world distance)
   kwFar,                               // box entry bound of an occlusion query (world)
@@ -205,7 +219,7 @@ __device__ __forceinline__ uint32_t wide_leaf(const DevScene& S, uint32_t& grp) 
 
 // The next group of the BLAS, or its end; kwSp holds the new stack.
 __device__ __forceinline__ uint32_t wide_pop(const WideRay& R, uint32_t spx) {
-  const bool some = (spx & 0x7fu) > ((spx >> 7) & 0x1fu);
+  const bool some = (spx & 0x7fu) > ((spx >> 7) & 0x7fu);
   if (some) {
     --spx;
     R.set(kwGrp, R.stack(spx & 0x7fu));
@@ -219,9 +233,10 @@ __device__ __forceinline__ uint32_t wide_top_pop(const WideRay& R, uint32_t sp, 
   uint32_t next = kwDone;
   while (sp > 0u) {
     const uint32_t e = R.stack(--sp);
-    if (__uint_as_float((e >> 18) << 17) > bound) continue;
-    R.set(kwCur, (e >> 1) & ((1u << kTopIndexBits) - 1u));
-    next = e & 1u ? kwInstance : kwNode;
+    const bool again = e >= kTopAgain;
+    if (!again && __uint_as_float((e >> 18) << 17) > bound) continue;
+    R.set(kwCur, again ? e & ~kTopAgain : (e >> 1) & kTopIndexMask);
+    next = !again && (e & 1u) ? kwInstance : kwNode;
     break;
   }
   R.set(kwSp, sp);
@@ -316,7 +331,8 @@ __device__ __forceinline__ uint32_t wide_node(const WideRay& R, const DevScene& 
     if (rest >> 24) R.stack(spx++ & 0x7fu) = rest;
   }
   float tn[8];
-  const uint4* np = (blas ? S.wide_blas : S.wide_tlas) + (size_t)at * (kWideNodeWords / 4);
+  const uint32_t node = blas ? at : at & kTopIndexMask;
+  const uint4* np = (blas ? S.wide_blas : S.wide_tlas) + (size_t)node * (kWideNodeWords / 4);
   const WideTest w = wide_test(np, R.f3(kwOX), rinv, R.f(kwCull), [&](int k, float t) { tn[k] = t; });
   const uint32_t ih = ~w.miss & ((1u << w.ni) - 1u), lh = ~w.miss & (0xff00u >> w.nl) & 0xffu;
   if (blas) {
@@ -338,10 +354,14 @@ __device__ __forceinline__ uint32_t wide_node(const WideRay& R, const DevScene& 
   }
   const float rec_t = R.f(kwRecT), slack = S.wide_slack;
   const float bound = fminf(wide_bound(rec_t, kLeastSlack), R.f(kwFar));
-  const uint32_t hit = ih | lh;
+  uint32_t hit = (ih | lh) & ~(at >> kTopIndexBits);
   uint32_t sp = spx;
   if (hit) {
-    if (sp + __popc(hit) > cfg.stack_top) return kwRedo;
+    if (sp + __popc(hit) > cfg.stack_top) {
+      const uint32_t rest = hit & (hit - 1u);
+      if (rest) R.stack(sp++) = kTopAgain | ((rest ^ 0xffu) << kTopIndexBits) | node;
+      hit ^= rest;
+    }
     const uint4 ra = __ldg(np + 1), rb = __ldg(np + 5);  // references of the leaves
     const uint32_t ref[8] = {ra.x, rb.w, rb.z, rb.y, rb.x, ra.w, ra.z, ra.y};
     const uint32_t child = w.child & kWideIndexMask;
@@ -428,7 +448,7 @@ __device__ __forceinline__ uint32_t wide_tri(const WideRay& R, const DevScene& S
     if (w < best) {
       R.setf(kwRecT, w);
       R.set(kwRecSlot, slot);
-      R.set(kwRecInst, (R.u(kwRecInst) & ~kInstMask) | ((spx >> 12) & kInstMask));
+      R.set(kwRecInst, (R.u(kwRecInst) & ~kInstMask) | ((spx >> 14) & kInstMask));
       R.setf(kwCull, fminf(wide_bound(M, R.f(kwSlack)) * len, R.f(kwCull)));
     }
     if (decided) return kwVerify;
@@ -463,7 +483,7 @@ __device__ __forceinline__ uint32_t wide_instance(const WideRay& R, const DevSce
   const float rec_t = R.f(kwRecT), far = R.f(kwFar);
   if (sp & kInBlas) {
     const uint32_t next =
-        wide_top_pop(R, (sp >> 7) & 0x1fu, fminf(wide_bound(rec_t, kLeastSlack), far), rec_t);
+        wide_top_pop(R, (sp >> 7) & 0x7fu, fminf(wide_bound(rec_t, kLeastSlack), far), rec_t);
     if (next == kwNode) wide_world(R, S, wo, wd, rec_t, far);
     if (next != kwInstance) return next;
     sp = R.u(kwSp);
@@ -474,7 +494,7 @@ __device__ __forceinline__ uint32_t wide_instance(const WideRay& R, const DevSce
   const float4 wx = __ldg(ip + 4);
   float3 o, d;
   const float len = wide_object_ray(w2o, wo, wd, o, d);
-  R.set(kwSp, sp | (sp << 7) | (inst << 12) | kInBlas);
+  R.set(kwSp, sp | (sp << 7) | (inst << 14) | kInBlas);
   R.setf3(kwOX, o);
   R.setf3(kwDX, d);
   R.setf(kwLen, len);

@@ -149,3 +149,22 @@ def test_hits_equal_the_oracle(ctx, kind, quirks):
         assert np.array_equal(got[a], ref[b])
     for k in "uv":
         assert np.array_equal(got[k].view(np.uint32), ref[k].view(np.uint32))
+
+
+@pytest.mark.parametrize("count,box", [(300, 2.0), (3000, 2.0), (3000, 6.0), (20000, 3.0)])
+def test_more_children_than_the_stack_takes(ctx, count, box):
+    """Instances that overlap many times over: rays enter more boxes of the instance tree
+    than its part of the stack takes, from its third level down."""
+    meshes, instances = _spheres(count, 1, box, 9, lambda rng: rng.uniform(0.3, 1.0))
+    sb = oracle.assemble(meshes, MAT * 8, instances, 20, 4, 2, 1)
+    rays = _rays(box, np.zeros(3), 12)
+    ref = oracle.trace(sb, rays)
+    sc = Scene(ctx)
+    ids = [sc.upload_mesh(m, 20, 4) for m in meshes]
+    sc.set_materials(MAT * 8)
+    sc.set_instances(instances, ids, 2, 1)
+    got = sc.trace(rays)
+    sc.close()
+    assert np.array_equal(got["t"].view(np.uint32), ref["t"].view(np.uint32))
+    for a, b in (("instance_index", "instance"), ("triangle_index", "triangle")):
+        assert np.array_equal(got[a], ref[b])
