@@ -873,7 +873,7 @@ cudaError_t wf_render_gi(const TraceCfg& tc, const WfScene& scene, const float4*
                one.S.wide_top);
   L.wide = wide_allowed(tcs, one.S);
   L.one = &one;
-  if (L.wide && !wf_segments) L.wf_segments = kDefaultWideSegments;
+  if (L.wide && !wf_segments) L.wf_segments = wide_segments(1, L.total_paths);
   cudaError_t e = wf_upload_table(&one, 1, B.table, st);
   if (e != cudaSuccess) return e;
   if (launches) *launches += 1;
@@ -915,7 +915,7 @@ cudaError_t wf_render(int mode, const TraceCfg& tc, const WfScene* scenes, uint3
   if (n == 1) L.one = tab;
   L.wide = true;  // one scene that cannot keeps the batch on the binary traversal
   for (uint32_t i = 0; i < n; ++i) L.wide = L.wide && wide_allowed(tcs, tab[i].S);
-  if (L.wide && !wf_segments) L.wf_segments = kDefaultWideSegments;
+  if (L.wide && !wf_segments) L.wf_segments = wide_segments(mode, L.total_paths);
   cudaError_t e = wf_upload_table(tab, n, B.table, st);
   if (e != cudaSuccess) return e;
   if (launches) *launches += (n + kTableChunk - 1) / kTableChunk;

@@ -15,9 +15,20 @@ constexpr uint32_t kWfTailOnly = 0xffffffffu;
 // from 2 to 3; the realtime GI frame is fastest at 2).
 constexpr uint32_t kDefaultWfSegments = 3;
 constexpr uint32_t kDefaultGiWfSegments = 2;
-// The same with the eight-wide traversal: its launches drain quickly, and the tail's
-// shading thrashes the instruction cache beside the traversal's code.
-constexpr uint32_t kDefaultWideSegments = 16;
+// The same with the eight-wide traversal.  A wavefront segment costs its launches and the
+// drain of its last rays (25 to 80 us), the tail kernel more for every path (its shading
+// competes with the traversal's code for the instruction cache), so the tail starts the
+// later the more paths there are, and earlier in mode 0, whose roulette ends more of them.
+// Frames of depth 16 with 3 / this many / 16 segments, in us: Cornell mode 2, 128 x 72 455 / 474 /
+// 672, 1066 x 599 2195 / 1425 / 1515, 1080p 4352 / 2960 / 2951; 50 spheres mode 2, 341 x 191
+// 1567 / 1739 / 2094, 1080p 6361 / 5450 / 5347; mode 0, 341 x 191 883 / 883 / 1246, 1080p
+// 3028 / 3101 / 3687; Cornell mode 1, 341 x 191 663 / 598 / 752.
+inline uint32_t wide_segments(int mode, uint32_t paths) {
+  uint32_t log2 = 0;
+  while (paths >> 1 >> log2) ++log2;
+  const uint32_t s = log2 > 9u ? log2 - 9u : 0u, by_mode = mode == 0 ? s / 2u : s;
+  return by_mode > 3u ? by_mode : 3u;
+}
 // Traversal blocks per SM when the parameter is 0: eight 128-thread blocks of
 // a 64-register budget fill the register file (1080p sphere frame: 5 blocks
 // 138.7, 6 blocks 140.9, 8 blocks 143.7 Mpaths/s; the spills of the 64-register

@@ -71,14 +71,14 @@ __device__ void quantize(uint32_t* words, const Boxes& c, uint32_t used, uint32_
     const double need = fmax(fmax(((double)hi - lo) / 254.0, mag * 7.63e-6), 1e-30);
     int e;
     frexp(need, &e);  // need <= 2^e
-    const double s = ldexp(1.0, e);
-    const float p = __double2float_rd((double)lo - s / 32.0);
+    const double s = ldexp(1.0, e), inv = ldexp(1.0, -e);  // (powers of two: the products are the quotients)
+    const float p = __double2float_rd((double)lo - s * (1.0 / 32.0));
     words[j] = __float_as_uint(p);
     words[3] |= (uint32_t)(e + 127 + 15) << (8 * j);
     for (uint32_t k = 0; k < 8; ++k) {
       if (!(used & (1u << k))) continue;
-      const double ql = floor((c.lo[k][j] - (double)p) / s - 1.0 / 64.0);
-      const double qh = ceil((c.hi[k][j] - (double)p) / s + 1.0 / 64.0);
+      const double ql = floor((c.lo[k][j] - (double)p) * inv - 1.0 / 64.0);
+      const double qh = ceil((c.hi[k][j] - (double)p) * inv + 1.0 / 64.0);
       if (!(ql >= 0.0) || !(qh <= 255.0)) bad = true;
       q8[16 * j + k] = (uint8_t)ql;
       q8[16 * j + 8 + k] = (uint8_t)qh;

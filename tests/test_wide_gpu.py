@@ -12,7 +12,7 @@ import pytest
 import oracle
 from pulse_b200 import scenes
 from pulse_b200.layout import Instance, Material, Mesh
-from pulse_b200.tracer import Scene
+from pulse_b200.tracer import Scene, Target, render_forward
 
 pytestmark = pytest.mark.gpu
 
@@ -168,3 +168,26 @@ def test_more_children_than_the_stack_takes(ctx, count, box):
     assert np.array_equal(got["t"].view(np.uint32), ref["t"].view(np.uint32))
     for a, b in (("instance_index", "instance"), ("triangle_index", "triangle")):
         assert np.array_equal(got[a], ref[b])
+
+
+@pytest.mark.parametrize("segments", [0, 1, 2, 6, 8, 0xFFFFFFFF])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_frames_equal_the_oracle(ctx, mode, segments):
+    """Two accumulated frames of two samples at the default and at every other place of
+    the tail kernel: after the first segment, the last but one, the last, never, at once."""
+    d = scenes.cornell(67, 41)
+    params = dict(max_depth=7, nee_mode=mode, light_pick=1 if mode == 2 else 0, quirks=1, spp=2)
+    sb = oracle.assemble(d.meshes, d.materials, d.instances, 20, 4)
+    sc = Scene(ctx)
+    ids = [sc.upload_mesh(m, 20, 4) for m in d.meshes]
+    sc.set_materials(d.materials)
+    sc.set_instances(d.instances, ids)
+    tg = Target(ctx, d.width, d.height)
+    ref = np.zeros((d.height, d.width, 4), np.float32)
+    for acc in range(2):
+        render_forward(sc, d.view, tg, acc, wf_segments=segments, **params)
+        oracle.render(sb, d.view, d.width, d.height, acc, image=ref, **params)
+    got = tg.download()
+    tg.close()
+    sc.close()
+    assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
