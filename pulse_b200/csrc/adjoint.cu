@@ -320,7 +320,7 @@ cudaError_t launch_backward(const DevScene& S, const TraceCfg& tc, const PathCfg
   const int trace_grid = sms * (int)(trace_blocks ? trace_blocks : kDefaultTraceBlocks);
   const bool wide = wide_allowed(tc, S);
   uint32_t n = 0;
-  e = cudaMemsetAsync(B.counts, 0, 8 * sizeof(uint32_t), st);
+  e = cudaMemsetAsync(B.counts, 0, kCounts * sizeof(uint32_t), st);
   if (e != cudaSuccess) return e;
   k_adj_generate<<<light_blocks, kAdjBlock, 0, st>>>(pc, fc, B, rec, dimg, one.paths);
   ++n;

@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(BS, MINB * kWfBlock / BS) k_wf_extend(TraceCfg
 constexpr int kShadeBlocks = 8;
 
 template <int MODE, bool COUNT>
-__global__ void __launch_bounds__(kWfBlock, kShadeBlocks) k_wf_shade(WfBuffers B, uint32_t n_scenes, int qi,
+__global__ void __launch_bounds__(kWfBlock, kShadeBlocks) k_wf_shade(WfBuffers B, uint32_t n_scenes, int qi, int sq,
                                                        unsigned long long* work) {
   extern __shared__ uint32_t smem[];
   const WfScene* tab = load_table(B.table, n_scenes, smem);
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(kWfBlock, kShadeBlocks) k_wf_shade(WfBuffers B
     }
     const uint32_t ns = warp_append(alive, B.counts + (qi ^ 1));
     if (alive) qn[ns] = p;
-    const uint32_t ss = warp_append(shadow, B.counts + 2);
+    const uint32_t ss = warp_append(shadow, B.counts + sq);
     if (i < n) store_state(B, p, ps);
     if (shadow) {
       put_shadow(B, ss, rq, p, sid);
@@ -533,13 +533,16 @@ __global__ void __launch_bounds__(kWfBlock) k_sort_scatter(WfBuffers B, uint32_t
 __global__ void k_wf_reset(uint32_t* counts, int next, int snap) {
   if (threadIdx.x == 0) {
     counts[3] = snap ? counts[2] : 0u;
-    counts[next] = 0; counts[2] = 0; counts[4] = 0; counts[5] = 0; counts[6] = 0;
+    counts[next] = 0; counts[2] = 0;
+    for (int i = kCountExtend; i < kCounts; ++i) counts[i] = 0;
   }
 }
 
 struct WfTableChunk { WfScene e[kTableChunk]; };
 
-__global__ void k_wf_set_table(WfTableChunk c, WfScene* dst, uint32_t k) {
+// Also zeros the counters at `counts`, unless it is null.
+__global__ void k_wf_set_table(WfTableChunk c, WfScene* dst, uint32_t k, uint32_t* counts) {
+  if (counts && threadIdx.x < kCounts) counts[threadIdx.x] = 0u;
   const uint4* src = reinterpret_cast<const uint4*>(c.e);
   uint4* d = reinterpret_cast<uint4*>(dst);
   const uint32_t words = k * (uint32_t)(sizeof(WfScene) / sizeof(uint4));
@@ -669,9 +672,9 @@ uint32_t record_segments(const TraceCfg& tc, const WfBuffers& B, const WfLaunch&
   const bool wide = L.wide && !COUNT;
   uint32_t n = 0;
   const uint32_t wf = L.wf_segments < L.segments ? L.wf_segments : L.segments;
-  int qi = 0;
+  int qi = 0, sq = kCountRequests;
   auto resolve = [&]() {
-    if (wide) wide_shadow(MODE, tc, B, L, ctr, st);
+    if (wide) wide_shadow(MODE, tc, B, L, sq, ctr, st);
     else shadow<<<grid, tb, smem_tr, st>>>(tc, B, ns, ctr, work);
     ++n;
     pending = false;
@@ -688,12 +691,17 @@ uint32_t record_segments(const TraceCfg& tc, const WfBuffers& B, const WfLaunch&
       n += 3;
       qi ^= 1;
     }
-    k_wf_reset<<<1, 32, 0, st>>>(B.counts, qi ^ 1, pending ? 1 : 0);
-    if (wide) wide_extend(pending ? MODE : -1, tc, B, L, qi, ctr, st);
-    else (pending ? extend_sh : extend)<<<grid, tb, smem_tr, st>>>(tc, B, ns, qi, ctr, work);
+    if (wide) {
+      wide_extend(pending ? MODE : -1, tc, B, L, qi, sq, ctr, st);
+      sq ^= 1;
+    } else {
+      k_wf_reset<<<1, 32, 0, st>>>(B.counts, qi ^ 1, pending ? 1 : 0);
+      (pending ? extend_sh : extend)<<<grid, tb, smem_tr, st>>>(tc, B, ns, qi, ctr, work);
+      ++n;
+    }
     pending = false;
-    k_wf_shade<MODE, COUNT><<<L.sms * kShadeBlocks, kWfBlock, g.tab, st>>>(B, ns, qi, work);
-    n += 3;
+    k_wf_shade<MODE, COUNT><<<L.sms * kShadeBlocks, kWfBlock, g.tab, st>>>(B, ns, qi, sq, work);
+    n += 2;
     if (MODE != 0) {
       if (merge && seg + 1 < wf) pending = true;
       else resolve();
@@ -702,10 +710,14 @@ uint32_t record_segments(const TraceCfg& tc, const WfBuffers& B, const WfLaunch&
   }
   if (pending) resolve();  // no wavefront segment follows (no bounce, or tail only)
   if (!COUNT && wf < L.segments) {
-    k_wf_reset<<<1, 32, 0, st>>>(B.counts, qi ^ 1, 0);
-    if (wide) wide_tail(MODE, tc, B, L, qi, ctr, st);
-    else tail<<<grid, tb, smem_tr, st>>>(tc, B, ns, qi, ctr);
-    n += 2;
+    if (wide) {
+      wide_tail(MODE, tc, B, L, qi, ctr, st);
+    } else {
+      k_wf_reset<<<1, 32, 0, st>>>(B.counts, qi ^ 1, 0);
+      tail<<<grid, tb, smem_tr, st>>>(tc, B, ns, qi, ctr);
+      ++n;
+    }
+    ++n;
   }
   return n;
 }
@@ -715,16 +727,12 @@ cudaError_t record(const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, Co
                    uint32_t* launches, cudaStream_t st) {
   const Shapes g = shapes(tc, L);
   const uint32_t ns = L.n_scenes;
-  cudaError_t e = cudaMemsetAsync(B.counts, 0, 8 * sizeof(uint32_t), st);
-  if (e != cudaSuccess) return e;
   uint32_t n = 0;
   k_wf_generate<MODE><<<g.light_blocks, kWfBlock, g.tab, st>>>(B, ns, L.total_paths);
   ++n;
   n += record_segments<MODE, COUNT>(tc, B, L, ctr, work, st);
-  if (L.image_wait) {
-    e = cudaStreamWaitEvent(st, L.image_wait, 0);
-    if (e != cudaSuccess) return e;
-  }
+  if (L.image_wait)
+    if (cudaError_t e = cudaStreamWaitEvent(st, L.image_wait, 0)) return e;
   k_wf_accumulate<<<g.light_blocks, kWfBlock, g.tab, st>>>(B, ns);
   ++n;
   if (launches) *launches += n;
@@ -739,7 +747,7 @@ cudaError_t record_gi(const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L,
   const float spp_inv = 1.0f / (float)spp;
   uint32_t n = 0;
   for (uint32_t s = 0; s < spp; ++s) {
-    cudaError_t e = cudaMemsetAsync(B.counts, 0, 8 * sizeof(uint32_t), st);
+    cudaError_t e = cudaMemsetAsync(B.counts, 0, kCounts * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
     k_gi_generate<<<g.light_blocks, kWfBlock, g.tab, st>>>(B, gbuf, gw, gh, s);
     n += 1 + record_segments<1, false>(tc, B, L, ctr, nullptr, st, true);
@@ -785,13 +793,13 @@ cudaError_t wf_record(int mode, const TraceCfg& tc, const WfBuffers& B, const Wf
   }
 }
 
-cudaError_t wf_upload_table(const WfScene* host, uint32_t n, WfScene* dev, cudaStream_t st) {
+cudaError_t wf_upload_table(const WfScene* host, uint32_t n, const WfBuffers& B, cudaStream_t st) {
   for (uint32_t i = 0; i < n; i += kTableChunk) {
     WfTableChunk c;
     std::memset(&c, 0, sizeof(c));
     const uint32_t k = n - i < kTableChunk ? n - i : kTableChunk;
     std::memcpy(c.e, host + i, k * sizeof(WfScene));
-    k_wf_set_table<<<1, 128, 0, st>>>(c, dev + i, k);
+    k_wf_set_table<<<1, 128, 0, st>>>(c, B.table + i, k, i ? nullptr : B.counts);
   }
   return cudaGetLastError();
 }
@@ -805,7 +813,7 @@ cudaError_t wf_extend_step(const TraceCfg& tc, const WfBuffers& B, int qi, uint3
     L.one = wide;
     L.trace_blocks_per_sm = trace_blocks;
     L.sms = device_sms();
-    wide_extend(-1, tc, B, L, qi, ctr, st);
+    wide_extend(-1, tc, B, L, qi, kCountRequests, ctr, st);
     return cudaGetLastError();
   }
   const uint32_t tbps = trace_blocks ? trace_blocks : kDefaultTraceBlocks;
@@ -833,8 +841,7 @@ cudaError_t wf_gbuffer_primary(const TraceCfg& tc, const WfScene& scene, float4*
   const int sms = device_sms();
   const size_t tab = sizeof(WfScene);
   const size_t smem = tab + (size_t)trace_smem_words(tcs) * kWfBlock * 4;
-  cudaError_t e = wf_upload_table(&one, 1, B.table, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(B.counts, 0, 8 * sizeof(uint32_t), st);
+  cudaError_t e = wf_upload_table(&one, 1, B, st);
   if (e != cudaSuccess) return e;
   k_gbuf_generate<<<sms * 16, kWfBlock, tab, st>>>(B);
   if (wide_allowed(tcs, one.S)) {
@@ -843,7 +850,7 @@ cudaError_t wf_gbuffer_primary(const TraceCfg& tc, const WfScene& scene, float4*
     L.one = &one;
     L.trace_blocks_per_sm = trace_blocks;
     L.sms = sms;
-    wide_extend(-1, tcs, B, L, 0, ctr, st);
+    wide_extend(-1, tcs, B, L, 0, kCountRequests, ctr, st);
   } else {
     extend_kernel<false>(budget(tbps))<<<sms * (int)tbps, kWfBlock, smem, st>>>(tcs, B, 1, 0, ctr, nullptr);
   }
@@ -874,7 +881,7 @@ cudaError_t wf_render_gi(const TraceCfg& tc, const WfScene& scene, const float4*
   L.wide = wide_allowed(tcs, one.S);
   L.one = &one;
   if (L.wide && !wf_segments) L.wf_segments = wide_segments(1, L.total_paths);
-  cudaError_t e = wf_upload_table(&one, 1, B.table, st);
+  cudaError_t e = wf_upload_table(&one, 1, B, st);
   if (e != cudaSuccess) return e;
   if (launches) *launches += 1;
   return record_gi(tcs, B, L, gbuf, gw, gh, scene.pc.spp, one.image, ctr, launches, st);
@@ -916,7 +923,7 @@ cudaError_t wf_render(int mode, const TraceCfg& tc, const WfScene* scenes, uint3
   L.wide = true;  // one scene that cannot keeps the batch on the binary traversal
   for (uint32_t i = 0; i < n; ++i) L.wide = L.wide && wide_allowed(tcs, tab[i].S);
   if (L.wide && !wf_segments) L.wf_segments = wide_segments(mode, L.total_paths);
-  cudaError_t e = wf_upload_table(tab, n, B.table, st);
+  cudaError_t e = wf_upload_table(tab, n, B, st);
   if (e != cudaSuccess) return e;
   if (launches) *launches += (n + kTableChunk - 1) / kTableChunk;
   return wf_record(mode, tcs, B, L, ctr, work, launches, st);

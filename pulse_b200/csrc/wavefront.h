@@ -55,10 +55,16 @@ struct WfBuffers {
   float* h1;        // per path: v
   uint32_t* q[2];   // ping-pong queues of live path ids
   float4* shadow;   // 4 x float4 per shadow request
-  uint32_t* counts; // [q0, q1, shadow, unused, extend cursor, shadow cursor, tail cursor, unused]
+  uint32_t* counts; // [q0, q1, shadow requests (two), extend cursors (two), tail cursor, shadow cursor]
   WfScene* table;   // kMaxBatch entries
   uint32_t* sort_bins;  // kSortBins counters of the ray sort
 };
+
+// Indexes of WfBuffers::counts.  With the wide traversal a segment's shading lists its
+// shadow requests under the count that its extend does not read, in turn (kCountRequests or
+// the next), and each extend takes the cursor of the one it reads.  The binary kernels
+// take the first of both.
+constexpr int kCountRequests = 2, kCountExtend = 4, kCountTail = 6, kCountShadow = 7, kCounts = 8;
 
 // Bins of the ray sort: direction octant (3 bits) x origin cell (8^3).
 constexpr uint32_t kSortBins = 4096;
@@ -96,15 +102,15 @@ inline WfBuffers wf_carve(void* base, size_t paths) {
   B.h1 = (float*)take(paths * 4);
   B.q[0] = (uint32_t*)take(paths * 4);
   B.q[1] = (uint32_t*)take(paths * 4);
-  B.counts = (uint32_t*)take(8 * sizeof(uint32_t));
+  B.counts = (uint32_t*)take(kCounts * sizeof(uint32_t));
   B.table = (WfScene*)take((size_t)kMaxBatch * sizeof(WfScene));
   B.sort_bins = (uint32_t*)take(kSortBins * 4);
   return B;
 }
 
-// Writes n table entries from host memory to dev with small kernels (the
+// Writes n table entries from host memory to B.table and zeros B.counts with small kernels (the
 // entries travel as kernel parameters: no host staging, capturable).
-cudaError_t wf_upload_table(const WfScene* host, uint32_t n, WfScene* dev, cudaStream_t st);
+cudaError_t wf_upload_table(const WfScene* host, uint32_t n, const WfBuffers& B, cudaStream_t st);
 
 // Enqueue one frame of the scenes already in B.table (no host synchronisation,
 // so a stream capture of it is a complete frame).
@@ -152,11 +158,13 @@ cudaError_t wf_reset_step(const WfBuffers& B, int next, cudaStream_t st);
 // The frame's traversal launches with the eight-wide trees (wavefront_wide.cu), for
 // launches whose scenes all allow it (pt_wide.cuh); errors are left for
 // cudaGetLastError.  shadow: the estimator mode whose previous segment's shadow requests
-// the extend also resolves, or -1.
+// the extend also resolves, or -1; sq: the count of those (kCountRequests or the next).  An
+// extend zeros the counts and cursors of the launches after it.
 cudaError_t wide_prepare(int mode);
-void wide_extend(int shadow, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, int qi, Counters* ctr,
+void wide_extend(int shadow, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, int qi, int sq, Counters* ctr,
                  cudaStream_t st);
-void wide_shadow(int mode, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, Counters* ctr, cudaStream_t st);
+void wide_shadow(int mode, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, int sq, Counters* ctr,
+                 cudaStream_t st);
 void wide_tail(int mode, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, int qi, Counters* ctr,
                cudaStream_t st);
 // The adjoint's shadow rays: visible ones set flag in word 3 (w) of their path's record.

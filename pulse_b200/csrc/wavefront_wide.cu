@@ -94,21 +94,29 @@ __device__ __forceinline__ Scenes<ONE> block_scenes(const WfScene& one, const Wf
 template <int SHADOW, bool ONE, int BS>
 __global__ void __launch_bounds__(BS, kWideBlocks * kWfBlock / BS)
     k_wide_extend(const __grid_constant__ TraceCfg tc, const __grid_constant__ WfBuffers B,
-                  const __grid_constant__ WfScene one, uint32_t n_table, int qi, Counters* ctr) {
+                  const __grid_constant__ WfScene one, uint32_t n_table, int qi, int sq, Counters* ctr) {
   extern __shared__ uint32_t smem[];
   const uint32_t n = B.counts[qi];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    // nothing of this launch reads these: the next queue's and the next shadow requests'
+    // counts, the other cursors (a launch of its own for them took 2 to 3 us a segment)
+    B.counts[qi ^ 1] = 0u;
+    B.counts[sq ^ 1] = 0u;
+    B.counts[kCountExtend + (sq & 1 ^ 1)] = 0u;
+    B.counts[kCountShadow] = 0u;
+  }
   ExtendItem<SHADOW, ONE> it{block_scenes<ONE>(one, B, n_table, smem), B, tc, B.q[qi], n};
-  wide_run(it, tc, warp_pool(smem, n_table, tc), B.counts + 4, SHADOW >= 0 ? n + B.counts[3] : n, ctr);
+  wide_run(it, tc, warp_pool(smem, n_table, tc), B.counts + kCountExtend + (sq & 1), SHADOW >= 0 ? n + B.counts[sq] : n, ctr);
 }
 
 // The last segment's shadow requests.
 template <int MODE, bool ONE, int BS>
 __global__ void __launch_bounds__(BS, kWideBlocks * kWfBlock / BS)
     k_wide_shadow(const __grid_constant__ TraceCfg tc, const __grid_constant__ WfBuffers B,
-                  const __grid_constant__ WfScene one, uint32_t n_table, Counters* ctr) {
+                  const __grid_constant__ WfScene one, uint32_t n_table, int sq, Counters* ctr) {
   extern __shared__ uint32_t smem[];
   ExtendItem<MODE, ONE> it{block_scenes<ONE>(one, B, n_table, smem), B, tc, nullptr, 0u};
-  wide_run(it, tc, warp_pool(smem, n_table, tc), B.counts + 5, B.counts[2], ctr);
+  wide_run(it, tc, warp_pool(smem, n_table, tc), B.counts + kCountShadow, B.counts[sq], ctr);
 }
 
 // Every path still alive, to its end: a finished ray's slot waits for its shading (or for
@@ -174,7 +182,7 @@ __global__ void __launch_bounds__(BS, kWideBlocks * kWfBlock / BS)
                 const __grid_constant__ WfScene one, uint32_t n_table, int qi, Counters* ctr) {
   extern __shared__ uint32_t smem[];
   TailItem<MODE, ONE> it{block_scenes<ONE>(one, B, n_table, smem), B, tc, B.q[qi]};
-  wide_run(it, tc, warp_pool(smem, n_table, tc), B.counts + 6, B.counts[qi], ctr);
+  wide_run(it, tc, warp_pool(smem, n_table, tc), B.counts + kCountTail, B.counts[qi], ctr);
 }
 
 // The adjoint's shadow requests: visibility only.
@@ -215,7 +223,7 @@ __global__ void __launch_bounds__(kWfBlock, kWideBlocks) k_wide_adj_shadow(const
                                                                            Counters* ctr) {
   extern __shared__ uint32_t smem[];
   AdjShadowItem it{S, B, tc, rec, rows, flag};
-  wide_run(it, tc, warp_pool(smem, 0u, tc), B.counts + 5, B.counts[2], ctr);
+  wide_run(it, tc, warp_pool(smem, 0u, tc), B.counts + kCountShadow, B.counts[2], ctr);
 }
 
 struct RayItem {
@@ -306,7 +314,7 @@ cudaError_t wide_prepare(int mode) {
   return e;
 }
 
-void wide_extend(int shadow, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, int qi, Counters* ctr,
+void wide_extend(int shadow, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, int qi, int sq, Counters* ctr,
                  cudaStream_t st) {
   const Shape g = shape(tc, L);
   by_shape(g.block, L.one != nullptr, [&](auto bs, auto on) {
@@ -315,17 +323,18 @@ void wide_extend(int shadow, const TraceCfg& tc, const WfBuffers& B, const WfLau
     const auto k = shadow == 1   ? k_wide_extend<1, ONE, BS>
                    : shadow == 2 ? k_wide_extend<2, ONE, BS>
                                  : k_wide_extend<-1, ONE, BS>;
-    k<<<g.grid, g.block, g.smem, st>>>(tc, B, ONE ? *L.one : WfScene{}, ONE ? 0u : L.n_scenes, qi, ctr);
+    k<<<g.grid, g.block, g.smem, st>>>(tc, B, ONE ? *L.one : WfScene{}, ONE ? 0u : L.n_scenes, qi, sq, ctr);
   });
 }
 
-void wide_shadow(int mode, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, Counters* ctr, cudaStream_t st) {
+void wide_shadow(int mode, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, int sq, Counters* ctr,
+                 cudaStream_t st) {
   const Shape g = shape(tc, L);
   by_shape(g.block, L.one != nullptr, [&](auto bs, auto on) {
     constexpr int BS = decltype(bs)::value;
     constexpr bool ONE = decltype(on)::value;
     const auto k = mode == 1 ? k_wide_shadow<1, ONE, BS> : k_wide_shadow<2, ONE, BS>;
-    k<<<g.grid, g.block, g.smem, st>>>(tc, B, ONE ? *L.one : WfScene{}, ONE ? 0u : L.n_scenes, ctr);
+    k<<<g.grid, g.block, g.smem, st>>>(tc, B, ONE ? *L.one : WfScene{}, ONE ? 0u : L.n_scenes, sq, ctr);
   });
 }
 
