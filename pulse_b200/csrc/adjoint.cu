@@ -61,14 +61,42 @@ struct GradSink {
     if (m < kGradSlots) atomicAdd(smem + m * kGradStride + field, v);
     else atomicAdd(global + (size_t)m * kGradStride + field, v);
   }
-  // d loss / d (base, roughness) of material m through d gv (coef = delta * dL/dgv).
-  __device__ __forceinline__ void bsdf(uint32_t m, float3 coef, const float3& db, const float3& dr) const {
-    add(m, 0, coef.x * db.x);
-    add(m, 1, coef.y * db.y);
-    add(m, 2, coef.z * db.z);
-    add(m, 6, coef.x * dr.x + coef.y * dr.y + coef.z * dr.z);
+  // Adds v[0..3) to fields field.. and v[3], if there is one, to the roughness's of material m
+  // for every lane of the (whole) warp with m below n_mat: lanes of the same material are
+  // summed first where there are kShare of them, as additions to one shared word run one
+  // after another (backward pass of the 256^2 x 16 Cornell workload 4330 -> 4130 us; the first
+  // resolve was 196 us of it; kShare 1 4166, 8 4141).
+  template <int N>
+  __device__ __forceinline__ void add_warp(uint32_t m, int field, const float (&v)[N]) const {
+    constexpr int kShare = 3;
+    uint32_t left = __ballot_sync(0xffffffffu, m < n_mat);
+    while (left) {
+      const uint32_t lead = __ffs(left) - 1u, m0 = __shfl_sync(0xffffffffu, m, (int)lead);
+      const bool mine = m == m0;
+      const uint32_t same = __ballot_sync(0xffffffffu, mine);
+      left &= ~same;
+      if (__popc(same) < kShare) {
+        if (mine)
+          for (int i = 0; i < N; ++i) add(m, i < 3 ? field + i : 6, v[i]);
+        continue;
+      }
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        float x = mine ? v[i] : 0.0f;
+        for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+        if (lane_id() == lead) add(m0, i < 3 ? field + i : 6, x);
+      }
+    }
   }
 };
+
+// d loss / d (base, roughness) through d gv (coef = delta * dL/dgv), added to g.
+__device__ __forceinline__ void add_bsdf(float (&g)[4], float3 coef, const float3& db, const float3& dr) {
+  g[0] += coef.x * db.x;
+  g[1] += coef.y * db.y;
+  g[2] += coef.z * db.z;
+  g[3] += coef.x * dr.x + coef.y * dr.y + coef.z * dr.z;
+}
 
 __device__ __forceinline__ GradSink grad_begin(uint32_t* smem, float* grads, uint32_t n_mat) {
   const uint32_t slots = n_mat < kGradSlots ? n_mat : kGradSlots;
@@ -131,7 +159,8 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_shade(DevScene S, PathCfg pc,
   for (uint32_t base = warp_base; base < n; base += gridDim.x * blockDim.x) {
     const uint32_t i = base + lane_id();
     bool alive = false, shadow = false;
-    uint32_t p = 0;
+    uint32_t p = 0, me = 0xffffffffu;  // no light was hit
+    float ge[3] = {0.0f, 0.0f, 0.0f};
     ShadowReq rq;
     rq.active = false;
     if (i < n) {
@@ -152,9 +181,10 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_shade(DevScene S, PathCfg pc,
         if (vr.w_le != 0.0f) {
           const float3 d = path_delta(dimg, p, pc.spp, inv_n);
           const Material m = load_material(S, vr.mat);
-          G.add(vr.mat, 3, d.x * vr.thr.x * vr.w_le);
-          G.add(vr.mat, 4, d.y * vr.thr.y * vr.w_le);
-          G.add(vr.mat, 5, d.z * vr.thr.z * vr.w_le);
+          me = vr.mat;
+          ge[0] = d.x * vr.thr.x * vr.w_le;
+          ge[1] = d.y * vr.thr.y * vr.w_le;
+          ge[2] = d.z * vr.thr.z * vr.w_le;
           L_rem = sub(L_rem, muls(mul(vr.thr, m.emissive), vr.w_le));
           r[5] = make_float4(L_rem.x, L_rem.y, L_rem.z, 0.0f);
         }
@@ -168,6 +198,7 @@ __global__ void __launch_bounds__(kAdjBlock) k_adj_shade(DevScene S, PathCfg pc,
         shadow = vr.nee;
       }
     }
+    G.add_warp(me, 3, ge);
     const uint32_t ns = warp_append(alive, B.counts + (qi ^ 1));
     if (alive) qn[ns] = p;
     const uint32_t ss = warp_append(shadow, B.counts + 2);
@@ -229,9 +260,8 @@ __global__ void __launch_bounds__(kAdjBlock, 8) k_adj_shadow(DevScene S, TraceCf
 
 // The NEE term (when its shadow ray reached the light) and the BSDF sample of
 // every vertex recorded for queue qi.
-// Eight blocks per SM (64 registers, 12 bytes of spill) rather than the seven
-// that 69 registers allow: backward pass of the 512^2 x 64 spp Cornell
-// workload 145.3 -> 143.1 ms.
+// Bound by issue and the latency of its loads.  Eight blocks per SM (64 registers, 28
+// bytes of spill): the pass takes 4130 us, with seven or six 4160 and 4175.
 __global__ void __launch_bounds__(kAdjBlock, 8) k_adj_resolve(DevScene S, PathCfg pc, WfBuffers B, float4* rec,
                                                            const float4* __restrict__ dimg, int qi, float* grads,
                                                            uint32_t n_mat) {
@@ -240,47 +270,56 @@ __global__ void __launch_bounds__(kAdjBlock, 8) k_adj_resolve(DevScene S, PathCf
   const float inv_n = 1.0f / __uint2float_rn(pc.spp);
   const uint32_t n = B.counts[qi];
   const uint32_t* q = B.q[qi];
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t p = q[i];
+  const uint32_t warp_base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;
+  for (uint32_t base = warp_base; base < n; base += gridDim.x * blockDim.x) {
+    const uint32_t i = base + lane_id();
+    uint32_t mi = 0xffffffffu, ml = 0xffffffffu;  // none
+    float gm[4] = {0.0f, 0.0f, 0.0f, 0.0f}, ge[3] = {0.0f, 0.0f, 0.0f};
+    const uint32_t p = i < n ? q[i] : 0u;
     float4* r = rec + kRec * (size_t)p;
-    const float4 a3 = r[3];
+    const float4 a3 = i < n ? r[3] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const uint32_t flags = __float_as_uint(a3.w);
-    if (!(flags & kVert)) continue;
-    const float4 a0 = r[0], a1 = r[1];
-    const float3 nn = xyz(a0), wo = xyz(a1), Tv = xyz(a3);
-    const uint32_t mi = __float_as_uint(a1.w);
-    const Material m = load_material(S, mi);
-    const Lobe lobe = lobe_at(nn, wo, m);
-    const float3 d = path_delta(dimg, p, pc.spp, inv_n);
-    float3 L_rem = xyz(r[5]);
-    float pb;
-    if ((flags & kNee) && (flags & kVisible)) {
-      const float4 a2 = r[2];
-      const float3 wl = xyz(a2);
-      const uint32_t ml = __float_as_uint(a2.w);
-      const float sc = a0.w;
-      float3 gl;
-      eval_lobe(nn, wo, wl, m, lobe, gl, pb);
-      const float3 Le = load_material(S, ml).emissive;
-      G.add(ml, 3, d.x * Tv.x * gl.x * sc);
-      G.add(ml, 4, d.y * Tv.y * gl.y * sc);
-      G.add(ml, 5, d.z * Tv.z * gl.z * sc);
-      float3 db, dr;
-      eval_g_grad(nn, wo, wl, m, db, dr);
-      G.bsdf(mi, muls(mul(mul(d, Tv), Le), sc), db, dr);
-      L_rem = sub(L_rem, muls(mul(mul(Tv, gl), Le), sc));
-      r[5] = make_float4(L_rem.x, L_rem.y, L_rem.z, 0.0f);
+    if (flags & kVert) {
+      const float4 a0 = r[0], a1 = r[1];
+      const float3 nn = xyz(a0), wo = xyz(a1), Tv = xyz(a3);
+      const uint32_t mat = __float_as_uint(a1.w);
+      const Material m = load_material(S, mat);
+      const Lobe lobe = lobe_at(nn, wo, m);
+      const float3 d = path_delta(dimg, p, pc.spp, inv_n);
+      float3 L_rem = xyz(r[5]);
+      float pb;
+      if ((flags & kNee) && (flags & kVisible)) {
+        const float4 a2 = r[2];
+        const float3 wl = xyz(a2);
+        mi = mat;
+        ml = __float_as_uint(a2.w);
+        const float sc = a0.w;
+        float3 gl;
+        eval_lobe(nn, wo, wl, m, lobe, gl, pb);
+        const float3 Le = load_material(S, ml).emissive;
+        ge[0] = d.x * Tv.x * gl.x * sc;
+        ge[1] = d.y * Tv.y * gl.y * sc;
+        ge[2] = d.z * Tv.z * gl.z * sc;
+        float3 db, dr;
+        eval_g_grad(nn, wo, wl, m, db, dr);
+        add_bsdf(gm, muls(mul(mul(d, Tv), Le), sc), db, dr);
+        L_rem = sub(L_rem, muls(mul(mul(Tv, gl), Le), sc));
+        r[5] = make_float4(L_rem.x, L_rem.y, L_rem.z, 0.0f);
+      }
+      if (flags & kCont) {
+        mi = mat;
+        const float3 wi = xyz(r[4]);
+        float3 gv;
+        eval_lobe(nn, wo, wi, m, lobe, gv, pb);
+        float3 db, dr;
+        eval_g_grad(nn, wo, wi, m, db, dr);
+        const float3 coef = v3(gv.x != 0.0f ? d.x * L_rem.x / gv.x : 0.0f, gv.y != 0.0f ? d.y * L_rem.y / gv.y : 0.0f,
+                               gv.z != 0.0f ? d.z * L_rem.z / gv.z : 0.0f);
+        add_bsdf(gm, coef, db, dr);
+      }
     }
-    if (flags & kCont) {
-      const float3 wi = xyz(r[4]);
-      float3 gv;
-      eval_lobe(nn, wo, wi, m, lobe, gv, pb);
-      float3 db, dr;
-      eval_g_grad(nn, wo, wi, m, db, dr);
-      const float3 coef = v3(gv.x != 0.0f ? d.x * L_rem.x / gv.x : 0.0f, gv.y != 0.0f ? d.y * L_rem.y / gv.y : 0.0f,
-                             gv.z != 0.0f ? d.z * L_rem.z / gv.z : 0.0f);
-      G.bsdf(mi, coef, db, dr);
-    }
+    G.add_warp(mi, 0, gm);
+    G.add_warp(ml, 3, ge);
   }
   grad_end(G);
 }

@@ -20,6 +20,7 @@ import pytest
 
 import oracle
 from pulse_b200 import _ffi, diff, scenes
+from pulse_b200.layout import Instance, Material
 from pulse_b200.tracer import PulseError, Scene, Target, make_view, render_backward, render_forward, render_params
 
 pytestmark = pytest.mark.gpu
@@ -243,3 +244,30 @@ def test_materials_set_relights_prepared_scene(ctx):
     assert e.value.code == _ffi.PULSE_ERR_NOT_READY
     tg.close()
     sc.close()
+
+
+@pytest.mark.parametrize("count", [1, 3, 40, 300])
+def test_backward_of_many_materials(ctx, count):
+    """Warps whose paths meet one material, a few and all different ones, up to more
+    materials than a block sums in shared memory (256)."""
+    W, H, n = 32, 24, 8
+    d = scenes.spheres_1080p(level=1, n_instances=320, width=W, height=H, box=6.0)
+    light = next(i for i, m in enumerate(d.materials) if max(m.emissive[:3]) > 0.0)
+    rng = np.random.default_rng(count)
+    mats = [Material((*rng.uniform(0.2, 0.9, 3), 1.0), (0, 0, 0, 1), rng.uniform(0.3, 0.9), 0.5, 0.0)
+            for _ in range(count)] + [d.materials[light]]
+    inst = [Instance(x.mesh, count if max(d.materials[x.material].emissive[:3]) > 0.0 else i % count, x.object_world)
+            for i, x in enumerate(d.instances)]
+    sb = oracle.assemble(d.meshes, mats, inst, 16, 4)
+    w = np.random.default_rng(8).normal(size=(H, W, 4)).astype(np.float32)
+    ref = oracle.backward(sb, d.view, W, H, n, w, **PARAMS)[:, :7]
+    sc = Scene(ctx)
+    ids = [sc.upload_mesh(m, 16, 4) for m in d.meshes]
+    sc.set_materials(mats)
+    sc.set_instances(inst, ids)
+    got = render_backward(sc, d.view, W, H, n, w, **PARAMS)
+    sc.close()
+    scale = np.abs(ref).max()
+    assert scale > 0
+    err = np.abs(got - ref).max() / scale
+    assert err < 2e-4, err
