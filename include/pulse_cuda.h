@@ -131,12 +131,16 @@ typedef struct {
                            register budget)                                       */
   uint32_t min_blocks;  /* register budget: 0 auto, else 4, 6 or 8 resident blocks per SM */
   uint32_t wf_segments; /* wavefront: segments traced as separate kernels before one
-                           persistent kernel finishes the remaining paths; 0 auto (3;
-                           2 for pulse_render_gi),
+                           persistent kernel finishes the remaining paths; 0 auto
+                           (prepared scenes: the logarithm of the path count less
+                           9, half that with nee_mode 0, at least 3; scenes set as
+                           buffers: 3, 2 for pulse_render_gi),
                            0xffffffff: no separate segments (the persistent kernel
                            runs every path from its primary ray)                      */
-  uint32_t trace_blocks; /* wavefront: resident traversal blocks per SM, 0 auto (8), <= 8 */
-  uint32_t step_policy;  /* wavefront traversal: which action a warp's step performs.
+  uint32_t trace_blocks; /* wavefront: resident traversal blocks per SM, 0 auto (4 with the
+                            eight-wide trees of prepared scenes, else 8), <= 8          */
+  uint32_t step_policy;  /* wavefront traversal over the binary trees (other values than 0
+                            select them): which action a warp's step performs.
                             0 auto; 1 every lane its own (divergent); else one weight
                             byte per action, node | tri << 8 | enter << 16 | leave << 24:
                             the action with the largest lane count x weight runs   */

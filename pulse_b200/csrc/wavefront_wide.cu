@@ -2,8 +2,12 @@
 // (pt_wide.cuh): every warp works on a pool of 64 rays in shared memory and performs, per
 // step, one action for up to 32 of them.
 //
-// What bounds the binary kernels (wavefront.cu) is issue with few lanes: one ray per
-// lane, 28 of 32 busy, of which 11 to 15 share an action; 66 node visits a ray.
+// What bounded the binary kernels (wavefront.cu) here is issue with few lanes: one ray per
+// lane, 28 of 32 busy, of which 11 to 15 share an action; 66 node visits a ray.  With the wide
+// trees a ray takes 33 steps, 21 lanes an action: the 1080p sphere frame 13.9 -> 9.3 ms,
+// the 4K terrain frame 39 -> 24 ms, a million query rays 3.9 -> 1.55 ms.  What bounds these
+// kernels is still issue (57% of the slots; 380 instructions a node step), then the drain of
+// each launch: the longest ray takes 466 steps.
 #include <atomic>
 
 #include "pt_wide.cuh"
@@ -16,8 +20,9 @@ namespace {
 
 using namespace wf;
 
-// Blocks of four warps resident per SM: three pools' shared memory (about 56 KB a block)
-// leave some 60 KB of L1.
+// Blocks of four warps resident per SM.  1080p sphere frame, at the time: three 13.0 ms,
+// four 11.9; later four 9.3, five and six 10.5 (their registers spill, and the pools'
+// shared memory, about 50 KB a block, leaves less L1).
 constexpr int kWideBlocks = 4;
 
 // The scenes of a launch: one, in the kernel's parameters (ONE: reading its pointers from
@@ -48,7 +53,7 @@ struct ExtendItem {
       const float4 a = e[0], b = e[1];
       const uint32_t sid = ONE ? 0u : __float_as_uint(e[2].w);
       R.set(kwId, (i - n) | 0x80000000u);
-        return wide_begin(R, sid, sc.at(sid).S, xyz(a), xyz(b), occ_limit(tc, a.w));
+      return wide_begin(R, sid, sc.at(sid).S, xyz(a), xyz(b), occ_limit(tc, a.w));
     }
     const uint32_t p = q[i], sid = sc.of_path(p);
     const float4 a = B.s[4 * (size_t)p], b = B.s[4 * (size_t)p + 1];

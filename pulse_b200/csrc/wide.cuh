@@ -12,7 +12,6 @@ enum Head : uint32_t {
   kBad,     // nonzero: no wide tree (a box not finite or above 1e9, a leaf out of the references' range)
   kLevels,  // levels of the wide tree
   kArea,    // largest |e1| |e2| of a triangle (float bits)
-  kEdge,    // longest edge of a triangle (float bits)
   kHeadWords = 8
 };
 
@@ -43,7 +42,7 @@ cudaError_t hull(const uint4* wide_nodes, uint32_t n_wide, const float4* nodes, 
 cudaError_t relocate(const uint32_t* nodes, uint32_t n, uint32_t node_add, uint32_t slot_add, uint32_t* out,
                      cudaStream_t st);
 
-// Raises head's kArea and kEdge (zero to begin with) to those of n std430 triangles.
+// Raises head's kArea (zero to begin with) to that of n std430 triangles.
 cudaError_t extents(const float4* prims, uint32_t n, uint32_t* head, cudaStream_t st);
 
 // Share of the distance by which the computed t of a hit may lie before its
