@@ -111,8 +111,8 @@ enum WideWord : uint32_t {
                                        // not to visit << 17) or instance
   kwSp,                                // stack entries | those of the TLAS level << 7 | instance << 14 | in a BLAS << 31
   kwLen, kwSlack,                      // object distance per world distance; slack of the mesh
-  kwExit,                              // an occlusion query is decided by a hit before it (world distance)
-  kwFar,                               // box entry bound of an occlusion query (world)
+  kwLimit,                             // of an occlusion query, else 3e38
+  kwFar,                               // box entry bound of an occlusion query (world), else infinity
   kwEps,                               // rounding of world distances
   kwRecT, kwRecSlot, kwRecInst,        // nearest candidate: world distance, triangle slot, instance | scene << 20
   kwId,                                // the kernel's
@@ -182,6 +182,13 @@ __device__ __forceinline__ float wide_gate(float t, float eps) { return t * 1.00
 // The bound of boxes whose hits may be found up to the slack before them.
 __device__ __forceinline__ float wide_bound(float t, float slack) { return t * (1.0f + slack) + slack; }
 
+// Whether a hit at world distance t decides an occlusion query, before its exact distance
+// is known: it lies before the limit by world_cull's margins.  Never for other queries (their
+// bound is infinite and the difference no number).
+__device__ __forceinline__ bool wide_decides(const WideRay& R, float t) {
+  return t < 2.0f * R.f(kwLimit) - R.f(kwFar);
+}
+
 // The level becomes the TLAS.
 __device__ __forceinline__ void wide_world(const WideRay& R, const DevScene& S, float3 wo, float3 wd, float rec_t,
                                            float far) {
@@ -194,7 +201,7 @@ __device__ __forceinline__ void wide_world(const WideRay& R, const DevScene& S, 
 // query.
 __device__ __forceinline__ uint32_t wide_begin(const WideRay& R, uint32_t scene, const DevScene& S, float3 wo,
                                                float3 wd, float limit) {
-  const float far = world_cull(limit, wo);
+  const float far = limit < 1e29f ? world_cull(limit, wo) : __int_as_float(0x7f800000);
   wide_world(R, S, wo, wd, 1e30f, far);
   R.set(kwSp, 0u);
   R.setf(kwRecT, 1e30f);
@@ -202,8 +209,7 @@ __device__ __forceinline__ uint32_t wide_begin(const WideRay& R, uint32_t scene,
   R.set(kwCur, 0u);  // the root node
   R.setf(kwFar, far);
   R.setf(kwEps, 1e-6f * max_abs3(wo));
-  const float x = limit * 0.9999f - 1e-3f * (1.0f + max_abs3(wo));
-  R.setf(kwExit, limit < 1e29f && x < 3.0e38f ? x : -1.0f);
+  R.setf(kwLimit, limit < 1e29f ? limit : 3.0e38f);
   if (!(limit > 0.0f)) return kwDone;
   return wide_ray_ok(wo, wd) ? kwNode : kwRedo;
 }
@@ -425,7 +431,10 @@ __device__ __forceinline__ uint32_t wide_tri(const WideRay& R, const DevScene& S
     }
   const float3 o = R.f3(kwOX), d = R.f3(kwDX);
   const float len = R.f(kwLen), best = R.f(kwRecT), eps = R.f(kwEps);
-  const float gate = best < 1e30f ? wide_gate(best, eps) * len : 1e30f;
+  // (a hit beyond an occlusion query's limit and the rounding of distances hides nothing, and a
+  // hit before it has its boxes verified: most shadow rays end without a candidate to
+  // verify or to trace again.  512^2 x 16 spp Cornell frame 5.72 -> 5.46 ms)
+  const float gate = fminf(best < 1e30f ? wide_gate(best, eps) * len : 1e30f, wide_gate(R.f(kwLimit), eps) * len);
   float ta = 1e30f, tb = 1e30f;  // the nearest candidate and the second
   uint32_t ka = 0;
 #pragma unroll
@@ -441,7 +450,7 @@ __device__ __forceinline__ uint32_t wide_tri(const WideRay& R, const DevScene& S
     const float scale = __fdividef(1.0f, len);
     const float w = ta * scale;
     const uint32_t spx = R.u(kwSp), slot = first + ka;
-    const bool decided = w < R.f(kwExit);  // an occlusion query's light is hidden, if this hit is verified
+    const bool decided = wide_decides(R, w);  // an occlusion query's light is hidden, if this hit is verified
     // the nearest of all and the second: ambiguous within the nearest's gate
     const float second = fminf(fmaxf(w, best), tb < 1e30f ? tb * scale : 1e30f), M = wide_gate(fminf(w, best), eps);
     if (!decided && second <= M) return kwRedo;
@@ -533,7 +542,7 @@ __device__ __forceinline__ void wide_store(const WideRay& R, const Hit& h) {
 __device__ __forceinline__ uint32_t wide_verify(const WideRay& R, const DevScene& S, const TraceCfg& cfg, float3 wo,
                                                 float3 wd) {
   const float rec_t = R.f(kwRecT);
-  const bool decided = rec_t < R.f(kwExit);
+  const bool decided = wide_decides(R, rec_t);
   Hit h;
   h.inst = R.u(kwRecInst) & kInstMask;
   const uint32_t slot = R.u(kwRecSlot);

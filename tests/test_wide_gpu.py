@@ -191,3 +191,29 @@ def test_frames_equal_the_oracle(ctx, mode, segments):
     tg.close()
     sc.close()
     assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
+
+
+@pytest.mark.parametrize("mode", [1, 2])
+@pytest.mark.parametrize("gap", [0.0, 1e-6, 1e-4, 1e-3, 2e-3, 0.1])
+def test_occluder_before_the_light_equals_the_oracle(ctx, mode, gap):
+    """A second surface in the light's plane, and within, at and past the slack of a shadow
+    ray's limit before it: what hides the light and what does not."""
+    d = scenes.cornell(48, 36)
+    light = next(x for x in d.instances if max(d.materials[x.material].emissive[:3]) > 0.0)
+    dark = next(k for k, m in enumerate(d.materials) if max(m.emissive[:3]) == 0.0)
+    half = scenes.trs((0.25, -gap, 0.0))  # over a part of the light, towards the floor
+    inst = [*d.instances, Instance(light.mesh, dark, half @ np.asarray(light.object_world))]
+    params = dict(max_depth=4, nee_mode=mode, light_pick=0, quirks=0, spp=4)
+    sb = oracle.assemble(d.meshes, d.materials, inst, 20, 4)
+    sc = Scene(ctx)
+    ids = [sc.upload_mesh(m, 20, 4) for m in d.meshes]
+    sc.set_materials(d.materials)
+    sc.set_instances(inst, ids)
+    tg = Target(ctx, d.width, d.height)
+    ref = np.zeros((d.height, d.width, 4), np.float32)
+    render_forward(sc, d.view, tg, 0, **params)
+    oracle.render(sb, d.view, d.width, d.height, 0, image=ref, **params)
+    got = tg.download()
+    tg.close()
+    sc.close()
+    assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
