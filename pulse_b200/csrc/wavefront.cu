@@ -827,6 +827,17 @@ cudaError_t wf_reset_step(const WfBuffers& B, int next, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+// Whether camera rays alone (a frame of one segment, the G-buffer) keep the binary trees
+// although the wide ones are there: these rays are coherent, so a ray per lane wastes little,
+// and through trees of a handful of levels the pools' steps cost more than they save.
+// Wide / binary in us, Cornell box (5 + 3 levels): one-segment frames of mode 2, 256^2 110 / 108,
+// 384 x 256 122 / 113, 540p 268 / 228, 1080p 770 / 713; of mode 0, 74 / 77, 85 / 81, 163 / 154,
+// 460 / 473; G-buffer 58 / 60, 66 / 60, 122 / 102, 342 / 286.  A sphere of 320 triangles (5 + 8
+// levels), 540p: 151 / 216, 110 / 126 and 90 / 99.
+static bool camera_rays_binary(uint32_t tlas_levels, uint32_t blas_levels, uint32_t paths) {
+  return tlas_levels + blas_levels <= 8u && paths >= 96u * 1024u;
+}
+
 cudaError_t wf_gbuffer_primary(const TraceCfg& tc, const WfScene& scene, float4* gbuf, uint32_t trace_blocks,
                                const WfBuffers& B, Counters* ctr, uint32_t* launches, cudaStream_t st) {
   if (cudaError_t e = wf_prepare(1)) return e;
@@ -844,7 +855,7 @@ cudaError_t wf_gbuffer_primary(const TraceCfg& tc, const WfScene& scene, float4*
   cudaError_t e = wf_upload_table(&one, 1, B, st);
   if (e != cudaSuccess) return e;
   k_gbuf_generate<<<sms * 16, kWfBlock, tab, st>>>(B);
-  if (wide_allowed(tcs, one.S)) {
+  if (wide_allowed(tcs, one.S) && !camera_rays_binary(one.S.tlas_levels, one.S.blas_levels, one.paths)) {
     WfLaunch L{};
     L.n_scenes = 1;
     L.one = &one;
@@ -922,6 +933,7 @@ cudaError_t wf_render(int mode, const TraceCfg& tc, const WfScene* scenes, uint3
   if (n == 1) L.one = tab;
   L.wide = true;  // one scene that cannot keeps the batch on the binary traversal
   for (uint32_t i = 0; i < n; ++i) L.wide = L.wide && wide_allowed(tcs, tab[i].S);
+  if (L.segments == 1 && camera_rays_binary(tl, bl, L.total_paths)) L.wide = false;
   if (L.wide && !wf_segments) L.wf_segments = wide_segments(mode, L.total_paths);
   cudaError_t e = wf_upload_table(tab, n, B, st);
   if (e != cudaSuccess) return e;

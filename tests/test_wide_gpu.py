@@ -12,7 +12,7 @@ import pytest
 import oracle
 from pulse_b200 import scenes
 from pulse_b200.layout import Instance, Material, Mesh
-from pulse_b200.tracer import Scene, Target, render_forward
+from pulse_b200.tracer import Scene, Target, gbuffer_primary, render_forward
 
 pytestmark = pytest.mark.gpu
 
@@ -217,3 +217,28 @@ def test_occluder_before_the_light_equals_the_oracle(ctx, mode, gap):
     tg.close()
     sc.close()
     assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
+
+
+@pytest.mark.parametrize("width", [383, 384])  # of 256 rows: below the line of the dispatch, and on it
+@pytest.mark.parametrize("mode", [0, 2])
+def test_camera_rays_alone_equal_the_oracle(ctx, mode, width):
+    """A frame of one segment over trees of few levels: the wide or the binary trees by its paths."""
+    d = scenes.cornell(width, 256)
+    params = dict(max_depth=1, nee_mode=mode, light_pick=1 if mode == 2 else 0, quirks=1)
+    sb = oracle.assemble(d.meshes, d.materials, d.instances, 20, 4)
+    sc = Scene(ctx)
+    ids = [sc.upload_mesh(m, 20, 4) for m in d.meshes]
+    sc.set_materials(d.materials)
+    sc.set_instances(d.instances, ids)
+    tg = Target(ctx, width, 256)
+    ref = np.zeros((256, width, 4), np.float32)
+    render_forward(sc, d.view, tg, 0, **params)
+    oracle.render(sb, d.view, width, 256, 0, image=ref, **params)
+    got = tg.download()
+    # the G-buffer: the same rule
+    g = np.asarray(gbuffer_primary(sc, d.view, width, 256))
+    want = oracle.gbuffer_primary(sb, d.view, width, 256)
+    tg.close()
+    sc.close()
+    assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
+    assert np.array_equal(g.reshape(-1).view(np.uint32), np.asarray(want).reshape(-1).view(np.uint32))
