@@ -162,12 +162,27 @@ __device__ __forceinline__ bool wide_ray_ok(float3 o, float3 d) {
   return fabsf(dd - 1.0f) < 1e-4f && max_abs3(o) <= 1e9f && o.x == o.x && o.y == o.y && o.z == o.z;
 }
 
-// The reference's slab test of a box without its record comparison
-// (src/utilities.wgsl:405-426): true with t_min when the box is entered.
-__device__ __forceinline__ bool hit_leaf_box(float3 o, float3 d, const float4* node, float& t_min) {
+// Whether the reference's slab test without its record comparison (src/utilities.wgsl:405-426)
+// passes a box and its t_min is at most bound.  Answered from planes by reciprocals, within
+// 4e-7 of the reference's quotients, where every comparison holds by 2e-6 (the planes of one
+// axis need none: their quotients are ordered like them, so boxes without thickness are
+// answered too); rays that pass an edge closer, or fail, take the exact test.
+__device__ __forceinline__ bool enters_box(float3 o, float3 d, const float4* node, float bound) {
   const float4 lo = __ldg(node), hi = __ldg(node + 1);
-  t_min = ray_aabb(o, d, 1e30f, lo, hi);
-  return t_min < 1e30f;
+  const float3 r = v3(__fdividef(1.0f, d.x), __fdividef(1.0f, d.y), __fdividef(1.0f, d.z));
+  const float ax = (lo.x - o.x) * r.x, bx = (hi.x - o.x) * r.x;
+  const float ay = (lo.y - o.y) * r.y, by = (hi.y - o.y) * r.y;
+  const float az = (lo.z - o.z) * r.z, bz = (hi.z - o.z) * r.z;
+  const float nx = fminf(ax, bx), ny = fminf(ay, by), nz = fminf(az, bz);
+  const float fx = fmaxf(ax, bx), fy = fmaxf(ay, by), fz = fmaxf(az, bz);
+  const float tn = fmaxf(fmaxf(nx, ny), nz), tf = fminf(fminf(fx, fy), fz);
+  const float most = fmaxf(fmaxf(fabsf(ax), fabsf(bx)),
+                           fmaxf(fmaxf(fabsf(ay), fabsf(by)), fmaxf(fabsf(az), fabsf(bz))));
+  const float gap = fminf(fminf(fx - fmaxf(ny, nz), fy - fmaxf(nx, nz)), fz - fmaxf(nx, ny));
+  const float least = fminf(fminf(fabsf(d.x), fabsf(d.y)), fabsf(d.z));
+  if (gap > 2e-6f * most && tf > 1e-30f && tn + 2e-6f * fabsf(tn) <= bound && most < 1e28f && least > 1e-18f) return true;
+  const float t = ray_aabb(o, d, 1e30f, lo, hi);
+  return t < 1e30f && t <= bound;
 }
 
 constexpr uint32_t kInBlas = 1u << 31;
@@ -538,7 +553,12 @@ __device__ __forceinline__ void wide_store(const WideRay& R, const Hit& h) {
   R.setf(kwV, h.v);
 }
 
-// Verify a finished ray's candidate: kwDone, or kwRedo when it fails.
+// Verify a finished ray's candidate: kwDone, or kwRedo when it fails.  The candidate of an
+// occlusion query ended early needs no exact distance; its boxes of both levels are tested
+// like any other's, and are entered before the limit too, so that a hit which kept the
+// reference out of them hides the light as well.  (Without the instance's box, 5 of 2.7e9
+// rays of Cornell frames, past the edge of a mesh of one leaf, were answered wrongly.  Testing
+// it: the 512^2 x 16 spp frame 4.96 ms before and after, 5.07 with the exact test alone.)
 __device__ __forceinline__ uint32_t wide_verify(const WideRay& R, const DevScene& S, const TraceCfg& cfg, float3 wo,
                                                 float3 wd) {
   const float rec_t = R.f(kwRecT);
@@ -553,20 +573,19 @@ __device__ __forceinline__ uint32_t wide_verify(const WideRay& R, const DevScene
   float3 o, d;
   const float len = wide_object_ray(load_m4(ip), wo, wd, o, d);
   const float gate = wide_gate(rec_t, R.f(kwEps)) * 0.999999f;
-  float t = 0.0f, m;
+  const float by = decided ? (2.0f * R.f(kwLimit) - R.f(kwFar)) * 0.999999f : gate;
+  float t = 0.0f;
   h.u = h.v = 0.0f;
   bool ok = ray_triangle_v(o, d, 1e30f, xyz(t0), xyz(t1), xyz(t2), cfg, t, h.u, h.v);
   const uint32_t leaf = __float_as_uint(t1.w), tleaf = __float_as_uint(wy.z);
   if (leaf != kWideRootLeaf)
-    ok = ok && hit_leaf_box(o, d, S.blas_nodes + 2 * (size_t)(__float_as_uint(wy.y) + leaf), m) &&
-         (decided || m <= gate * len);
+    ok = ok && enters_box(o, d, S.blas_nodes + 2 * (size_t)(__float_as_uint(wy.y) + leaf), by * len);
+  if (tleaf != kWideRootLeaf) ok = ok && enters_box(wo, wd, S.tlas_nodes + 2 * (size_t)tleaf, by);
   h.t = -3.0e38f;
   if (!decided) {
     const M4 o2w = load_m4(S.instances + (size_t)h.inst * 10);
     h.t = length(sub(transform_position(o2w, add(o, muls(d, t))), wo));
     ok = ok && h.t < 1e30f && h.t <= gate;
-    if (tleaf != kWideRootLeaf)
-      ok = ok && hit_leaf_box(wo, wd, S.tlas_nodes + 2 * (size_t)tleaf, m) && m <= gate;
   }
   h.slot = slot - __float_as_uint(wy.x);  // within the mesh
   wide_store(R, h);

@@ -242,3 +242,68 @@ def test_camera_rays_alone_equal_the_oracle(ctx, mode, width):
     sc.close()
     assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
     assert np.array_equal(g.reshape(-1).view(np.uint32), np.asarray(want).reshape(-1).view(np.uint32))
+
+
+def _prepare(ctx, meshes, materials, instances, leaf=4):
+    sc = Scene(ctx)
+    ids = [sc.upload_mesh(m, 20, leaf) for m in meshes]
+    sc.set_materials(materials)
+    sc.set_instances(instances, ids)
+    return sc
+
+
+@pytest.mark.parametrize("mode", [1, 2])
+def test_occluders_whose_boxes_are_rounded_equal_the_oracle(ctx, mode):
+    """Small quads between a floor and its light, 40,000 units from the origin: an instance's
+    bounds are rounded to 1/256 there, its triangles in object space are not.  A shadow ray that
+    passes a quad's edge outside the bounds misses the quad, however far before the light it lies."""
+    centre = np.array([2e4, -1e4, 3e4])
+    rng = np.random.default_rng(21)
+
+    def at(*p):
+        return scenes.trs(centre + p)
+
+    def quad(h, ny):
+        return scenes.quad_mesh([(-h, 0, ny * h), (h, 0, ny * h), (h, 0, -ny * h), (-h, 0, -ny * h)], (0, ny, 0))
+
+    meshes = [quad(40.0, 1), quad(8.0, -1), quad(0.77, 1)]
+    mats = [Material((0.7, 0.7, 0.7, 1), (0, 0, 0, 1), 0.8, 0.5, 0.0), Material((0.7, 0.7, 0.7, 1), (9, 9, 9, 1), 0.8, 0.5, 0.0)]
+    inst = [Instance(0, 0, at(0, 0, 0)), Instance(1, 1, at(0, 70, 0))]
+    for x in range(-10, 11):
+        for z in range(-10, 11):
+            inst.append(Instance(2, 0, at(2.1 * x + rng.uniform(), rng.uniform(2, 20), 2.1 * z + rng.uniform())))
+    view = scenes.bevy_view(centre + (3.0, 45.0, 60.0), centre, aspect=96 / 64)
+    params = dict(max_depth=3, nee_mode=mode, light_pick=0, quirks=0, spp=4)
+    sb = oracle.assemble(meshes, mats, inst, 20, 4)
+    sc = _prepare(ctx, meshes, mats, inst)
+    tg = Target(ctx, 96, 64)
+    ref = np.zeros((64, 96, 4), np.float32)
+    render_forward(sc, view, tg, 0, **params)
+    oracle.render(sb, view, 96, 64, 0, image=ref, **params)
+    got = tg.download()
+    tg.close()
+    sc.close()
+    assert ref[..., :3].max() > 0
+    assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
+
+
+def test_shadow_ray_past_the_edge_of_the_light_equals_the_oracle(ctx):
+    """A texel of the Cornell box with a shadow ray that grazes the light's edge outside its
+    bounds: the reference misses the light, and the texel is lit."""
+    rng = np.random.default_rng(12)
+    d = scenes.cornell()
+    mats = [Material((*rng.uniform(0.1, 0.9, 3), 1), m.emissive, rng.uniform(0.2, 1.0), 0.5, 0.0) for m in d.materials]
+    view = scenes.bevy_view((rng.uniform(-0.2, 0.2), rng.uniform(-0.2, 0.2), 3.0), (0.0, 0.0, 0.0), aspect=1.0)
+    params = dict(max_depth=6, nee_mode=2, light_pick=1, quirks=0, spp=16, seed=12)
+    sb = oracle.assemble(d.meshes, mats, d.instances, 20, 8)
+    sc = _prepare(ctx, d.meshes, mats, d.instances, 8)
+    tg = Target(ctx, 512, 512)
+    texels = [106 * 512 + x for x in range(250, 265)]
+    ref = np.zeros((512, 512, 4), np.float32)
+    render_forward(sc, view, tg, 0, **params)
+    oracle.render(sb, view, 512, 512, 0, image=ref, pixels=texels, **params)
+    got = tg.download()
+    tg.close()
+    sc.close()
+    a, b = (x.reshape(-1, 4)[texels].view(np.uint32) for x in (got, ref))
+    assert np.array_equal(a, b)
