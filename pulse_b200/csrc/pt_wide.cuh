@@ -616,9 +616,10 @@ __device__ __forceinline__ Hit wide_hit(const WideRay& R) {
 // Each step performs the class most slots wait for (at most 32 count); rays to be traced
 // again wait for kRedoAt of them, as they run alone in the warp (lane by lane they took
 // 1.5 of the 7.2 ms of the 512^2 x 16 spp Cornell frame, whose boxes stand on the floor).  New items
-// are fetched once kFetchAt slots are empty; the warp's first kPool items are those of
-// its number, later ones come from the cursor kFetchChunk at a time (an atomic takes
-// about 2 us when every warp asks).
+// are fetched once kFetchAt slots are empty, or once one is and no other class has a slot.  (A
+// pool full of rays to be traced again has none empty: those are traced then, so that every step
+// takes a slot on.)  The warp's first kPool items are those of its number, later ones come from
+// the cursor kFetchChunk at a time (an atomic takes about 2 us when every warp asks).
 constexpr uint32_t kFetchAt = 16, kFetchChunk = 64, kRedoAt = 16;
 
 template <class Item>
@@ -653,7 +654,8 @@ __device__ __forceinline__ void wide_run(Item& it, const TraceCfg& tc, uint32_t*
         ns = __popc(__ballot_sync(0xffffffffu, c0 == kwShade)) + __popc(__ballot_sync(0xffffffffu, c1 == kwShade));
         key = max(key, (ns << 3) | kwShade);
       }
-      if (!drained && (rest - nr - ns >= kFetchAt || key < 8u)) key = kwEmpty;
+      const uint32_t free = rest - nr - ns;
+      if (!drained && (free >= kFetchAt || (key < 8u && free))) key = kwEmpty;
       else if (nr >= kRedoAt || (key < 8u && nr)) key = kwRedo;
       else if (key < 8u) break;
     }

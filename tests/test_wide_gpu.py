@@ -307,3 +307,65 @@ def test_shadow_ray_past_the_edge_of_the_light_equals_the_oracle(ctx):
     sc.close()
     a, b = (x.reshape(-1, 4)[texels].view(np.uint32) for x in (got, ref))
     assert np.array_equal(a, b)
+
+
+def _many_rays(n, half, refused):
+    """n rays, of which every second run of `refused` is not for the wide trees."""
+    rays = np.resize(_rays(half, np.zeros(3), 13)[:2000], (n, 6))
+    rng = np.random.default_rng(14)
+    rays[:, :3] += rng.uniform(-0.1, 0.1, (n, 3)) * half
+    if refused:
+        run = np.arange(n) // refused
+        rays[run % 8 == 1, 3:] = 0.0
+        rays[run % 8 == 3, 3:] *= 2.5
+        rays[run % 8 == 5, 3:] = np.nan
+        rays[run % 8 == 7, :3] += 3e9
+    return rays.astype(np.float32)
+
+
+# Warps of a B200's launch: 148 SMs x 4 blocks x 4.  With more than 64 rays for each, pools are
+# refilled from the shared cursor.
+POOLED = 148 * 16 * 64
+
+
+@pytest.mark.parametrize("count", [POOLED - 1, POOLED, POOLED + 1, 200003])
+@pytest.mark.parametrize("kind,refused", [("cornell", 0), ("cornell", 7), ("cornell", 64), ("cornell", 4096),
+                                          ("overlapping", 200), ("duplicates", 0), ("duplicates", 64)])
+def test_queries_larger_than_the_pools(ctx, kind, refused, count):
+    """Every pool refilled, whole pools of rays to be traced again (refused ones, or hits at
+    the same distance), against the binary trees, and some against the oracle."""
+    meshes, instances, leaf, tlas_leaf, half = _scene(kind)
+    rays = _many_rays(count, half, refused)
+    sc = Scene(ctx)
+    ids = [sc.upload_mesh(m, 20, leaf) for m in meshes]
+    sc.set_materials(MAT * 8)
+    sc.set_instances(instances, ids, 2, tlas_leaf)
+    want = sc.trace(rays, step_policy=1)
+    got = sc.trace(rays)
+    sc.close()
+    for k in ("instance_index", "triangle_index"):
+        assert np.array_equal(got[k], want[k])
+    for k in "tuv":
+        assert np.array_equal(got[k].view(np.uint32), want[k].view(np.uint32))
+    some = np.arange(0, count, 97)
+    ref = oracle.trace(oracle.assemble(meshes, MAT * 8, instances, 20, leaf, 2, tlas_leaf), rays[some])
+    assert np.array_equal(got["t"][some].view(np.uint32), ref["t"].view(np.uint32))
+    assert np.array_equal(got["triangle_index"][some], ref["triangle"])
+
+
+@pytest.mark.parametrize("mode", [0, 2])
+@pytest.mark.parametrize("segments", [0, 0xFFFFFFFF])
+def test_frames_of_refused_camera_rays(ctx, mode, segments):
+    """A camera beyond the wide trees' range, over more paths than the pools hold."""
+    d = scenes.cornell(640, 400)
+    view = scenes.bevy_view((0.0, 0.0, 3e9), (0.0, 0.0, 0.0), aspect=1.6)
+    params = dict(max_depth=3, nee_mode=mode, light_pick=1 if mode == 2 else 0, wf_segments=segments)
+    sc = _prepare(ctx, d.meshes, d.materials, d.instances)
+    tg = Target(ctx, 640, 400)
+    images = []
+    for policy in (1, 0):
+        render_forward(sc, view, tg, 0, step_policy=policy, **params)
+        images.append(tg.download().copy())
+    tg.close()
+    sc.close()
+    assert np.array_equal(images[0].view(np.uint32), images[1].view(np.uint32))
