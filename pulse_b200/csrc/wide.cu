@@ -279,8 +279,12 @@ __global__ void __launch_bounds__(kBlock) k_collapse(const float4* __restrict__ 
   }
   if (tid == 0) head[kLevels] = levels;
   if (!leaf_of.instance_of) return;
-  // TLAS: bottom-up, the deepest level first
-  if (levels >= kMaxLevels || *(volatile uint32_t*)(head + kBad)) {
+  // TLAS: bottom-up, the deepest level first.  Fitting a box that is out of range sets kBad too,
+  // so every thread has read it before the first one fits: all leave here, or all meet at every
+  // barrier below.
+  const bool bad = levels >= kMaxLevels || *(volatile uint32_t*)(head + kBad);
+  sync();
+  if (bad) {
     if (tid == 0) head[kBad] = 1u;
     return;
   }

@@ -369,3 +369,26 @@ def test_frames_of_refused_camera_rays(ctx, mode, segments):
     tg.close()
     sc.close()
     assert np.array_equal(images[0].view(np.uint32), images[1].view(np.uint32))
+
+
+@pytest.mark.parametrize("count", [1, 6, 40, 8300])  # a root leaf, one block, and the grid's barriers from 8,193 on
+@pytest.mark.parametrize("far", ["translation", "extent"])
+def test_instance_out_of_range_keeps_the_binary_trees(ctx, count, far):
+    """One instance whose bounds pass 1e9 leaves the whole scene to the binary trees; moved
+    back, the scene takes the wide ones again."""
+    meshes, instances = _spheres(count, 1, 8.0, 15, lambda rng: rng.uniform(0.05, 0.2))
+    home = instances[count // 2].object_world
+    away = scenes.trs((0, 2e9, 0)) if far == "translation" else scenes.trs((0, 9e8, 0), scale=(2e8, 2e8, 2e8))
+    rays = _rays(8.0, np.zeros(3), 16)
+    sc = Scene(ctx)
+    ids = [sc.upload_mesh(m, 20, 4) for m in meshes]
+    sc.set_materials(MAT * 8)
+    for world in (away, home):
+        instances[count // 2].object_world = world
+        sc.set_instances(instances, ids, 2, 1)
+        got = sc.trace(rays)
+        ref = oracle.trace(oracle.assemble(meshes, MAT * 8, instances, 20, 4, 2, 1), rays)
+        assert np.array_equal(got["t"].view(np.uint32), ref["t"].view(np.uint32))
+        for a, b in (("instance_index", "instance"), ("triangle_index", "triangle")):
+            assert np.array_equal(got[a], ref[b])
+    sc.close()
