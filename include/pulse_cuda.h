@@ -230,6 +230,8 @@ PULSE_API int32_t pulse_ctx_set_pipeline(PulseCtx* ctx, uint32_t depth);
  * PULSE_ERR_OOM after releasing what they hold, and every context stays
  * usable.  n = 0 disarms.  Nothing is allocated or faulted on the device. */
 PULSE_API int32_t pulse_debug_fail_allocations(uint32_t n);
+/* The same after the next skip allocations, which succeed. */
+PULSE_API int32_t pulse_debug_fail_allocations_after(PulseCtx* ctx, uint32_t skip, uint32_t n);
 
 /* ------------------------------------------------------------------ scene */
 PULSE_API int32_t pulse_scene_create(PulseCtx* ctx, PulseScene** out);

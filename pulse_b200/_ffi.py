@@ -103,6 +103,7 @@ SIGNATURES = {
     "pulse_ctx_get_stream": (C.c_int32, [P, C.POINTER(C.c_void_p)]),
     "pulse_ctx_set_pipeline": (C.c_int32, [P, C.c_uint32]),
     "pulse_debug_fail_allocations": (C.c_int32, [C.c_uint32]),
+    "pulse_debug_fail_allocations_after": (C.c_int32, [C.c_void_p, C.c_uint32, C.c_uint32]),
     "pulse_scene_create": (C.c_int32, [P, C.POINTER(C.c_void_p)]),
     "pulse_scene_destroy": (C.c_int32, [P]),
     "pulse_scene_set_buffers": (C.c_int32, [P, C.POINTER(SceneBuffersC)]),

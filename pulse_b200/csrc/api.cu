@@ -26,13 +26,16 @@
 
 namespace pt {
 namespace {
-std::atomic<uint32_t> g_fail_allocs{0};  // armed by pulse_debug_fail_allocations
+// Armed by pulse_debug_fail_allocations and _after: allocations that succeed before (upper
+// half) and that fail then.
+std::atomic<uint64_t> g_fail_allocs{0};
 }
 cudaError_t dev_alloc(void** p, size_t bytes) {
-  uint32_t n = g_fail_allocs.load();
-  while (n > 0 && !g_fail_allocs.compare_exchange_weak(n, n - 1)) {
+  constexpr uint64_t kSkip = (uint64_t)1 << 32;
+  uint64_t n = g_fail_allocs.load();
+  while (n > 0 && !g_fail_allocs.compare_exchange_weak(n, n >= kSkip ? n - kSkip : n - 1)) {
   }
-  if (n > 0) {
+  if (n > 0 && n < kSkip) {
     *p = nullptr;
     return cudaErrorMemoryAllocation;
   }
@@ -129,6 +132,8 @@ struct PulseScene {
   DevBuf wide_blas, leaf_of, hulls;               // of every mesh, concatenated
   DevBuf wide_tlas, wide_thead, inst_wide;  // of the instances (pt_wide.cuh)
   DevBuf wide_queue, wide_box, wide_bounds;       // scratch of the instance tree's collapse
+  bool wide_meshes = false;                       // wide_blas, leaf_of and hulls hold every live mesh's
+  bool wide_records = false;                      // inst_wide holds every instance's record
   std::vector<uint32_t> mesh_wide;                // per mesh id: first wide node in wide_blas
   uint64_t wide_nodes = 0;                        // rows of wide_blas
   bool tri_bvh_current = false;  // tri_bvh gathered from the current primitives and triangle_indices
@@ -227,6 +232,7 @@ struct PulseScene {
     for (DevBuf* b : {&inst_light, &tri_bvh, &wide_blas, &leaf_of, &hulls, &wide_tlas, &wide_thead, &inst_wide})
       free_buf(*b);
     dev.wide = 0u;
+    wide_meshes = wide_records = false;
     tri_bvh_current = false;
     free_buf(inst_bounds);
     free_back();
@@ -600,6 +606,14 @@ int32_t pulse_debug_fail_allocations(uint32_t n) {
   return PULSE_OK;
 }
 
+int32_t pulse_debug_fail_allocations_after(PulseCtx* ctx, uint32_t skip, uint32_t n) {
+  if (!ctx) return PULSE_ERR_INVALID_ARG;
+  cudaSetDevice(ctx->device);
+  quiesce(ctx);
+  pt::g_fail_allocs.store(n ? (uint64_t)skip << 32 | n : 0);
+  return PULSE_OK;
+}
+
 int32_t pulse_ctx_get_stream(const PulseCtx* ctx, void** out) {
   if (!ctx || !out) return PULSE_ERR_INVALID_ARG;
   // ordered after the pipelined frames in flight, so that work the caller
@@ -883,7 +897,17 @@ int32_t pulse_build_tlas(PulseCtx* ctx, const float* bounds9, uint32_t n, const 
 }
 
 // ------------------------------------------------- scene-preparation path
-// The eight-wide tree of a mesh whose nodes and triangles are on the device.
+// Whether an error in making the eight-wide trees leaves the scene to the binary ones: no
+// memory for them, or no room for the launch that collapses a large tree.  They are an option
+// of the traversal, so the call that makes them goes on without.
+static bool without_wide(cudaError_t e) {
+  if (e != cudaErrorMemoryAllocation && e != cudaErrorCooperativeLaunchTooLarge) return false;
+  cudaGetLastError();
+  return true;
+}
+
+// The eight-wide tree of a mesh whose nodes and triangles are on the device; wide_ok tells
+// whether it has one.
 static cudaError_t collapse_mesh(PulseCtx* ctx, MeshRec& m, cudaStream_t st) {
   const size_t cap = wide::capacity(m.node_count), out_bytes = cap * pt::kWideNodeWords * 4;
   uint32_t h[wide::kHeadWords] = {};
@@ -916,7 +940,11 @@ static cudaError_t collapse_mesh(PulseCtx* ctx, MeshRec& m, cudaStream_t st) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     m.wide_ok = e == cudaSuccess;
   }
-  return e;
+  if (!m.wide_ok) {
+    for (DevBuf* x : {&m.wide, &m.leaf_of, &m.hull}) PulseScene::free_buf(*x);
+    m.wide_count = m.wide_root = m.wide_levels = 0u;
+  }
+  return without_wide(e) ? cudaSuccess : e;
 }
 
 // Whether an instance's transform is affine and far enough from singular for the
@@ -937,10 +965,11 @@ static bool wide_transform(const float* m) {
 
 // What the collapse of the instance tree reported.
 struct WideTree {
+  bool made = false;  // a collapse was queued
   bool ok = false;
   uint32_t levels = 0, count = 0;
   void read(const uint32_t* head) {
-    ok = !head[wide::kBad];
+    ok = made && !head[wide::kBad];
     levels = head[wide::kLevels];
     count = head[wide::kCount];
   }
@@ -1089,6 +1118,31 @@ int32_t pulse_materials_set(PulseScene* s, const PulseMaterial* mats, uint32_t n
   return PULSE_OK;
 }
 
+// The meshes' eight-wide trees, if all of them have one and there is memory for their copy.
+static cudaError_t concat_wide(PulseScene* s, uint64_t nt, uint64_t nw, cudaStream_t st) {
+  const size_t node_bytes = pt::kWideNodeWords * 4, hull_bytes = wide::kHullBoxes * 32;
+  bool all = true;
+  for (const MeshRec& m : s->meshes) all = all && (!m.alive || m.wide_ok);
+  cudaError_t e = all ? cudaSuccess : cudaErrorMemoryAllocation;
+  if (e == cudaSuccess) e = ensure(s->wide_blas, nw * node_bytes);
+  if (e == cudaSuccess) e = ensure(s->leaf_of, nt * 4);
+  if (e == cudaSuccess) e = ensure(s->hulls, s->meshes.size() * hull_bytes);  // by mesh id
+  for (const MeshRec& m : s->meshes) {
+    if (!m.alive || e != cudaSuccess) continue;
+    const auto& t = s->mesh_table[m.id];
+    e = cudaMemcpyAsync((char*)s->leaf_of.p + (size_t)t[2] * 4, m.leaf_of.p, (size_t)m.ntris * 4, cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync((char*)s->hulls.p + m.id * hull_bytes, m.hull.p, hull_bytes, cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess && m.wide_count)
+      e = wide::relocate((const uint32_t*)m.wide.p, m.wide_count, s->mesh_wide[m.id], t[2],
+                         (uint32_t*)s->wide_blas.p + (size_t)s->mesh_wide[m.id] * pt::kWideNodeWords, st);
+  }
+  s->wide_meshes = e == cudaSuccess;
+  if (!s->wide_meshes)
+    for (DevBuf* x : {&s->wide_blas, &s->leaf_of, &s->hulls}) PulseScene::free_buf(*x);
+  return without_wide(e) ? cudaSuccess : e;
+}
+
 // prepare_mesh_data (src/scene/mod.rs:471-510): concatenation of every live
 // mesh in id order with its offsets.
 static cudaError_t concat_meshes(PulseScene* s) {
@@ -1106,15 +1160,10 @@ static cudaError_t concat_meshes(PulseScene* s) {
     nn += m.node_count;
     nw += m.wide_count;
   }
-  const size_t wide_bytes = pt::kWideNodeWords * 4;
   cudaError_t e = ensure(s->primitives, nt * 48);
   if (e == cudaSuccess) e = ensure(s->triangle_data, nt * 80);
   if (e == cudaSuccess) e = ensure(s->triangle_indices, nt * 4);
   if (e == cudaSuccess) e = ensure(s->blas_nodes, nn * 32);
-  if (e == cudaSuccess) e = ensure(s->wide_blas, nw * wide_bytes);
-  if (e == cudaSuccess) e = ensure(s->leaf_of, nt * 4);
-  const size_t hull_bytes = wide::kHullBoxes * 32;
-  if (e == cudaSuccess) e = ensure(s->hulls, s->meshes.size() * hull_bytes);  // by mesh id
   for (const MeshRec& m : s->meshes) {
     if (!m.alive || e != cudaSuccess) continue;
     const auto& t = s->mesh_table[m.id];
@@ -1122,13 +1171,8 @@ static cudaError_t concat_meshes(PulseScene* s) {
     if (e == cudaSuccess) e = cudaMemcpyAsync((char*)s->triangle_data.p + (size_t)t[0] * 80, m.tdata.p, (size_t)m.ntris * 80, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync((char*)s->triangle_indices.p + (size_t)t[2] * 4, m.idx.p, (size_t)m.ntris * 4, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync((char*)s->blas_nodes.p + (size_t)t[3] * 32, m.nodes.p, (size_t)m.node_count * 32, cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync((char*)s->leaf_of.p + (size_t)t[2] * 4, m.leaf_of.p, (size_t)m.ntris * 4, cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess && m.wide_ok)
-      e = cudaMemcpyAsync((char*)s->hulls.p + m.id * hull_bytes, m.hull.p, hull_bytes, cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess && m.wide_count)
-      e = wide::relocate((const uint32_t*)m.wide.p, m.wide_count, s->mesh_wide[m.id], t[2],
-                         (uint32_t*)s->wide_blas.p + (size_t)s->mesh_wide[m.id] * pt::kWideNodeWords, st);
   }
+  if (e == cudaSuccess) e = concat_wide(s, nt, nw, st);
   s->wide_nodes = nw;
   s->counts.primitive_count = (uint32_t)nt;
   s->counts.triangle_index_count = (uint32_t)nt;
@@ -1145,11 +1189,14 @@ static cudaError_t concat_meshes(PulseScene* s) {
 __global__ void k_meta_to_host(const uint32_t* __restrict__ meta, const uint32_t* __restrict__ head,
                                volatile uint32_t* host) {
   if (threadIdx.x < 4) host[threadIdx.x] = meta[threadIdx.x];
-  else if (threadIdx.x < 4 + wide::kHeadWords) host[threadIdx.x] = head[threadIdx.x - 4];
+  else if (head && threadIdx.x < 4 + wide::kHeadWords) host[threadIdx.x] = head[threadIdx.x - 4];
 }
 
-// The eight-wide instance tree from the binary one of n instances just queued on st.
-static cudaError_t collapse_tlas(PulseScene* s, uint32_t n, const uint32_t* meta, cudaStream_t st) {
+// The eight-wide instance tree from the binary one of n instances just queued on st, if the
+// meshes and the instances' records have what it takes.
+static cudaError_t collapse_tlas(PulseScene* s, uint32_t n, const uint32_t* meta, WideTree* wt, cudaStream_t st) {
+  wt->made = false;
+  if (!s->wide_meshes || !s->wide_records) return cudaSuccess;
   const uint32_t n_nodes = 2 * n - 1;
   const size_t cap = wide::capacity(n_nodes);
   cudaError_t e = ensure(s->wide_tlas, cap * pt::kWideNodeWords * 4);
@@ -1160,11 +1207,13 @@ static cudaError_t collapse_tlas(PulseScene* s, uint32_t n, const uint32_t* meta
   if (e == cudaSuccess)
     e = prep::tight_bounds(n, (const float4*)s->instances.p, (const float4*)s->inst_wide.p,
                            (const float*)s->inst_bounds.p, (const float4*)s->hulls.p, (float4*)s->wide_bounds.p, st);
-  if (e != cudaSuccess) return e;
-  s->ctx->stats.kernel_launches += 2;
-  return wide::collapse_tlas((const float4*)s->tlas_nodes.p, n_nodes, meta, (const uint32_t*)s->instance_indices.p,
-                             (float4*)s->inst_wide.p, (const float4*)s->wide_bounds.p, (float4*)s->wide_box.p,
-                             (uint4*)s->wide_tlas.p, (uint32_t*)s->wide_queue.p, (uint32_t*)s->wide_thead.p, st);
+  if (e == cudaSuccess)
+    e = wide::collapse_tlas((const float4*)s->tlas_nodes.p, n_nodes, meta, (const uint32_t*)s->instance_indices.p,
+                            (float4*)s->inst_wide.p, (const float4*)s->wide_bounds.p, (float4*)s->wide_box.p,
+                            (uint4*)s->wide_tlas.p, (uint32_t*)s->wide_queue.p, (uint32_t*)s->wide_thead.p, st);
+  wt->made = e == cudaSuccess;
+  if (wt->made) s->ctx->stats.kernel_launches += 2;
+  return without_wide(e) ? cudaSuccess : e;
 }
 
 static int32_t rebuild_tlas(PulseScene* s, uint32_t n, const PulseBvhParams* tp, uint32_t* count, uint32_t* levels,
@@ -1208,10 +1257,10 @@ static int32_t rebuild_tlas(PulseScene* s, uint32_t n, const PulseBvhParams* tp,
     if (e == cudaSuccess)
       e = bvh::build_direct(in, bvh::Params{tp->bins, tp->max_leaf, 1}, (uint32_t*)s->tlas_nodes.p,
                             (uint32_t*)s->instance_indices.p, (uint32_t*)s->tlas_meta.p, st);
-    if (e == cudaSuccess) e = collapse_tlas(s, n, (const uint32_t*)s->tlas_meta.p, st);
+    if (e == cudaSuccess) e = collapse_tlas(s, n, (const uint32_t*)s->tlas_meta.p, wt, st);
     if (e == cudaSuccess) {
-      k_meta_to_host<<<1, 32, 0, st>>>((const uint32_t*)s->tlas_meta.p, (const uint32_t*)s->wide_thead.p,
-                                       s->meta_mapped);
+      k_meta_to_host<<<1, 32, 0, st>>>((const uint32_t*)s->tlas_meta.p,
+                                       wt->made ? (const uint32_t*)s->wide_thead.p : nullptr, s->meta_mapped);
       e = cudaGetLastError();
     }
     if (e != cudaSuccess) return cuda_err(ctx, e, "TLAS");
@@ -1231,8 +1280,8 @@ static int32_t rebuild_tlas(PulseScene* s, uint32_t n, const PulseBvhParams* tp,
   }
   if (rc == PULSE_OK) {
     uint32_t h[wide::kHeadWords] = {};
-    e = collapse_tlas(s, n, nullptr, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h, s->wide_thead.p, sizeof(h), cudaMemcpyDeviceToHost, st);
+    e = collapse_tlas(s, n, nullptr, wt, st);
+    if (e == cudaSuccess && wt->made) e = cudaMemcpyAsync(h, s->wide_thead.p, sizeof(h), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) rc = cuda_err(ctx, e, "TLAS: eight-wide tree");
     wt->read(h);
@@ -1359,10 +1408,15 @@ int32_t pulse_instances_set(PulseScene* s, const PulseInstanceDesc* inst, uint32
   e = upload_keep(d_ii, ii.data(), (size_t)n * sizeof(prep::InstanceIn), st);
   if (e == cudaSuccess) e = ensure(s->instances, (size_t)n * 160);
   if (e == cudaSuccess) e = ensure(s->inst_bounds, (size_t)n * 36);
-  if (e == cudaSuccess) e = ensure(s->inst_wide, (size_t)n * pt::kWideInstRows * 16);
+  s->wide_records = false;
+  if (e == cudaSuccess && s->wide_meshes) {
+    e = ensure(s->inst_wide, (size_t)n * pt::kWideInstRows * 16);
+    s->wide_records = e == cudaSuccess;
+    if (without_wide(e)) e = cudaSuccess;
+  }
   if (e == cudaSuccess)
     e = prep::instances((const prep::InstanceIn*)d_ii.p, n, (const float4*)s->blas_nodes.p, (float4*)s->instances.p,
-                        (float*)s->inst_bounds.p, (float4*)s->inst_wide.p, st);
+                        (float*)s->inst_bounds.p, s->wide_records ? (float4*)s->inst_wide.p : nullptr, st);
   if (e == cudaSuccess) e = upload_keep(d_lights, lights.data(), (size_t)L * sizeof(prep::LightIn), st);
   if (e == cudaSuccess) e = ensure(s->tri_cdfs, (size_t)cdf_len * 4);
   if (e == cudaSuccess) e = ensure(s->mesh_areas, (size_t)L * 4);
@@ -1452,7 +1506,8 @@ int32_t pulse_instances_update(PulseScene* s, const uint32_t* idx, const float* 
   if (e == cudaSuccess) e = upload_keep(d_slot, idx, (size_t)n * 4, st);
   if (e == cudaSuccess)
     e = prep::instances((const prep::InstanceIn*)d_ii.p, n, (const float4*)s->blas_nodes.p, (float4*)s->instances.p,
-                        (float*)s->inst_bounds.p, (float4*)s->inst_wide.p, st, (const uint32_t*)d_slot.p);
+                        (float*)s->inst_bounds.p, s->wide_records ? (float4*)s->inst_wide.p : nullptr, st,
+                        (const uint32_t*)d_slot.p);
   int32_t rc = e == cudaSuccess ? PULSE_OK : cuda_err(ctx, e, "instance update");
   ctx->stats.kernel_launches += n ? 1 : 0;
   uint32_t tlas_count = 1, tlas_levels = 1;

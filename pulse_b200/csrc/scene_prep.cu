@@ -83,12 +83,13 @@ __global__ void k_instances(const InstanceIn* __restrict__ in, uint32_t n, const
   o[8] = make_float4(__uint_as_float(x.triangle_offset), __uint_as_float(x.triangle_count),
                      __uint_as_float(x.index_offset), __uint_as_float(x.node_offset));
   o[9] = make_float4(__uint_as_float(x.material_index), 0.0f, 0.0f, 0.0f);
-  // the wide traversal's record (pt_wide.cuh); its TLAS leaf comes with the tree
-  float4* wo = wide_out + (size_t)i * kWideInstRows;
-  for (int c = 0; c < 4; ++c) wo[c] = make_float4(inv[4 * c], inv[4 * c + 1], inv[4 * c + 2], inv[4 * c + 3]);
-  wo[4] = make_float4(__uint_as_float(x.wide_root), __uint_as_float(x.wide_leaf), x.wide_slack, __uint_as_float(x.hull));
-  wo[5] = make_float4(__uint_as_float(x.index_offset), __uint_as_float(x.node_offset),
-                      __uint_as_float(kWideRootLeaf), 0.0f);
+  if (wide_out) {  // the wide traversal's record (pt_wide.cuh); its TLAS leaf comes with the tree
+    float4* wo = wide_out + (size_t)i * kWideInstRows;
+    for (int c = 0; c < 4; ++c) wo[c] = make_float4(inv[4 * c], inv[4 * c + 1], inv[4 * c + 2], inv[4 * c + 3]);
+    wo[4] = make_float4(__uint_as_float(x.wide_root), __uint_as_float(x.wide_leaf), x.wide_slack, __uint_as_float(x.hull));
+    wo[5] = make_float4(__uint_as_float(x.index_offset), __uint_as_float(x.node_offset),
+                        __uint_as_float(kWideRootLeaf), 0.0f);
+  }
   // World bounds of the root box (src/scene/mod.rs:625-658).
   const float4 lo = blas_nodes[2 * (size_t)x.node_offset], hi = blas_nodes[2 * (size_t)x.node_offset + 1];
   const M4 m{o[0], o[1], o[2], o[3]};

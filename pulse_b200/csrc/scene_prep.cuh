@@ -21,7 +21,7 @@ struct InstanceIn {
 // prepare_mesh_instances (src/scene/mod.rs:561-681) per instance: the 160 B
 // record with the inverse transform, and the world bounds of the BLAS root
 // (8 transformed corners) with their centre -> bounds9; the wide traversal's record
-// (pt_wide.cuh) -> wide_out.  With `slot`, input i writes records and bounds slot[i] (an
+// (pt_wide.cuh) -> wide_out, unless it is null.  With `slot`, input i writes records and bounds slot[i] (an
 // incremental update of some instances).
 cudaError_t instances(const InstanceIn* in, uint32_t n, const float4* blas_nodes, float4* inst_out, float* bounds9,
                       float4* wide_out, cudaStream_t st, const uint32_t* slot = nullptr);

@@ -10,9 +10,9 @@ import numpy as np
 import pytest
 
 import oracle
-from pulse_b200 import scenes
+from pulse_b200 import _ffi, scenes
 from pulse_b200.layout import Instance, Material, Mesh
-from pulse_b200.tracer import Scene, Target, gbuffer_primary, render_forward
+from pulse_b200.tracer import Context, PulseError, Scene, Target, gbuffer_primary, render_forward
 
 pytestmark = pytest.mark.gpu
 
@@ -392,3 +392,54 @@ def test_instance_out_of_range_keeps_the_binary_trees(ctx, count, far):
         for a, b in (("instance_index", "instance"), ("triangle_index", "triangle")):
             assert np.array_equal(got[a], ref[b])
     sc.close()
+
+
+def test_no_memory_for_the_wide_trees():
+    """Every allocation of a scene's preparation fails once.  The calls return PULSE_ERR_OOM and
+    succeed when repeated, or, where only the wide trees wanted the memory, succeed at once; the
+    scene renders the oracle's bits either way."""
+    meshes, instances, leaf, _, _ = _scene("coplanar")
+    mats = [MAT[0], Material((0.7, 0.7, 0.7, 1), (3.0, 3.0, 3.0, 1), 0.8, 0.5, 0.0)]
+    instances[4].material = 1
+    view = scenes.bevy_view((1.0, 3.0, 5.0), (0.0, 0.0, 0.0), aspect=1.5)
+    params = dict(max_depth=4, nee_mode=2, light_pick=1)
+    sb = oracle.assemble(meshes, mats, instances, 20, leaf)
+    ref = np.zeros((24, 36, 4), np.float32)
+    oracle.render(sb, view, 36, 24, 0, image=ref, **params)
+
+    def prepare(sc):
+        ids = [sc.upload_mesh(m, 20, leaf) for m in meshes]
+        sc.set_materials(mats)
+        sc.set_instances(instances, ids)
+        sc.set_instances(instances, ids)  # into the second set of buffers
+        sc.update_instances([2], [instances[2].columns()])
+
+    without = refused = 0
+    for skip in range(1000):
+        with Context(0) as c:  # (its workspaces are not there yet)
+            sc = Scene(c)
+            c.check(c.lib.pulse_debug_fail_allocations_after(c.h, skip, 1), "arm")
+            try:
+                try:
+                    prepare(sc)
+                    failed = False
+                except PulseError as e:
+                    assert e.code == _ffi.PULSE_ERR_OOM, skip
+                    failed = True
+                try:
+                    Target(c, 8, 8).close()
+                except PulseError:
+                    break  # the failure was still to come: the preparation allocates no more
+            finally:
+                c.check(c.lib.pulse_debug_fail_allocations_after(c.h, 0, 0), "disarm")
+            if failed:
+                refused += 1
+                prepare(sc)
+            else:
+                without += 1
+            tg = Target(c, 36, 24)
+            render_forward(sc, view, tg, 0, **params)
+            assert np.array_equal(tg.download().view(np.uint32), ref.view(np.uint32)), skip
+            tg.close()
+            sc.close()
+    assert refused > 0 and without > 0
