@@ -12,6 +12,15 @@
  *     Nothing aborts or traps; pulse_last_error() gives a message.
  *   - Host pointers passed in are read during the call only (the library
  *     copies).  The library owns all device memory.
+ *   - A context keeps device memory between calls: the path buffers of its
+ *     largest frame, and the workspaces of pulse_trace (44 bytes a ray),
+ *     pulse_render_backward (96 bytes a path), pulse_build_blas/_tlas and
+ *     pulse_mesh_upload, up to 512 MiB, and of the tree builds of
+ *     pulse_build_blas/_tlas, up to another 512 MiB (a larger workspace is given
+ *     back by the call that grew it).  pulse_ctx_destroy gives all of it back.
+ *     A prepared scene holds its eight-wide trees besides the binary ones (96
+ *     bytes a node, 4 a triangle, once for each mesh and once joined); without
+ *     memory for them its calls succeed and rays take the binary trees.
  *   - One PulseCtx per render thread, one CUDA stream per context (and two
  *     internal ones for pipelined frames, pulse_ctx_set_pipeline); calls are
  *     asynchronous on that stream except downloads and pulse_sync().
