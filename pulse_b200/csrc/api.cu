@@ -117,7 +117,7 @@ struct MeshRec {
   DevBuf wide, leaf_of, hull;
   bool wide_ok = false;
   uint32_t wide_count = 0, wide_root = 0, wide_levels = 0;
-  float wide_slack = 0.0f;
+  float wide_slack = 0.0f, wide_slack_abs = 0.0f;  // pt_wide.cuh
 };
 
 struct PulseScene {
@@ -928,9 +928,10 @@ static cudaError_t collapse_mesh(PulseCtx* ctx, MeshRec& m, cudaStream_t st) {
     m.wide_count = h[wide::kCount];
     m.wide_root = h[wide::kRoot];
     m.wide_levels = h[wide::kLevels];
-    float area;
-    std::memcpy(&area, &h[wide::kArea], 4);
-    m.wide_slack = wide::slack(area);
+    std::memcpy(&m.wide_slack, &h[wide::kSlack], 4);
+    std::memcpy(&m.wide_slack_abs, &h[wide::kSlackAbs], 4);
+    if (!(m.wide_slack <= pt::kMostSlack)) m.wide_slack = pt::kNoSlackBound, m.wide_slack_abs = 0.0f;
+    m.wide_slack = std::max(m.wide_slack, pt::kLeastSlack);
     const size_t bytes = (size_t)m.wide_count * pt::kWideNodeWords * 4;
     e = ensure(m.wide, bytes);
     if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(m.wide.p, out, bytes, cudaMemcpyDeviceToDevice, st);
@@ -968,8 +969,10 @@ struct WideTree {
   bool made = false;  // a collapse was queued
   bool ok = false;
   uint32_t levels = 0, count = 0;
+  float slack = 0.0f;  // the largest of the loose instances
   void read(const uint32_t* head) {
     ok = made && !head[wide::kBad];
+    std::memcpy(&slack, &head[wide::kSlack], 4);
     levels = head[wide::kLevels];
     count = head[wide::kCount];
   }
@@ -979,12 +982,10 @@ struct WideTree {
 // take the wide traversal.
 static void decide_wide(PulseScene* s, const std::vector<prep::InstanceIn>& ii, const WideTree& tree) {
   bool ok = tree.ok && !ii.empty();
-  float slack = pt::kLeastSlack;
   uint32_t levels = 0;
   for (const MeshRec& m : s->meshes)
     if (m.alive) {
       ok = ok && m.wide_ok;
-      slack = std::max(slack, m.wide_slack);
       levels = std::max(levels, m.wide_levels);
     }
   // TLAS: every child hit, up to a fixed size, and beyond it an entry a level and the
@@ -999,7 +1000,7 @@ static void decide_wide(PulseScene* s, const std::vector<prep::InstanceIn>& ii, 
   ok = ok && s->dev.wide_stack <= 96 && std::max((size_t)tree.count, ii.size()) < (1u << pt::kTopIndexBits) &&
        s->wide_nodes < (1ull << pt::kWideIndexBits) && s->counts.triangle_index_count < (1u << pt::kWideFirstBits);
   for (size_t i = 0; ok && i < ii.size(); ++i) ok = wide_transform(ii[i].object_world);
-  s->dev.wide_slack = slack;
+  s->dev.wide_slack = std::max(tree.slack, pt::kLeastSlack);
   s->dev.wide = ok ? 1u : 0u;
 }
 
@@ -1369,6 +1370,7 @@ int32_t pulse_instances_set(PulseScene* s, const PulseInstanceDesc* inst, uint32
     const MeshRec& mesh = s->meshes[d.mesh_id];
     ii[i].wide_root = mesh.wide_root ? 0u : s->mesh_wide[d.mesh_id] | (1u << 24);
     ii[i].wide_slack = mesh.wide_slack;
+    ii[i].wide_slack_abs = mesh.wide_slack_abs;
     ii[i].hull = d.mesh_id;
     ii[i].wide_leaf = mesh.wide_root ? mesh.wide_root + t[2] : 0u;
     const float* em = s->host_materials[d.material_index].emissive;

@@ -41,7 +41,7 @@ struct DevScene {
   const uint4* __restrict__ wide_blas;       // 6 x uint4 per node, every mesh's tree
   const uint4* __restrict__ wide_tlas;
   const float4* __restrict__ inst_wide;      // 6 x float4 per instance (pt_wide.cuh)
-  float wide_slack;                          // the largest slack of the scene's meshes
+  float wide_slack;                          // the largest slack of the scene's instances
   uint32_t wide, wide_stack, wide_top;       // stack entries: in all, and for the TLAS
 };
 

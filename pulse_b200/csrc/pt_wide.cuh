@@ -31,10 +31,16 @@
 //   * Every leaf holding a hit with t <= M must be visited.  Quantized boxes
 //     contain the exact ones with 1/64 of a quantum to spare, the far planes are
 //     scaled by 1 + 2e-6 (the rounding of a plane's t is below 5e-7 of it
-//     plus 1/100 of a quantum), and boxes are skipped only beyond the gate times
-//     1 + slack: the computed t of a hit may lie before its box by the rounding of
-//     the reference's triangle test, 56 * 2^-24 * |e1||e2| / eps_par of the distance at
-//     worst, which the slack of the scene covers (1e-4 to 0.02).
+//     plus 1/100 of a quantum), and boxes are skipped only beyond the gate and a slack:
+//     the computed t of a hit may lie before its box by the rounding of the reference's
+//     triangle test, which for a ray along the plane of a large triangle is a good part of
+//     the distance.  triangle_slack (wide.cu) bounds it by (t + longer edge) * slack; meshes
+//     whose triangles have no such bound are not culled by distance at all.  (A slack of at most
+//     0.02 answered 1 in 10,000 rays along triangles of 20 to 200 units wrongly.  Without it
+//     720p frames of a terrain of 400 units in 8 to 96 squares a side take 0 to 8% longer
+//     than with it, 17% at worst; the binary trees take 1.2 to 1.6 times as long.)  Left out is a hit
+//     whose ray passes beside the triangle by a rounding and enters its box later by that
+//     over the direction's component, if that is below 0.01.
 // Rays and scenes outside these arguments (a direction that is not
 // normalized, coordinates above 1e9, boxes that do not nest, transforms that are
 // not affine or nearly singular, stacks or iteration caps that bind) take the binary
@@ -69,8 +75,8 @@ constexpr uint32_t kWideIndexMask = (1u << kWideIndexBits) - 1u;
 // In the TLAS, whose boxes overlap and whose leaves are costly, every child hit is a
 // stack word of its own, the nearest on top: the entry distance's upper 14
 // bits (rounded down: entries beyond the record are dropped when popped), then
-// interior: child index << 1; leaf: instance << 1 | 1.  The distance of a child that may
-// hold a mesh of more than the least slack is lowered by the largest slack of the scene.
+// interior: child index << 1; leaf: instance << 1 | 1.  The distance of a child that
+// holds an instance of more than the least slack is lowered by the largest slack of the scene.
 // Where the children hit do not fit, one is gone on with and the node itself is the
 // entry of the rest, to be visited again without the children that were missed or are done:
 // kTopAgain | those << 17 | node (distances stay below 2^97, boxes lying within 1e9, so no
@@ -80,6 +86,10 @@ constexpr uint32_t kTopIndexBits = 17, kTopIndexMask = (1u << kTopIndexBits) - 1
 constexpr uint32_t kTopAgain = 0xe0000000u;
 constexpr uint32_t kLooseRef = 0x80000000u;
 constexpr float kLeastSlack = 1e-4f;
+// Node word 4 of the TLAS from this bit: the interior children that hold a loose instance.
+constexpr uint32_t kTopLooseShift = 24;
+// A slack that culls nothing, and up to which one bounds a hit (wide.cu).
+constexpr float kNoSlackBound = 1e9f, kMostSlack = 0.5f;
 // Entries up to which children are pushed: 16 for trees of up to 3 levels (the 1080p
 // sphere frame: 9.3 ms, with 24 and the less L1 they leave 9.45), 24 for deeper ones as far as
 // the stack of both levels stays within 36 words, the most with which four blocks fit an SM
@@ -99,8 +109,9 @@ constexpr uint32_t kWideStack = 36, kTopLeast = 12, kTopShallow = 16, kTopMost =
 constexpr uint32_t kPool = 64;
 
 // An instance's record for entering it (DevScene::inst_wide), 96 bytes: its
-// world-to-object matrix, (root group of the mesh's tree, or 0 and its only leaf's reference,
-// slack of the mesh, 0), (first triangle slot, first binary node, TLAS leaf node or kWideRootLeaf, 0).
+// world-to-object matrix (affine: the first three columns' w hold the mesh's slack in units of
+// its space, 0, 0), (root group of the mesh's tree, or 0 and its only leaf's reference, slack of the
+// mesh, mesh id), (first triangle slot, first binary node, TLAS leaf node or kWideRootLeaf, 0).
 constexpr uint32_t kWideInstRows = 6;
 
 enum WideWord : uint32_t {
@@ -385,14 +396,14 @@ __device__ __forceinline__ uint32_t wide_node(const WideRay& R, const DevScene& 
     }
     const uint4 ra = __ldg(np + 1), rb = __ldg(np + 5);  // references of the leaves
     const uint32_t ref[8] = {ra.x, rb.w, rb.z, rb.y, rb.x, ra.w, ra.z, ra.y};
-    const uint32_t child = w.child & kWideIndexMask;
+    const uint32_t child = w.child & kWideIndexMask, loose = w.child >> kTopLooseShift;
     const float less = __fdividef(1.0f, 1.0f + slack);
     float best = 3.4e38f;
     uint32_t best_e = 0, best_at = sp, e = 0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const bool inner = (uint32_t)k < w.ni;
-      if (inner || (ref[k] & kLooseRef)) tn[k] = fmaxf((tn[k] - slack) * less, 0.0f);
+      if (inner ? (loose >> k) & 1u : ref[k] >> 31) tn[k] = fmaxf((tn[k] - slack) * less, 0.0f);
       if ((hit & (1u << k)) && tn[k] <= bound) {
         e = ((__float_as_uint(tn[k]) >> 17) << 18) | (inner ? (child + (uint32_t)k) << 1 : (ref[k] << 1) | 1u);
         if (tn[k] < best) { best = tn[k]; best_e = e; best_at = sp; }
@@ -491,10 +502,12 @@ __device__ __forceinline__ uint32_t wide_tri(const WideRay& R, const DevScene& S
   return wide_pop(R, R.u(kwSp));
 }
 
-// The object-space ray of an instance, as trace_do enters it; returns the length of the
-// transformed direction.
+// The object-space ray of an instance (the first columns of its record), as trace_do enters it;
+// returns the length of the transformed direction.  The matrix is affine and the ray finite, so
+// the position's fourth component is that of the fourth column.
 __device__ __forceinline__ float wide_object_ray(const M4& w2o, float3 wo, float3 wd, float3& o, float3& d) {
-  o = transform_position(w2o, wo);
+  const float4 p = mul4(w2o, wo.x, wo.y, wo.z, 1.0f);
+  o = v3(p.x / w2o.c3.w, p.y / w2o.c3.w, p.z / w2o.c3.w);
   const float3 dw = transform_direction(w2o, wd);
   const float len = length(dw);
   d = divs(dw, len);
@@ -523,8 +536,9 @@ __device__ __forceinline__ uint32_t wide_instance(const WideRay& R, const DevSce
   R.setf3(kwDX, d);
   R.setf(kwLen, len);
   R.setf(kwEps, fmaxf(R.f(kwEps), __fdividef(1.6e-6f * max_abs3(o), len)));
-  R.setf(kwSlack, wx.z);
-  R.setf(kwCull, (fminf(wide_bound(rec_t, wx.z), far) + 1e-3f * (1.0f + max_abs3(wo))) * len);
+  const float slack = fmaxf(wx.z, __fdividef(w2o.c0.w, len));
+  R.setf(kwSlack, slack);
+  R.setf(kwCull, (fminf(wide_bound(rec_t, slack), far) + 1e-3f * (1.0f + max_abs3(wo))) * len);
   const uint32_t root = __float_as_uint(wx.x);
   R.set(kwCur, __float_as_uint(wx.y));
   R.set(kwGrp, root);

@@ -86,6 +86,7 @@ __global__ void k_instances(const InstanceIn* __restrict__ in, uint32_t n, const
   if (wide_out) {  // the wide traversal's record (pt_wide.cuh); its TLAS leaf comes with the tree
     float4* wo = wide_out + (size_t)i * kWideInstRows;
     for (int c = 0; c < 4; ++c) wo[c] = make_float4(inv[4 * c], inv[4 * c + 1], inv[4 * c + 2], inv[4 * c + 3]);
+    wo[0].w = x.wide_slack_abs;
     wo[4] = make_float4(__uint_as_float(x.wide_root), __uint_as_float(x.wide_leaf), x.wide_slack, __uint_as_float(x.hull));
     wo[5] = make_float4(__uint_as_float(x.index_offset), __uint_as_float(x.node_offset),
                         __uint_as_float(kWideRootLeaf), 0.0f);
@@ -138,6 +139,10 @@ __global__ void __launch_bounds__(256) k_tight_bounds(uint32_t n, const float4* 
             fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, off)));
   }
   if (lane != 0u) return;
+  // hits may lie before their box by the mesh's slack, its absolute part in world units along any direction
+  const float4 w0 = __ldg(inst_wide + (size_t)i * kWideInstRows), wx = __ldg(inst_wide + (size_t)i * kWideInstRows + 4);
+  const float stretch = sqrtf(dot(xyz(m.c0), xyz(m.c0)) + dot(xyz(m.c1), xyz(m.c1)) + dot(xyz(m.c2), xyz(m.c2)));
+  const float slack = fminf(fmaxf(wx.z, w0.w * stretch), kNoSlackBound);
   const float* b = bounds9 + (size_t)i * 9;
   float l[3] = {b[0], b[1], b[2]}, u[3] = {b[3], b[4], b[5]};
   auto entry = [](const M4& x) {
@@ -152,7 +157,7 @@ __global__ void __launch_bounds__(256) k_tight_bounds(uint32_t n, const float4* 
       if (x <= y) l[k] = x, u[k] = y;
     }
   }
-  out[2 * (size_t)i] = make_float4(l[0], l[1], l[2], 0.0f);
+  out[2 * (size_t)i] = make_float4(l[0], l[1], l[2], slack);
   out[2 * (size_t)i + 1] = make_float4(u[0], u[1], u[2], 0.0f);
 }
 

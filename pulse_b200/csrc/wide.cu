@@ -36,9 +36,12 @@ struct LeafSink {
     else records[(size_t)instance_of[slot] * pt::kWideInstRows + 5].z = __uint_as_float(node);
   }
   // A TLAS element's reference.
-  __device__ __forceinline__ uint32_t ref(uint32_t slot) const {
+  __device__ __forceinline__ uint32_t ref(uint32_t slot, uint32_t* head) const {
     const uint32_t i = instance_of[slot];
-    return i | (records[(size_t)i * pt::kWideInstRows + 4].z > pt::kLeastSlack ? pt::kLooseRef : 0u);
+    const float slack = bounds[2 * (size_t)i].w;
+    if (slack <= pt::kLeastSlack) return i;
+    atomicMax(head + kSlack, __float_as_uint(slack));
+    return i | pt::kLooseRef;
   }
 };
 
@@ -152,7 +155,7 @@ __device__ void make_node(const float4* __restrict__ nodes, uint32_t b, uint32_t
       for (uint32_t i = 0; i < count; ++i) leaf_of.put(start + i, c[k]);
       for (uint32_t i = 0; i < mult[k]; ++i) {
         set_box(7u - nl, c[k]);
-        words[pt::wide_ref_word(nl++)] = tlas ? leaf_of.ref(start + i) : leaf_ref(start, count, head);
+        words[pt::wide_ref_word(nl++)] = tlas ? leaf_of.ref(start + i, head) : leaf_ref(start, count, head);
       }
       continue;
     }
@@ -197,22 +200,25 @@ __device__ void make_root_leaf(uint32_t start, uint32_t count, uint32_t* out, co
   out[3] = count << 28;
   for (uint32_t i = 0; i < count; ++i) {
     leaf_of.put(start + i, pt::kWideRootLeaf);
-    out[pt::wide_ref_word(i)] = leaf_of.ref(start + i);
+    out[pt::wide_ref_word(i)] = leaf_of.ref(start + i, head);
   }
 }
 
 // The planes of TLAS node i from its instances' bounds and its interior children's
-// boxes (made before it), and its own box.
+// boxes (made before it), its interior children that hold a loose instance, and its own box (and
+// in the first w whether it holds one).
 __device__ void fit_node(uint32_t i, uint32_t* out, const LeafSink& leaf_of, uint32_t* head) {
   uint32_t* w = out + (size_t)i * pt::kWideNodeWords;
   const uint32_t ni = (w[3] >> 24) & 15u, nl = w[3] >> 28, used = used_slots(ni, nl);
   Boxes box;
   float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
+  uint32_t loose = 0;
   for (uint32_t k = 0; k < 8; ++k) {
     if (!(used & (1u << k))) continue;
     const float4* b = k < ni ? leaf_of.node_box + 2 * (size_t)((w[4] & pt::kWideIndexMask) + k)
                              : leaf_of.bounds + 2 * (size_t)(w[pt::wide_ref_word(7u - k)] & ~pt::kLooseRef);
     const float4 a = __ldcg(b), z = __ldcg(b + 1);
+    if (a.w > pt::kLeastSlack) loose |= 1u << k;
     box.lo[k][0] = a.x, box.lo[k][1] = a.y, box.lo[k][2] = a.z;
     box.hi[k][0] = z.x, box.hi[k][1] = z.y, box.hi[k][2] = z.z;
     for (int j = 0; j < 3; ++j) {
@@ -220,7 +226,8 @@ __device__ void fit_node(uint32_t i, uint32_t* out, const LeafSink& leaf_of, uin
       hi[j] = fmaxf(hi[j], box.hi[k][j]);
     }
   }
-  leaf_of.node_box[2 * (size_t)i] = make_float4(lo[0], lo[1], lo[2], 0.0f);
+  if (ni) w[4] |= (loose & ((1u << ni) - 1u)) << pt::kTopLooseShift;
+  leaf_of.node_box[2 * (size_t)i] = make_float4(lo[0], lo[1], lo[2], loose ? 1.0f : 0.0f);
   leaf_of.node_box[2 * (size_t)i + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
   quantize(w, box, used, head);
 }
@@ -250,6 +257,7 @@ __global__ void __launch_bounds__(kBlock) k_collapse(const float4* __restrict__ 
     const uint32_t start = __float_as_uint(rlo.w);
     const bool tlas = leaf_of.instance_of != nullptr;
     head[kBad] = 0u;
+    if (tlas) head[kSlack] = 0u;
     head[kLevels] = count && tlas ? 1u : 0u;
     head[kRoot] = count && !tlas ? leaf_ref(start, count, head) : 0u;
     queue[0] = 0u;
@@ -342,16 +350,47 @@ __global__ void __launch_bounds__(kBlock) k_relocate(const uint32_t* __restrict_
   for (uint32_t k = 0; k < pt::kWideNodeWords; ++k) b[k] = w[k];
 }
 
+// How far before its box the computed t of a hit may lie, for a ray of any direction that
+// passes the test's |a| >= eps_par: (t + L) * slack(triangle), L the longer edge.  First-order
+// rounding analysis of ray_triangle_v (u = 2^-24; products, sums and the edges' three-term
+// products bounded by permanents of the absolute values): t, u and v are off by at most
+// 27 u (t + L) |e1||e2| / |a| along the plane.  With edges that leave a plane of two axes by at
+// most e (its normal's component n, S = |e1||e2| / |n|), products with the third axis shrink
+// with e and the bound is u (t + L) (35 S + e L (100 S + 106) / |a|): a triangle that lies in
+// such a plane, like a wall or a floor, is exact to roundings at any size.  Both constants are
+// raised for the second order, which needs slack < 0.5; beyond there is no bound.
+__device__ __forceinline__ float triangle_slack(float3 e1, float3 e2, float l1, float l2) {
+  constexpr float kU = 5.9604645e-8f, kEps = 0.99e-4f;
+  const float x1[3] = {e1.x, e1.y, e1.z}, x2[3] = {e2.x, e2.y, e2.z};
+  const float area = l1 * l2, longer = fmaxf(l1, l2);
+  float k = 32.0f * area / kEps;
+  for (int i = 0; i < 3; ++i) {
+    const int a = (i + 1) % 3, b = (i + 2) % 3;
+    const float off = fmaxf(fabsf(x1[i]), fabsf(x2[i]));
+    const float s = area / fabsf(x1[a] * x2[b] - x1[b] * x2[a]);
+    k = fminf(k, 40.0f * s + off * longer * (110.0f * s + 120.0f) / kEps);  // (NaN: the general bound)
+  }
+  return kU * k;
+}
+
 __global__ void __launch_bounds__(kBlock) k_extents(const float4* __restrict__ prims, uint32_t n, uint32_t* head) {
-  float area = 0.0f;
+  float rel = 0.0f, abs = 0.0f;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float3 p0 = pt::xyz(prims[3 * (size_t)i]), p1 = pt::xyz(prims[3 * (size_t)i + 1]),
                  p2 = pt::xyz(prims[3 * (size_t)i + 2]);
+    const float3 e1 = pt::sub(p1, p0), e2 = pt::sub(p2, p0);
+    const float l1 = pt::length(e1), l2 = pt::length(e2);
     // a NaN vertex cannot be hit: its triangle does not count
-    area = fmaxf(area, pt::length(pt::sub(p1, p0)) * pt::length(pt::sub(p2, p0)));
+    const float s = triangle_slack(e1, e2, l1, l2);
+    rel = fmaxf(rel, s);
+    abs = fmaxf(abs, s * fmaxf(l1, l2));
   }
-  const uint32_t am = __reduce_max_sync(0xffffffffu, __float_as_uint(area));
-  if ((threadIdx.x & 31) == 0) atomicMax(head + kArea, am);
+  const uint32_t rm = __reduce_max_sync(0xffffffffu, __float_as_uint(rel));
+  const uint32_t am = __reduce_max_sync(0xffffffffu, __float_as_uint(abs));
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(head + kSlack, rm);
+    atomicMax(head + kSlackAbs, am);
+  }
 }
 
 }  // namespace
@@ -401,12 +440,6 @@ cudaError_t extents(const float4* prims, uint32_t n, uint32_t* head, cudaStream_
   const uint32_t blocks = (n + kBlock - 1) / kBlock;
   k_extents<<<blocks < 1184u ? blocks : 1184u, kBlock, 0, st>>>(prims, n, head);
   return cudaGetLastError();
-}
-
-float slack(float area) {
-  // 56 * 2^-24 * |e1||e2| / eps_par with the default eps_par of 1e-4
-  const float s = 56.0f * 5.9604645e-8f * area / 1e-4f;
-  return s < pt::kLeastSlack ? pt::kLeastSlack : s > 0.02f ? 0.02f : s;  // NaN: 0.02
 }
 
 }  // namespace wide

@@ -11,7 +11,10 @@ enum Head : uint32_t {
   kCount,   // wide nodes
   kBad,     // nonzero: no wide tree (a box not finite or above 1e9, a leaf out of the references' range)
   kLevels,  // levels of the wide tree
-  kArea,    // largest |e1| |e2| of a triangle (float bits)
+  // How far the computed t of a hit may lie before its box (float bits): share of the
+  // distance, and in units of the space.  A mesh's two (extents), or in the first the largest
+  // of both of a TLAS's loose instances.
+  kSlack, kSlackAbs,
   kHeadWords = 8
 };
 
@@ -26,7 +29,7 @@ cudaError_t collapse(const float4* nodes, uint32_t n_nodes, uint4* out, uint32_t
 
 // The same for an instance tree, whose elements' leaf nodes go into the instances'
 // records (pt_wide.cuh) and whose boxes are those of the instances' own bounds (two float4
-// each; node_box: scratch of two float4 per node).  meta: the words of a
+// each, the first's w the instance's slack; node_box: scratch of two float4 per node).  meta: the words of a
 // bvh::build_direct queued before (kBad and nothing read if it failed), or nullptr.
 cudaError_t collapse_tlas(const float4* nodes, uint32_t n_nodes, const uint32_t* meta, const uint32_t* instance_of,
                           float4* records, const float4* bounds, float4* node_box, uint4* out, uint32_t* queue,
@@ -42,11 +45,7 @@ cudaError_t hull(const uint4* wide_nodes, uint32_t n_wide, const float4* nodes, 
 cudaError_t relocate(const uint32_t* nodes, uint32_t n, uint32_t node_add, uint32_t slot_add, uint32_t* out,
                      cudaStream_t st);
 
-// Raises head's kArea (zero to begin with) to that of n std430 triangles.
+// Raises head's kSlack and kSlackAbs (zero to begin with) to those of n std430 triangles.
 cudaError_t extents(const float4* prims, uint32_t n, uint32_t* head, cudaStream_t st);
-
-// Share of the distance by which the computed t of a hit may lie before its
-// box (pt_wide.cuh), for triangles of the given extent: within [1e-4, 0.02].
-float slack(float area);
 
 }  // namespace wide

@@ -443,3 +443,52 @@ def test_no_memory_for_the_wide_trees():
             tg.close()
             sc.close()
     assert refused > 0 and without > 0
+
+
+def _rays_along(triangles, n, size, seed):
+    """Rays that meet a triangle at a small angle, most of them close to an edge."""
+    rng = np.random.default_rng(seed)
+    t = triangles[rng.integers(0, len(triangles), n)]
+    e1 = t[:, 1] - t[:, 0]
+    normal = np.cross(e1, t[:, 2] - t[:, 0])
+    normal /= np.linalg.norm(normal, axis=1, keepdims=True)
+    side = np.cross(normal, e1)
+    along = e1 * rng.normal(size=(n, 1)) + side * rng.normal(size=(n, 1))
+    along /= np.linalg.norm(along, axis=1, keepdims=True)
+    d = along + normal * (rng.choice([-1.0, 1.0], n) * np.exp(rng.uniform(np.log(1e-8), np.log(1e-3), n)))[:, None]
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    b = rng.uniform(size=(n, 3))
+    b[: 3 * n // 4, 0] *= np.exp(rng.uniform(np.log(1e-7), 0.0, 3 * n // 4))
+    b /= b.sum(1, keepdims=True)
+    b = rng.permuted(b, axis=1)
+    o = (t * b[:, :, None]).sum(1) - d * (size * np.exp(rng.uniform(np.log(1e-2), np.log(3.0), n)))[:, None]
+    return np.concatenate([o, d], 1).astype(np.float32)
+
+
+@pytest.mark.parametrize("joined", [False, True])
+@pytest.mark.parametrize("size,scale", [(200.0, 1.0), (20.0, 1.0), (2.0, 1.0), (0.2, 1000.0)])
+def test_rays_along_large_triangles_equal_the_oracle(ctx, size, scale, joined):
+    """Triangles of up to hundreds of units: the rounding of a hit's distance is a good part of
+    the distance itself, so a hit may lie far before the box that holds it."""
+    rng = np.random.default_rng(21)
+    p = (rng.uniform(-size, size, (200, 1, 3)) + rng.normal(size=(200, 3, 3)) * size * 0.5).astype(np.float32)
+    p = np.concatenate([p, (p[:100, :1] + rng.normal(size=(100, 3, 3)) * size * 0.01)]).astype(np.float32)
+
+    def mesh(q):
+        q = q.reshape(-1, 3)
+        return Mesh(q, np.tile([0.0, 1.0, 0.0], (len(q), 1)), np.zeros((len(q), 2)), np.arange(len(q), dtype=np.uint32))
+
+    world = scenes.trs(scale=(scale, scale, scale))
+    meshes = [mesh(p)] if joined else [mesh(q) for q in p]
+    instances = [Instance(k, 0, world) for k in range(len(meshes))]
+    rays = _rays_along(p.astype(np.float64) * scale, 150000, size * scale, 22)
+    ref = oracle.trace(oracle.assemble(meshes, MAT, instances, 20, 8, 2, 2), rays)
+    sc = Scene(ctx)
+    ids = [sc.upload_mesh(m, 20, 8) for m in meshes]
+    sc.set_materials(MAT)
+    sc.set_instances(instances, ids, 2, 2)
+    got = sc.trace(rays)
+    sc.close()
+    assert np.array_equal(got["t"].view(np.uint32), ref["t"].view(np.uint32))
+    for a, b in (("instance_index", "instance"), ("triangle_index", "triangle")):
+        assert np.array_equal(got[a], ref[b])
