@@ -1206,7 +1206,7 @@ static cudaError_t collapse_tlas(PulseScene* s, uint32_t n, const uint32_t* meta
   if (e == cudaSuccess) e = ensure(s->wide_box, cap * 32);
   if (e == cudaSuccess) e = ensure(s->wide_bounds, (size_t)n * 32);
   if (e == cudaSuccess)
-    e = prep::tight_bounds(n, (const float4*)s->instances.p, (const float4*)s->inst_wide.p,
+    e = prep::tight_bounds(n, (const float4*)s->instances.p, (float4*)s->inst_wide.p,
                            (const float*)s->inst_bounds.p, (const float4*)s->hulls.p, (float4*)s->wide_bounds.p, st);
   if (e == cudaSuccess)
     e = wide::collapse_tlas((const float4*)s->tlas_nodes.p, n_nodes, meta, (const uint32_t*)s->instance_indices.p,

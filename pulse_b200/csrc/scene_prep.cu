@@ -108,6 +108,30 @@ __global__ void k_instances(const InstanceIn* __restrict__ in, uint32_t n, const
   b[6] = center.x; b[7] = center.y; b[8] = center.z;
 }
 
+// Row i of an instance's matrices: what the rounding of a point's way into the object's space and
+// back, in units of 2^-24, multiplies the largest coordinate by (x), and adds to it (y); the
+// inverse's own error is in both.  x is at most 3 and the inverse's error at most 5 for rotations
+// and scales along the object's axes.
+__device__ __forceinline__ float2 way_back(const M4& m, const M4& w, int i, float& defect, float& offset) {
+  auto at = [](float4 c, int k) { return k == 0 ? c.x : k == 1 ? c.y : c.z; };
+  const float4 oc[3] = {m.c0, m.c1, m.c2};
+  const float4 wc[4] = {w.c0, w.c1, w.c2, w.c3};
+  const double by = 1.0 / w.c3.w;
+  float2 r = make_float2(0.0f, fabsf(at(m.c3, i)));
+  defect = offset = 0.0f;
+  for (int j = 0; j < 4; ++j) {
+    double sum = j == 3 ? (double)at(m.c3, i) : j == i ? -1.0 : 0.0;
+    float abs = 0.0f;
+    for (int k = 0; k < 3; ++k) {
+      sum += (double)at(oc[k], i) * at(wc[j], k) * by;
+      abs += fabsf(at(oc[k], i) * at(wc[j], k));
+    }
+    if (j < 3) r.x += abs, defect += (float)fabs(sum);
+    else r.y += abs, offset = (float)fabs(sum);
+  }
+  return r;
+}
+
 // One warp per instance, two hull boxes per lane.  A rotated mesh fills about half the
 // cross-section of the box around its root box's corners: the rays of the 1080p sphere
 // frame enter 4.5 instances instead of 6.9 (frame 11.9 -> 10.9 ms).
@@ -115,13 +139,12 @@ __global__ void k_instances(const InstanceIn* __restrict__ in, uint32_t n, const
 // times their amplification (the product of the matrix's and its inverse's largest
 // entries); where that exceeds 8 the reference's bounds stay.
 __global__ void __launch_bounds__(256) k_tight_bounds(uint32_t n, const float4* __restrict__ instances,
-                                                      const float4* __restrict__ inst_wide,
-                                                      const float* __restrict__ bounds9,
+                                                      float4* inst_wide, const float* __restrict__ bounds9,
                                                       const float4* __restrict__ hulls, float4* out) {
   const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
   if (i >= n) return;
   const M4 m = load_m4(instances + (size_t)i * 10), w = load_m4(instances + (size_t)i * 10 + 4);
-  const float4* h = hulls + (size_t)__float_as_uint(__ldg(inst_wide + (size_t)i * kWideInstRows + 4).w) * 128;
+  const float4* h = hulls + (size_t)__float_as_uint(inst_wide[(size_t)i * kWideInstRows + 4].w) * 128;
   float3 lo = v3(3e38f, 3e38f, 3e38f), hi = v3(-3e38f, -3e38f, -3e38f);
   for (uint32_t k = lane; k < 64u; k += 32u) {
     const float4 a = __ldg(h + 2 * k), z = __ldg(h + 2 * k + 1);
@@ -138,12 +161,33 @@ __global__ void __launch_bounds__(256) k_tight_bounds(uint32_t n, const float4* 
     hi = v3(fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, off)), fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, off)),
             fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, off)));
   }
-  if (lane != 0u) return;
-  // hits may lie before their box by the mesh's slack, its absolute part in world units along any direction
-  const float4 w0 = __ldg(inst_wide + (size_t)i * kWideInstRows), wx = __ldg(inst_wide + (size_t)i * kWideInstRows + 4);
-  const float stretch = sqrtf(dot(xyz(m.c0), xyz(m.c0)) + dot(xyz(m.c1), xyz(m.c1)) + dot(xyz(m.c2), xyz(m.c2)));
-  const float slack = fminf(fmaxf(wx.z, w0.w * stretch), kNoSlackBound);
+  // Distances of hits of a sheared instance are compared with those of others with its own
+  // margin (twice the error of the way back, of a distance and of a direction): per largest
+  // coordinate of the ray's origin (e1), and to add (e0).  Rotations and scales along the
+  // object's axes have the traversal's (wide_gate).
+  constexpr float kU = 5.9604645e-8f;
+  float defect, offset;
+  const float2 row = way_back(m, w, lane < 2u ? (int)lane : 2, defect, offset);
   const float* b = bounds9 + (size_t)i * 9;
+  float extent = 0.0f;
+  for (int k = 0; k < 6; ++k) extent = fmaxf(extent, fabsf(b[k]));
+  const bool own = row.x > 3.1f || defect > 8.0f * kU || offset > 6.0f * kU * row.y;
+  const float far = 3.5f * (defect + 20.0f * kU * row.x);
+  float e1 = 5.5f * defect + 86.0f * kU * row.x, e0 = 2.0f * offset + 20.0f * kU * row.y + far * extent;
+  if (!__any_sync(0xffffffffu, own)) e1 = e0 = 0.0f;
+  for (int off = 2; off > 0; off >>= 1) {
+    e1 = fmaxf(e1, __shfl_xor_sync(0xffffffffu, e1, off));
+    e0 = fmaxf(e0, __shfl_xor_sync(0xffffffffu, e0, off));
+  }
+  if (lane != 0u) return;
+  float4* rec = inst_wide + (size_t)i * kWideInstRows;
+  rec[1].w = e1;
+  rec[2].w = e0;
+  // hits may lie before their box by the mesh's slack, its absolute part in world units along any direction
+  const float stretch = sqrtf(dot(xyz(m.c0), xyz(m.c0)) + dot(xyz(m.c1), xyz(m.c1)) + dot(xyz(m.c2), xyz(m.c2)));
+  // and by the margin: within twice its extent of the middle an absolute one, farther out a relative
+  const float margin = fmaxf(4.0f * e1, 4.0f * (2.0f * extent * e1 + e0));
+  const float slack = fminf(fmaxf(fmaxf(rec[4].z, rec[0].w * stretch), margin), kNoSlackBound);
   float l[3] = {b[0], b[1], b[2]}, u[3] = {b[3], b[4], b[5]};
   auto entry = [](const M4& x) {
     return fmaxf(fmaxf(max_abs3(xyz(x.c0)), max_abs3(xyz(x.c1))), max_abs3(xyz(x.c2)));
@@ -221,7 +265,7 @@ cudaError_t instances(const InstanceIn* in, uint32_t n, const float4* blas_nodes
   return cudaGetLastError();
 }
 
-cudaError_t tight_bounds(uint32_t n, const float4* instances, const float4* inst_wide, const float* bounds9,
+cudaError_t tight_bounds(uint32_t n, const float4* instances, float4* inst_wide, const float* bounds9,
                          const float4* hulls, float4* out, cudaStream_t st) {
   if (!n) return cudaSuccess;
   k_tight_bounds<<<(n + 7) / 8, 256, 0, st>>>(n, instances, inst_wide, bounds9, hulls, out);

@@ -28,8 +28,9 @@ cudaError_t instances(const InstanceIn* in, uint32_t n, const float4* blas_nodes
 
 // Bounds (two float4) of each of the n instances for the wide traversal: around its
 // mesh's 64 hull boxes transformed, instead of the corners of its root box; and in the first's w
-// the instance's slack (pt_wide.cuh), relative and in world units.
-cudaError_t tight_bounds(uint32_t n, const float4* instances, const float4* inst_wide, const float* bounds9,
+// the instance's slack (pt_wide.cuh), relative and in world units.  Writes the distances' margins
+// of its transform into its record.
+cudaError_t tight_bounds(uint32_t n, const float4* instances, float4* inst_wide, const float* bounds9,
                          const float4* hulls, float4* out, cudaStream_t st);
 
 struct LightIn { uint32_t instance, triangle_offset, triangle_count, cdf_offset, material; };

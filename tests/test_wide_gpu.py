@@ -492,3 +492,34 @@ def test_rays_along_large_triangles_equal_the_oracle(ctx, size, scale, joined):
     assert np.array_equal(got["t"].view(np.uint32), ref["t"].view(np.uint32))
     for a, b in (("instance_index", "instance"), ("triangle_index", "triangle")):
         assert np.array_equal(got[a], ref[b])
+
+
+@pytest.mark.parametrize("far", [0.0, 1e3])
+@pytest.mark.parametrize("axis", [1.0, 0.1, 0.01, 0.001])
+def test_sheared_instances_that_coincide_equal_the_oracle(ctx, axis, far):
+    """Pairs of instances with the same surface and matrices some roundings apart, squeezed to
+    `axis` across their own axes: the distances' roundings grow with the shear."""
+    rng = np.random.default_rng(8)
+    mesh = scenes.displaced_icosphere(2, 0.1, 1, radius=1.0)
+    centre = far * np.array([1.0, 2.0, -3.0])
+    instances = []
+    for _ in range(8):
+        world = (scenes.trs(centre + rng.uniform(-2, 2, 3), scenes.random_rotation(rng))
+                 @ np.diag([1.0, axis, rng.uniform(axis, 1.0), 1.0]) @ scenes.trs((0, 0, 0), scenes.random_rotation(rng)))
+        other = world.copy()
+        other[:3] *= 1.0 + 3e-7 * rng.normal(size=(3, 4))
+        instances += [Instance(0, 0, world), Instance(0, 0, other)]
+    n = 150000
+    o = centre + rng.uniform(-3, 3, (n, 3))
+    d = centre + rng.uniform(-2, 2, (n, 3)) - o
+    rays = np.concatenate([o, d / np.linalg.norm(d, axis=1, keepdims=True)], 1).astype(np.float32)
+    ref = oracle.trace(oracle.assemble([mesh], MAT, instances, 20, 4, 2, 4), rays)
+    sc = Scene(ctx)
+    ids = [sc.upload_mesh(mesh, 20, 4)]
+    sc.set_materials(MAT)
+    sc.set_instances(instances, ids, 2, 4)
+    got = sc.trace(rays)
+    sc.close()
+    assert np.array_equal(got["t"].view(np.uint32), ref["t"].view(np.uint32))
+    for a, b in (("instance_index", "instance"), ("triangle_index", "triangle")):
+        assert np.array_equal(got[a], ref[b])
