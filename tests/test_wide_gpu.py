@@ -523,3 +523,29 @@ def test_sheared_instances_that_coincide_equal_the_oracle(ctx, axis, far):
     assert np.array_equal(got["t"].view(np.uint32), ref["t"].view(np.uint32))
     for a, b in (("instance_index", "instance"), ("triangle_index", "triangle")):
         assert np.array_equal(got[a], ref[b])
+
+
+@pytest.mark.parametrize("copies", [2, 3, 5])
+@pytest.mark.parametrize("leaf", [5, 8, 16])
+def test_surfaces_modelled_twice_equal_the_oracle(ctx, leaf, copies):
+    """Both sides of a surface as triangles of their own, and more copies: hits at the same
+    distance, or roundings apart, within one leaf and across the triangles of several steps."""
+    mesh = scenes.displaced_icosphere(2, 0.1, 4, radius=1.0)
+    one = np.asarray(mesh.indices).reshape(-1, 3)
+    turned = [one, one[:, ::-1], one[:, [1, 2, 0]], one, one[:, [2, 1, 0]]][:copies]
+    mesh.indices = np.concatenate(turned).reshape(-1).astype(np.uint32)
+    rng = np.random.default_rng(3)
+    instances = [Instance(0, 0, scenes.trs(rng.uniform(-2, 2, 3), scenes.random_rotation(rng))) for _ in range(6)]
+    rays = np.resize(_rays(3.0, np.zeros(3), 17), (30000, 6)).astype(np.float32)
+    rays[:, :3] += rng.uniform(-0.5, 0.5, (30000, 3)).astype(np.float32)
+    ref = oracle.trace(oracle.assemble([mesh], MAT, instances, 20, leaf, 2, 1), rays)
+    sc = Scene(ctx)
+    ids = [sc.upload_mesh(mesh, 20, leaf)]
+    sc.set_materials(MAT)
+    sc.set_instances(instances, ids, 2, 1)
+    got = sc.trace(rays)
+    sc.close()
+    for a, b in (("t", "t"), ("u", "u"), ("v", "v")):
+        assert np.array_equal(got[a].view(np.uint32), ref[b].view(np.uint32))
+    for a, b in (("instance_index", "instance"), ("triangle_index", "triangle")):
+        assert np.array_equal(got[a], ref[b])
