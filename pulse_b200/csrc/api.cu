@@ -108,13 +108,18 @@ void quiesce(PulseCtx* ctx) {
 
 }  // namespace
 
+constexpr size_t kHullBytes = wide::kHullBoxes * 32;
+
 struct MeshRec {
   uint32_t id = 0, ntris = 0, node_count = 0, levels = 1;
   bool alive = false;
   DevBuf prims, tdata, nodes, idx;
-  // The eight-wide tree (wide.cuh): nodes, leaf node of every slot, and what a
-  // collapse reported.
-  DevBuf wide, leaf_of, hull;
+  // The eight-wide tree (wide.cuh) in one allocation -- hull boxes, nodes, leaf node of every
+  // slot -- and what a collapse reported.
+  DevBuf wide;
+  float4* hull() const { return (float4*)wide.p; }
+  uint32_t* wide_nodes() const { return (uint32_t*)((char*)wide.p + kHullBytes); }
+  uint32_t* leaf_of() const { return wide_nodes() + (size_t)wide_count * pt::kWideNodeWords; }
   bool wide_ok = false;
   uint32_t wide_count = 0, wide_root = 0, wide_levels = 0;
   float wide_slack = 0.0f, wide_slack_abs = 0.0f;  // pt_wide.cuh
@@ -129,13 +134,19 @@ struct PulseScene {
       materials, strength_cdf, tri_cdfs, mesh_areas, light_indices;
   // Derived layouts.
   DevBuf inst_light, tri_bvh;
-  DevBuf wide_blas, leaf_of, hulls;               // of every mesh, concatenated
-  DevBuf wide_tlas, wide_thead, inst_wide;  // of the instances (pt_wide.cuh)
-  DevBuf wide_queue, wide_box, wide_bounds;       // scratch of the instance tree's collapse
-  bool wide_meshes = false;                       // wide_blas, leaf_of and hulls hold every live mesh's
-  bool wide_records = false;                      // inst_wide holds every instance's record
-  std::vector<uint32_t> mesh_wide;                // per mesh id: first wide node in wide_blas
-  uint64_t wide_nodes = 0;                        // rows of wide_blas
+  DevBuf wide_blas;                   // of every mesh: hull boxes (by mesh id), nodes, leaf nodes of the slots
+  DevBuf wide_tlas, inst_wide;        // of the instances (pt_wide.cuh); the tree's head words, then its nodes
+  DevBuf wide_tmp;                    // scratch of the instance tree's collapse
+  bool wide_meshes = false;           // wide_blas holds every live mesh's
+  bool wide_records = false;          // inst_wide holds every instance's record
+  std::vector<uint32_t> mesh_wide;    // per mesh id: first wide node in wide_blas
+  uint64_t wide_nodes = 0;            // nodes of wide_blas
+  float4* hulls() const { return (float4*)wide_blas.p; }
+  uint32_t* blas_wide() const { return (uint32_t*)((char*)wide_blas.p + mesh_wide.size() * kHullBytes); }
+  uint32_t* leaf_of() const { return blas_wide() + wide_nodes * pt::kWideNodeWords; }
+  static constexpr size_t kWideHeadBytes = 256;
+  uint32_t* wide_head() const { return (uint32_t*)wide_tlas.p; }
+  uint4* tlas_wide() const { return (uint4*)((char*)wide_tlas.p + kWideHeadBytes); }
   bool tri_bvh_current = false;  // tri_bvh gathered from the current primitives and triangle_indices
   pt::DevScene dev{};
   // Scene-preparation path.
@@ -172,7 +183,7 @@ struct PulseScene {
   // which then becomes the back set was queued before it.
   struct FrameSet {
     DevBuf tlas_nodes, instance_indices, instances, strength_cdf, tri_cdfs, mesh_areas, light_indices, inst_light,
-        inst_bounds, prep_ii, prep_lights, tlas_min, tlas_max, tlas_cent, tlas_meta, wide_tlas, wide_thead, inst_wide;
+        inst_bounds, prep_ii, prep_lights, tlas_min, tlas_max, tlas_cent, tlas_meta, wide_tlas, inst_wide;
     uint32_t* meta_host = nullptr;
     uint32_t* meta_mapped = nullptr;
   };
@@ -205,7 +216,6 @@ struct PulseScene {
     std::swap(tlas_cent, b.tlas_cent);
     std::swap(tlas_meta, b.tlas_meta);
     std::swap(wide_tlas, b.wide_tlas);
-    std::swap(wide_thead, b.wide_thead);
     std::swap(inst_wide, b.inst_wide);
     std::swap(meta_host, b.meta_host);
     std::swap(meta_mapped, b.meta_mapped);
@@ -214,7 +224,7 @@ struct PulseScene {
     FrameSet& b = back;
     for (DevBuf* x : {&b.tlas_nodes, &b.instance_indices, &b.instances, &b.strength_cdf, &b.tri_cdfs, &b.mesh_areas,
                       &b.light_indices, &b.inst_light, &b.inst_bounds, &b.prep_ii, &b.prep_lights, &b.tlas_min,
-                      &b.tlas_max, &b.tlas_cent, &b.tlas_meta, &b.wide_tlas, &b.wide_thead, &b.inst_wide})
+                      &b.tlas_max, &b.tlas_cent, &b.tlas_meta, &b.wide_tlas, &b.inst_wide})
       free_buf(*x);
     if (b.meta_host) cudaFreeHost(b.meta_host);
     b.meta_host = b.meta_mapped = nullptr;
@@ -229,8 +239,7 @@ struct PulseScene {
   }
   void free_all() {
     for (DevBuf* b : bind_group()) free_buf(*b);
-    for (DevBuf* b : {&inst_light, &tri_bvh, &wide_blas, &leaf_of, &hulls, &wide_tlas, &wide_thead, &inst_wide})
-      free_buf(*b);
+    for (DevBuf* b : {&inst_light, &tri_bvh, &wide_blas, &wide_tlas, &inst_wide}) free_buf(*b);
     dev.wide = 0u;
     wide_meshes = wide_records = false;
     tri_bvh_current = false;
@@ -243,7 +252,7 @@ struct PulseScene {
     meshes.clear();
   }
   static void free_mesh(MeshRec& m) {
-    for (DevBuf* x : {&m.prims, &m.tdata, &m.nodes, &m.idx, &m.wide, &m.leaf_of, &m.hull}) free_buf(*x);
+    for (DevBuf* x : {&m.prims, &m.tdata, &m.nodes, &m.idx, &m.wide}) free_buf(*x);
   }
   static void free_buf(DevBuf& b) {
     if (b.p) cudaFree(b.p);
@@ -684,7 +693,7 @@ int32_t pulse_scene_destroy(PulseScene* s) {
   s->free_meshes();
   s->bvh_scratch.release();
   for (DevBuf* x : {&s->tmp_a, &s->tmp_b, &s->tmp_c, &s->tmp_d, &s->prep_ii, &s->prep_lights, &s->prep_slot,
-                    &s->tlas_min, &s->tlas_max, &s->tlas_cent, &s->tlas_meta, &s->wide_queue, &s->wide_box, &s->wide_bounds})
+                    &s->tlas_min, &s->tlas_max, &s->tlas_cent, &s->tlas_meta, &s->wide_tmp})
     PulseScene::free_buf(*x);
   if (s->meta_host) cudaFreeHost(s->meta_host);
   if (s->upd_stream) cudaStreamDestroy(s->upd_stream);
@@ -695,7 +704,7 @@ int32_t pulse_scene_destroy(PulseScene* s) {
 }
 
 static void set_wide_tlas(PulseScene* s) {
-  s->dev.wide_tlas = (const uint4*)s->wide_tlas.p;
+  s->dev.wide_tlas = s->tlas_wide();
 }
 
 // Derived layouts (tri_bvh per distinct mesh range, instance -> light map) and
@@ -712,7 +721,7 @@ static cudaError_t finalize_scene(PulseScene* s, const std::vector<std::array<ui
     for (const auto& r : ranges) {  // {triangle_offset, index_offset, count}
       if (e != cudaSuccess) break;
       e = pt::launch_gather_tri_bvh((const float4*)s->primitives.p, (const uint32_t*)s->triangle_indices.p,
-                                    (const uint32_t*)s->leaf_of.p, (float4*)s->tri_bvh.p, r[0], r[1], r[2], st);
+                                    s->wide_meshes ? s->leaf_of() : nullptr, (float4*)s->tri_bvh.p, r[0], r[1], r[2], st);
     }
     if (e != cudaSuccess) return e;
     s->tri_bvh_current = true;
@@ -736,7 +745,7 @@ static cudaError_t finalize_scene(PulseScene* s, const std::vector<std::array<ui
   d.inst_light = (const int32_t*)s->inst_light.p;
   d.instance_count = c.instance_count;
   d.light_count = c.light_count;
-  d.wide_blas = (const uint4*)s->wide_blas.p;
+  d.wide_blas = (const uint4*)s->blas_wide();
   set_wide_tlas(s);
   d.inst_wide = (const float4*)s->inst_wide.p;
   return cudaSuccess;
@@ -910,17 +919,19 @@ static bool without_wide(cudaError_t e) {
 // whether it has one.
 static cudaError_t collapse_mesh(PulseCtx* ctx, MeshRec& m, cudaStream_t st) {
   const size_t cap = wide::capacity(m.node_count), out_bytes = cap * pt::kWideNodeWords * 4;
+  const size_t leaf_bytes = (size_t)m.ntris * 4;
   uint32_t h[wide::kHeadWords] = {};
   Work work(ctx);
-  cudaError_t e = ensure(m.leaf_of, (size_t)m.ntris * 4);
-  if (e == cudaSuccess) e = work.reserve(Work::piece(out_bytes) + Work::piece(cap * 4) + Work::piece(sizeof(h)));
+  cudaError_t e = work.reserve(Work::piece(out_bytes) + Work::piece(cap * 4) + Work::piece(leaf_bytes) +
+                               Work::piece(sizeof(h)));
   void* out = work.take(out_bytes);
   void* queue = work.take(cap * 4);
+  void* leaf_of = work.take(leaf_bytes);
   void* head = work.take(sizeof(h));
   if (e == cudaSuccess) e = cudaMemsetAsync(head, 0, sizeof(h), st);
   if (e == cudaSuccess)
-    e = wide::collapse((const float4*)m.nodes.p, m.node_count, (uint4*)out, (uint32_t*)m.leaf_of.p,
-                       (uint32_t*)queue, (uint32_t*)head, st);
+    e = wide::collapse((const float4*)m.nodes.p, m.node_count, (uint4*)out, (uint32_t*)leaf_of, (uint32_t*)queue,
+                       (uint32_t*)head, st);
   if (e == cudaSuccess) e = wide::extents((const float4*)m.prims.p, m.ntris, (uint32_t*)head, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(h, head, sizeof(h), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -933,16 +944,16 @@ static cudaError_t collapse_mesh(PulseCtx* ctx, MeshRec& m, cudaStream_t st) {
     if (!(m.wide_slack <= pt::kMostSlack)) m.wide_slack = pt::kNoSlackBound, m.wide_slack_abs = 0.0f;
     m.wide_slack = std::max(m.wide_slack, pt::kLeastSlack);
     const size_t bytes = (size_t)m.wide_count * pt::kWideNodeWords * 4;
-    e = ensure(m.wide, bytes);
-    if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(m.wide.p, out, bytes, cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = ensure(m.hull, wide::kHullBoxes * 32);
+    e = ensure(m.wide, kHullBytes + bytes + leaf_bytes);
+    if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(m.wide_nodes(), out, bytes, cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(m.leaf_of(), leaf_of, leaf_bytes, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess)
-      e = wide::hull((const uint4*)m.wide.p, m.wide_count, (const float4*)m.nodes.p, (float4*)m.hull.p, st);
+      e = wide::hull((const uint4*)m.wide_nodes(), m.wide_count, (const float4*)m.nodes.p, m.hull(), st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     m.wide_ok = e == cudaSuccess;
   }
   if (!m.wide_ok) {
-    for (DevBuf* x : {&m.wide, &m.leaf_of, &m.hull}) PulseScene::free_buf(*x);
+    PulseScene::free_buf(m.wide);
     m.wide_count = m.wide_root = m.wide_levels = 0u;
   }
   return without_wide(e) ? cudaSuccess : e;
@@ -1120,27 +1131,24 @@ int32_t pulse_materials_set(PulseScene* s, const PulseMaterial* mats, uint32_t n
 }
 
 // The meshes' eight-wide trees, if all of them have one and there is memory for their copy.
-static cudaError_t concat_wide(PulseScene* s, uint64_t nt, uint64_t nw, cudaStream_t st) {
-  const size_t node_bytes = pt::kWideNodeWords * 4, hull_bytes = wide::kHullBoxes * 32;
+static cudaError_t concat_wide(PulseScene* s, uint64_t nt, cudaStream_t st) {
   bool all = true;
   for (const MeshRec& m : s->meshes) all = all && (!m.alive || m.wide_ok);
   cudaError_t e = all ? cudaSuccess : cudaErrorMemoryAllocation;
-  if (e == cudaSuccess) e = ensure(s->wide_blas, nw * node_bytes);
-  if (e == cudaSuccess) e = ensure(s->leaf_of, nt * 4);
-  if (e == cudaSuccess) e = ensure(s->hulls, s->meshes.size() * hull_bytes);  // by mesh id
+  if (e == cudaSuccess)
+    e = ensure(s->wide_blas, s->meshes.size() * kHullBytes + s->wide_nodes * (pt::kWideNodeWords * 4) + nt * 4);
   for (const MeshRec& m : s->meshes) {
     if (!m.alive || e != cudaSuccess) continue;
-    const auto& t = s->mesh_table[m.id];
-    e = cudaMemcpyAsync((char*)s->leaf_of.p + (size_t)t[2] * 4, m.leaf_of.p, (size_t)m.ntris * 4, cudaMemcpyDeviceToDevice, st);
+    const uint32_t slot = s->mesh_table[m.id][2], node = s->mesh_wide[m.id];
+    e = cudaMemcpyAsync(s->leaf_of() + slot, m.leaf_of(), (size_t)m.ntris * 4, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess)
-      e = cudaMemcpyAsync((char*)s->hulls.p + m.id * hull_bytes, m.hull.p, hull_bytes, cudaMemcpyDeviceToDevice, st);
+      e = cudaMemcpyAsync((char*)s->hulls() + m.id * kHullBytes, m.hull(), kHullBytes, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess && m.wide_count)
-      e = wide::relocate((const uint32_t*)m.wide.p, m.wide_count, s->mesh_wide[m.id], t[2],
-                         (uint32_t*)s->wide_blas.p + (size_t)s->mesh_wide[m.id] * pt::kWideNodeWords, st);
+      e = wide::relocate(m.wide_nodes(), m.wide_count, node, slot,
+                         s->blas_wide() + (size_t)node * pt::kWideNodeWords, st);
   }
   s->wide_meshes = e == cudaSuccess;
-  if (!s->wide_meshes)
-    for (DevBuf* x : {&s->wide_blas, &s->leaf_of, &s->hulls}) PulseScene::free_buf(*x);
+  if (!s->wide_meshes) PulseScene::free_buf(s->wide_blas);
   return without_wide(e) ? cudaSuccess : e;
 }
 
@@ -1173,8 +1181,8 @@ static cudaError_t concat_meshes(PulseScene* s) {
     if (e == cudaSuccess) e = cudaMemcpyAsync((char*)s->triangle_indices.p + (size_t)t[2] * 4, m.idx.p, (size_t)m.ntris * 4, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync((char*)s->blas_nodes.p + (size_t)t[3] * 32, m.nodes.p, (size_t)m.node_count * 32, cudaMemcpyDeviceToDevice, st);
   }
-  if (e == cudaSuccess) e = concat_wide(s, nt, nw, st);
   s->wide_nodes = nw;
+  if (e == cudaSuccess) e = concat_wide(s, nt, st);
   s->counts.primitive_count = (uint32_t)nt;
   s->counts.triangle_index_count = (uint32_t)nt;
   s->counts.blas_node_count = (uint32_t)nn;
@@ -1200,18 +1208,18 @@ static cudaError_t collapse_tlas(PulseScene* s, uint32_t n, const uint32_t* meta
   if (!s->wide_meshes || !s->wide_records) return cudaSuccess;
   const uint32_t n_nodes = 2 * n - 1;
   const size_t cap = wide::capacity(n_nodes);
-  cudaError_t e = ensure(s->wide_tlas, cap * pt::kWideNodeWords * 4);
-  if (e == cudaSuccess) e = ensure(s->wide_thead, wide::kHeadWords * 4);
-  if (e == cudaSuccess) e = ensure(s->wide_queue, cap * 4);
-  if (e == cudaSuccess) e = ensure(s->wide_box, cap * 32);
-  if (e == cudaSuccess) e = ensure(s->wide_bounds, (size_t)n * 32);
+  const size_t box_bytes = cap * 32, bound_bytes = (size_t)n * 32;
+  cudaError_t e = ensure(s->wide_tlas, PulseScene::kWideHeadBytes + cap * pt::kWideNodeWords * 4);
+  if (e == cudaSuccess) e = ensure(s->wide_tmp, box_bytes + bound_bytes + cap * 4);
+  float4* box = (float4*)s->wide_tmp.p;
+  float4* bounds = (float4*)((char*)s->wide_tmp.p + box_bytes);
+  uint32_t* queue = (uint32_t*)((char*)bounds + bound_bytes);
   if (e == cudaSuccess)
-    e = prep::tight_bounds(n, (const float4*)s->instances.p, (float4*)s->inst_wide.p,
-                           (const float*)s->inst_bounds.p, (const float4*)s->hulls.p, (float4*)s->wide_bounds.p, st);
+    e = prep::tight_bounds(n, (const float4*)s->instances.p, (float4*)s->inst_wide.p, (const float*)s->inst_bounds.p,
+                           s->hulls(), bounds, st);
   if (e == cudaSuccess)
     e = wide::collapse_tlas((const float4*)s->tlas_nodes.p, n_nodes, meta, (const uint32_t*)s->instance_indices.p,
-                            (float4*)s->inst_wide.p, (const float4*)s->wide_bounds.p, (float4*)s->wide_box.p,
-                            (uint4*)s->wide_tlas.p, (uint32_t*)s->wide_queue.p, (uint32_t*)s->wide_thead.p, st);
+                            (float4*)s->inst_wide.p, bounds, box, s->tlas_wide(), queue, s->wide_head(), st);
   wt->made = e == cudaSuccess;
   if (wt->made) s->ctx->stats.kernel_launches += 2;
   return without_wide(e) ? cudaSuccess : e;
@@ -1261,7 +1269,7 @@ static int32_t rebuild_tlas(PulseScene* s, uint32_t n, const PulseBvhParams* tp,
     if (e == cudaSuccess) e = collapse_tlas(s, n, (const uint32_t*)s->tlas_meta.p, wt, st);
     if (e == cudaSuccess) {
       k_meta_to_host<<<1, 32, 0, st>>>((const uint32_t*)s->tlas_meta.p,
-                                       wt->made ? (const uint32_t*)s->wide_thead.p : nullptr, s->meta_mapped);
+                                       wt->made ? s->wide_head() : nullptr, s->meta_mapped);
       e = cudaGetLastError();
     }
     if (e != cudaSuccess) return cuda_err(ctx, e, "TLAS");
@@ -1282,7 +1290,7 @@ static int32_t rebuild_tlas(PulseScene* s, uint32_t n, const PulseBvhParams* tp,
   if (rc == PULSE_OK) {
     uint32_t h[wide::kHeadWords] = {};
     e = collapse_tlas(s, n, nullptr, wt, st);
-    if (e == cudaSuccess && wt->made) e = cudaMemcpyAsync(h, s->wide_thead.p, sizeof(h), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess && wt->made) e = cudaMemcpyAsync(h, s->wide_head(), sizeof(h), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) rc = cuda_err(ctx, e, "TLAS: eight-wide tree");
     wt->read(h);
