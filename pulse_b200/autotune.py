@@ -6,9 +6,10 @@ kernel family (1 megakernel, 2 wavefront), the megakernel's register budget
 (``min_blocks``), the wavefront/tail split (``wf_segments``), the persistent
 traversal grid (``trace_blocks`` per SM), the traversal block size
 (``block_size``: threads per block of the persistent traversal kernels), the
-warp step policy of the traversal (``step_policy``: which of the lanes'
+warp step policy of the binary traversal (``step_policy``: which of the lanes'
 pending actions -- node visit, triangle test, instance entry or exit -- a
-warp's step performs) and the ray-sort policy (``ray_sort``: whether each
+warp's step performs; any but the default keeps a prepared scene off the
+eight-wide trees) and the ray-sort policy (``ray_sort``: whether each
 bounce's queue is reordered by direction octant and origin cell before it is
 traced).
 
@@ -23,8 +24,8 @@ kept only if its frames dropped no push and hit no iteration cap.
 ``tune`` times one library render call per candidate with the context's own
 CUDA events (``last_render_ms``) and walks the knobs one at a time
 (coordinate descent from the defaults), so a tuning run costs about
-(candidates x (warmup + reps)) frames.  Results are keyed by device name and a
-workload signature and stored as JSON at ``path`` (default
+(candidates x (warmup + reps)) frames.  Results are keyed by device name, the
+kernels' generation and a workload signature and stored as JSON at ``path`` (default
 ``$PULSE_AUTOTUNE_CACHE`` or ``~/.cache/pulse_b200/autotune.json``).
 """
 from __future__ import annotations
@@ -33,6 +34,11 @@ import json
 import os
 import statistics
 from pathlib import Path
+
+# Part of the cache key: what was tuned for other kernels is tuned again.  A knob's best value
+# changes with them (a step_policy that paid with the binary trees keeps a scene off the
+# eight-wide ones: 1080p sphere frame 8.3 -> 13 ms).
+KERNELS = "wide8"
 
 TAIL_ONLY = 0xFFFFFFFF  # wf_segments value: no wavefront segments
 
@@ -43,13 +49,16 @@ def step_weights(node: int, tri: int, enter: int, leave: int) -> int:
 
 
 DEFAULT_SPACE = {
-    # wavefront segments before the persistent kernel; TAIL_ONLY: the
-    # persistent kernel runs every path (one traversal launch per frame)
-    "wf_segments": [1, 2, 3, 4, TAIL_ONLY],
-    "trace_blocks": [4, 5, 6, 8],
+    # wavefront segments before the persistent kernel (the library's own choice is 3 to 14, by
+    # the number of paths); TAIL_ONLY: the persistent kernel runs every path (one
+    # traversal launch per frame)
+    "wf_segments": [1, 2, 3, 4, 6, 9, 13, TAIL_ONLY],
+    # of the eight-wide traversal four are resident; more suit the binary trees
+    "trace_blocks": [3, 4, 5, 6, 8],
     # threads per traversal block: 0 = 128, or 64 (same threads per SM)
     "block_size": [0, 64],
-    # 0 = library default weights, 1 = divergent steps, then weight variants
+    # 0 = library default; the others select the binary trees, with divergent steps (1) or
+    # variants of their steps' weights
     "step_policy": [0, 1, step_weights(15, 30, 15, 20), step_weights(15, 25, 45, 45)],
     # reorder each bounce's queue by direction octant and origin cell
     "ray_sort": [0, 1],
@@ -132,7 +141,7 @@ def tune(ctx, call, base: dict, key: str, space: dict | None = None, warmup: int
     knobs; the timing table is stored beside them in the cache."""
     p = cache_path(path)
     data = _load(p)
-    full = f"{device_name()}|{key}"
+    full = f"{device_name()}|{KERNELS}|{key}"
     if not force and full in data:
         return dict(base, **data[full]["best"])
     space = DEFAULT_SPACE if space is None else space

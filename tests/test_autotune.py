@@ -86,3 +86,18 @@ def test_signature_buckets():
     b = autotune.signature("batched", 40_000_000, 15_000_000, 32, dict(nee_mode=2, max_depth=8))
     c = autotune.signature("batched", 40_000_000, 15_000_000, 31, dict(nee_mode=2, max_depth=8))
     assert a == b and a != c
+
+
+def test_results_of_other_kernels_are_tuned_again(tmp_path, monkeypatch):
+    """A result stored for another generation of the kernels is not returned, whether it was
+    stored with its generation or before there were any."""
+    ctx = FakeCtx()
+    path = tmp_path / "t.json"
+    stale = {"best": {"wf_segments": 1, "step_policy": 1}, "ms": 1.0, "table": []}
+    path.write_text(json.dumps({f"{autotune.device_name()}|k": stale}))
+    best = autotune.tune(ctx, ctx.render, {}, "k", path=path)
+    n = ctx.calls
+    assert n > 0 and best["wf_segments"] == 3 and best["step_policy"] == 0
+    monkeypatch.setattr(autotune, "KERNELS", "other")
+    autotune.tune(ctx, ctx.render, {}, "k", path=path)
+    assert ctx.calls > n
