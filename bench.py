@@ -1042,7 +1042,8 @@ def main():
                      "traffic": traffic, "peak_source": peak_kind,
                      "unit_of_work": "one frame: the wavefront's kernels share the path queues and the "
                                      "persistent tail kernel finishes what the segment kernels leave, so "
-                                     "algorithmic bytes (counted by the device) are defined per frame",
+                                     "algorithmic bytes (counted by the device: the reference's binary "
+                                     "trees; the eight-wide ones visit fewer nodes) are defined per frame",
                      "traffic_source": "profiles/wf_frame_spheres_1080p.md (ncu DRAM bytes of a 540p frame, "
                                        "scaled by paths)",
                      "bytes_per_path": b_path, "bytes_per_launch": bytes_per_launch,

@@ -103,9 +103,9 @@ constexpr uint32_t kWideStack = 36, kTopLeast = 12, kTopShallow = 16, kTopMost =
 // A warp keeps kPool rays in shared memory (word k of slot s at [k * kPool + s]), two
 // for each lane, and performs one action per step for up to 32 of those that wait
 // for it: with four classes of actions (node, triangles, instance, other) the
-// fullest one nearly always fills the warp, where one ray per lane in
-// registers left 11 to 15 lanes active per instruction (1080p sphere frame, first
-// extend; 21 with the pools).  Three rays a lane took 9.74 ms against 9.32 with two.
+// fullest one mostly fills the warp: 22 slots a step and 18 threads an instruction in the
+// first launches of the sphere frame, where one ray per lane in registers left 13 to
+// 14.  Three rays a lane took 9.74 ms against 9.32 with two.
 constexpr uint32_t kPool = 64;
 
 // An instance's record for entering it (DevScene::inst_wide), 96 bytes: its

@@ -3,11 +3,11 @@
 // step, one action for up to 32 of them.
 //
 // What bounded the binary kernels (wavefront.cu) here is issue with few lanes: one ray per
-// lane, 28 of 32 busy, of which 11 to 15 share an action; 66 node visits a ray.  With the wide
-// trees a ray takes 33 steps, 21 lanes an action: the 1080p sphere frame 13.9 -> 9.3 ms,
-// the 4K terrain frame 39 -> 24 ms, a million query rays 3.9 -> 1.55 ms.  What bounds these
-// kernels is still issue (57% of the slots; 380 instructions a node step), then the drain of
-// each launch: the longest ray takes 466 steps.
+// lane, 28 of 32 busy, of which 12 to 14 share an instruction.  With the wide trees a ray takes
+// 31 to 34 steps, of which 20 to 22 visit a node, 18 to 22 slots a step: the 1080p sphere
+// frame 13.5 -> 8.7 ms, the 4K terrain frame 42.0 -> 25.5 ms, a million query rays 4.1 -> 1.4
+// ms.  What bounds these kernels is still issue (55% of the slots with 16 warps an SM; 18
+// threads an instruction in the first launch, 8.5 in the last), then the drain of each launch.
 #include <atomic>
 
 #include "pt_wide.cuh"
