@@ -22,7 +22,9 @@ using namespace wf;
 
 // Blocks of four warps resident per SM.  1080p sphere frame, at the time: three 13.0 ms,
 // four 11.9; later four 9.3, five and six 10.5 (their registers spill, and the pools'
-// shared memory, about 50 KB a block, leaves less L1).
+// shared memory, about 50 KB a block, leaves less L1).  A launch with 64-thread blocks takes
+// the same kernels: an instance of each for it had doubled the module, whose load is part of a
+// process's first frame (24 -> 16 ms; frames with such blocks take the same time).
 constexpr int kWideBlocks = 4;
 
 // The scenes of a launch: one, in the kernel's parameters (ONE: reading its pointers from
@@ -96,8 +98,8 @@ __device__ __forceinline__ Scenes<ONE> block_scenes(const WfScene& one, const Wf
 }
 
 // n_table: scenes of the table (0 with ONE, then `one` is the scene).
-template <int SHADOW, bool ONE, int BS>
-__global__ void __launch_bounds__(BS, kWideBlocks * kWfBlock / BS)
+template <int SHADOW, bool ONE>
+__global__ void __launch_bounds__(kWfBlock, kWideBlocks)
     k_wide_extend(const __grid_constant__ TraceCfg tc, const __grid_constant__ WfBuffers B,
                   const __grid_constant__ WfScene one, uint32_t n_table, int qi, int sq, Counters* ctr) {
   extern __shared__ uint32_t smem[];
@@ -115,8 +117,8 @@ __global__ void __launch_bounds__(BS, kWideBlocks * kWfBlock / BS)
 }
 
 // The last segment's shadow requests.
-template <int MODE, bool ONE, int BS>
-__global__ void __launch_bounds__(BS, kWideBlocks * kWfBlock / BS)
+template <int MODE, bool ONE>
+__global__ void __launch_bounds__(kWfBlock, kWideBlocks)
     k_wide_shadow(const __grid_constant__ TraceCfg tc, const __grid_constant__ WfBuffers B,
                   const __grid_constant__ WfScene one, uint32_t n_table, int sq, Counters* ctr) {
   extern __shared__ uint32_t smem[];
@@ -181,8 +183,8 @@ struct TailItem {
   }
 };
 
-template <int MODE, bool ONE, int BS>
-__global__ void __launch_bounds__(BS, kWideBlocks * kWfBlock / BS)
+template <int MODE, bool ONE>
+__global__ void __launch_bounds__(kWfBlock, kWideBlocks)
     k_wide_tail(const __grid_constant__ TraceCfg tc, const __grid_constant__ WfBuffers B,
                 const __grid_constant__ WfScene one, uint32_t n_table, int qi, Counters* ctr) {
   extern __shared__ uint32_t smem[];
@@ -288,14 +290,10 @@ cudaError_t limit(K kernel) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
 }
 
-template <int BS>
-using Blk = std::integral_constant<int, BS>;
-
-// f(block size, one scene) with both as types.
+// f(whether the launch has one scene) with that as a type.
 template <typename F>
-void by_shape(uint32_t block, bool one, F f) {
-  if (block == 64) one ? f(Blk<64>{}, std::true_type{}) : f(Blk<64>{}, std::false_type{});
-  else one ? f(Blk<kWfBlock>{}, std::true_type{}) : f(Blk<kWfBlock>{}, std::false_type{});
+void by_scenes(bool one, F f) {
+  one ? f(std::true_type{}) : f(std::false_type{});
 }
 
 }  // namespace
@@ -305,16 +303,14 @@ cudaError_t wide_prepare(int mode) {
   auto raise = [&](auto kernel) {
     if (e == cudaSuccess) e = limit(kernel);
   };
-  for (uint32_t b : {64u, (uint32_t)kWfBlock})
-    for (bool one : {false, true})
-      by_shape(b, one, [&](auto bs, auto on) {
-        constexpr int BS = decltype(bs)::value;
-        constexpr bool ONE = decltype(on)::value;
-        raise(k_wide_extend<-1, ONE, BS>);
-        if (mode == 1) raise(k_wide_extend<1, ONE, BS>), raise(k_wide_shadow<1, ONE, BS>), raise(k_wide_tail<1, ONE, BS>);
-        if (mode == 2) raise(k_wide_extend<2, ONE, BS>), raise(k_wide_shadow<2, ONE, BS>), raise(k_wide_tail<2, ONE, BS>);
-        if (mode == 0) raise(k_wide_tail<0, ONE, BS>);
-      });
+  for (bool one : {false, true})
+    by_scenes(one, [&](auto on) {
+      constexpr bool ONE = decltype(on)::value;
+      raise(k_wide_extend<-1, ONE>);
+      if (mode == 1) raise(k_wide_extend<1, ONE>), raise(k_wide_shadow<1, ONE>), raise(k_wide_tail<1, ONE>);
+      if (mode == 2) raise(k_wide_extend<2, ONE>), raise(k_wide_shadow<2, ONE>), raise(k_wide_tail<2, ONE>);
+      if (mode == 0) raise(k_wide_tail<0, ONE>);
+    });
   if (mode == 2) raise(k_wide_adj_shadow);
   return e;
 }
@@ -322,12 +318,9 @@ cudaError_t wide_prepare(int mode) {
 void wide_extend(int shadow, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, int qi, int sq, Counters* ctr,
                  cudaStream_t st) {
   const Shape g = shape(tc, L);
-  by_shape(g.block, L.one != nullptr, [&](auto bs, auto on) {
-    constexpr int BS = decltype(bs)::value;
+  by_scenes(L.one != nullptr, [&](auto on) {
     constexpr bool ONE = decltype(on)::value;
-    const auto k = shadow == 1   ? k_wide_extend<1, ONE, BS>
-                   : shadow == 2 ? k_wide_extend<2, ONE, BS>
-                                 : k_wide_extend<-1, ONE, BS>;
+    const auto k = shadow == 1 ? k_wide_extend<1, ONE> : shadow == 2 ? k_wide_extend<2, ONE> : k_wide_extend<-1, ONE>;
     k<<<g.grid, g.block, g.smem, st>>>(tc, B, ONE ? *L.one : WfScene{}, ONE ? 0u : L.n_scenes, qi, sq, ctr);
   });
 }
@@ -335,10 +328,9 @@ void wide_extend(int shadow, const TraceCfg& tc, const WfBuffers& B, const WfLau
 void wide_shadow(int mode, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, int sq, Counters* ctr,
                  cudaStream_t st) {
   const Shape g = shape(tc, L);
-  by_shape(g.block, L.one != nullptr, [&](auto bs, auto on) {
-    constexpr int BS = decltype(bs)::value;
+  by_scenes(L.one != nullptr, [&](auto on) {
     constexpr bool ONE = decltype(on)::value;
-    const auto k = mode == 1 ? k_wide_shadow<1, ONE, BS> : k_wide_shadow<2, ONE, BS>;
+    const auto k = mode == 1 ? k_wide_shadow<1, ONE> : k_wide_shadow<2, ONE>;
     k<<<g.grid, g.block, g.smem, st>>>(tc, B, ONE ? *L.one : WfScene{}, ONE ? 0u : L.n_scenes, sq, ctr);
   });
 }
@@ -346,12 +338,9 @@ void wide_shadow(int mode, const TraceCfg& tc, const WfBuffers& B, const WfLaunc
 void wide_tail(int mode, const TraceCfg& tc, const WfBuffers& B, const WfLaunch& L, int qi, Counters* ctr,
                cudaStream_t st) {
   const Shape g = shape(tc, L);
-  by_shape(g.block, L.one != nullptr, [&](auto bs, auto on) {
-    constexpr int BS = decltype(bs)::value;
+  by_scenes(L.one != nullptr, [&](auto on) {
     constexpr bool ONE = decltype(on)::value;
-    const auto k = mode == 0   ? k_wide_tail<0, ONE, BS>
-                   : mode == 1 ? k_wide_tail<1, ONE, BS>
-                               : k_wide_tail<2, ONE, BS>;
+    const auto k = mode == 0 ? k_wide_tail<0, ONE> : mode == 1 ? k_wide_tail<1, ONE> : k_wide_tail<2, ONE>;
     k<<<g.grid, g.block, g.smem, st>>>(tc, B, ONE ? *L.one : WfScene{}, ONE ? 0u : L.n_scenes, qi, ctr);
   });
 }
