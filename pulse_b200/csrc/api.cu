@@ -123,6 +123,7 @@ struct MeshRec {
   bool wide_ok = false;
   uint32_t wide_count = 0, wide_root = 0, wide_levels = 0;
   float wide_slack = 0.0f, wide_slack_abs = 0.0f;  // pt_wide.cuh
+  float wide_leaves = 0.0f;  // without a slack: leaves that a line through the mesh meets on average
 };
 
 struct PulseScene {
@@ -949,7 +950,16 @@ static cudaError_t collapse_mesh(PulseCtx* ctx, MeshRec& m, cudaStream_t st) {
     if (e == cudaSuccess) e = cudaMemcpyAsync(m.leaf_of(), leaf_of, leaf_bytes, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess)
       e = wide::hull((const uint4*)m.wide_nodes(), m.wide_count, (const float4*)m.nodes.p, m.hull(), st);
+    const bool loose = m.wide_slack == pt::kNoSlackBound;
+    if (e == cudaSuccess && loose)
+      e = wide::leaf_area((const float4*)m.nodes.p, m.node_count, (uint32_t*)head, st);
+    if (e == cudaSuccess && loose) e = cudaMemcpyAsync(h, head, sizeof(h), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (loose) {
+      float area[2];
+      std::memcpy(area, &h[wide::kAreas], 8);
+      m.wide_leaves = area[1] > 0.0f ? area[0] / area[1] : 1.0f;  // (a box without area: one line)
+    }
     m.wide_ok = e == cudaSuccess;
   }
   if (!m.wide_ok) {
@@ -981,9 +991,13 @@ struct WideTree {
   bool ok = false;
   uint32_t levels = 0, count = 0;
   float slack = 0.0f;  // the largest of the loose instances
+  float pierced = 0.0f;  // leaves without a bound that a line through the scene meets on average
   void read(const uint32_t* head) {
     ok = made && !head[wide::kBad];
     std::memcpy(&slack, &head[wide::kSlack], 4);
+    float area[2];
+    std::memcpy(area, &head[wide::kAreas], 8);
+    pierced = area[1] > 0.0f ? area[0] / area[1] : 0.0f;
     levels = head[wide::kLevels];
     count = head[wide::kCount];
   }
@@ -992,7 +1006,16 @@ struct WideTree {
 // After the instances and their tree are in place: whether the scene's rays may
 // take the wide traversal.
 static void decide_wide(PulseScene* s, const std::vector<prep::InstanceIn>& ii, const WideTree& tree) {
-  bool ok = tree.ok && !ii.empty();
+  // Meshes of large triangles are not culled by distance (pt_wide.cuh), so a ray visits all of
+  // their leaves on its line, where the binary traversal stops at the first hits.  720p frames with
+  // wide / binary trees in ms, corrected estimator and the reference's, by such leaves a line: 1.6
+  // (40 spheres of 5,120 triangles, 240 units in radius) 1.50 / 2.12 and 1.27 / 1.40; 4.8 (300
+  // triangles in one mesh) 2.40 / 3.43 and 1.59 / 1.85; 5.0 (400 spheres of 1,280) 3.22 / 3.75 and
+  // 2.80 / 2.55; 6.9 (1,000 of 5,120) 5.14 / 5.31 and 4.48 / 3.59; 8.0 (4,000 triangles, sparse) 2.60 /
+  // 3.58 and 1.76 / 2.12; 12 (300 as instances) 5.67 / 6.94 and 4.28 / 4.36; 32 (4,000, dense) 12.9 /
+  // 9.6 and 10.9 / 6.0; 125 (as instances) 60 / 34 and 51 / 25.
+  constexpr float kMostPierced = 6.0f;
+  bool ok = tree.ok && !ii.empty() && tree.pierced <= kMostPierced;
   uint32_t levels = 0;
   for (const MeshRec& m : s->meshes)
     if (m.alive) {
@@ -1379,6 +1402,7 @@ int32_t pulse_instances_set(PulseScene* s, const PulseInstanceDesc* inst, uint32
     ii[i].wide_root = mesh.wide_root ? 0u : s->mesh_wide[d.mesh_id] | (1u << 24);
     ii[i].wide_slack = mesh.wide_slack;
     ii[i].wide_slack_abs = mesh.wide_slack_abs;
+    ii[i].wide_leaves = mesh.wide_leaves;
     ii[i].hull = d.mesh_id;
     ii[i].wide_leaf = mesh.wide_root ? mesh.wide_root + t[2] : 0u;
     const float* em = s->host_materials[d.material_index].emissive;

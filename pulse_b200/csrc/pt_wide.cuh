@@ -37,8 +37,9 @@
 //     the distance.  triangle_slack (wide.cu) bounds it by (t + longer edge) * slack; meshes
 //     whose triangles have no such bound are not culled by distance at all.  (A slack of at most
 //     0.02 answered 1 in 10,000 rays along triangles of 20 to 200 units wrongly.  Without it
-//     720p frames of a terrain of 400 units in 8 to 96 squares a side take 0 to 8% longer
-//     than with it, 17% at worst; the binary trees take 1.2 to 1.6 times as long.)  Left out is a hit
+//     720p frames of a terrain of 400 units in 8 to 96 squares a side take 0 to 5% longer
+//     than with it, 16% at worst; the binary trees take 1.2 to 1.6 times as long.  Scenes
+//     of many such triangles keep the binary trees: decide_wide, api.cu.)  Left out is a hit
 //     whose ray passes beside the triangle by a rounding and enters its box later by that
 //     over the direction's component, if that is below 0.01.
 // Rays and scenes outside these arguments (a direction that is not
@@ -110,8 +111,9 @@ constexpr uint32_t kPool = 64;
 
 // An instance's record for entering it (DevScene::inst_wide), 96 bytes: its
 // world-to-object matrix (affine: the first three columns' w hold the mesh's slack in units of
-// its space and the margins e1, e0 of its distances, 0 unless it is sheared), (root group of the mesh's tree, or 0 and its only leaf's reference, slack of the
-// mesh, mesh id), (first triangle slot, first binary node, TLAS leaf node or kWideRootLeaf, 0).
+// its space and the margins e1, e0 of its distances, 0 unless it is sheared), (root group of the
+// mesh's tree, or 0 and its only leaf's reference, slack of the mesh, mesh id), (first triangle
+// slot, first binary node, TLAS leaf node or kWideRootLeaf, scene_prep.cuh's wide_leaves).
 constexpr uint32_t kWideInstRows = 6;
 
 enum WideWord : uint32_t {
@@ -398,16 +400,23 @@ __device__ __forceinline__ uint32_t wide_node(const WideRay& R, const DevScene& 
     }
     const uint4 ra = __ldg(np + 1), rb = __ldg(np + 5);  // references of the leaves
     const uint32_t ref[8] = {ra.x, rb.w, rb.z, rb.y, rb.x, ra.w, ra.z, ra.y};
-    const uint32_t child = w.child & kWideIndexMask, loose = w.child >> kTopLooseShift;
+    const uint32_t child = w.child & kWideIndexMask;
+    uint32_t loose = 0;
+    if (slack > kLeastSlack) {
+      loose = ih & (w.child >> kTopLooseShift);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) loose |= lh & ((ref[k] >> 31) << k);
+    }
     const float less = __fdividef(1.0f, 1.0f + slack);
     float best = 3.4e38f;
     uint32_t best_e = 0, best_at = sp, e = 0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const bool inner = (uint32_t)k < w.ni;
-      if (inner ? (loose >> k) & 1u : ref[k] >> 31) tn[k] = fmaxf((tn[k] - slack) * less, 0.0f);
-      if ((hit & (1u << k)) && tn[k] <= bound) {
-        e = ((__float_as_uint(tn[k]) >> 17) << 18) | (inner ? (child + (uint32_t)k) << 1 : (ref[k] << 1) | 1u);
+      float at_least = tn[k];
+      if (loose & (1u << k)) at_least = fmaxf((at_least - slack) * less, 0.0f);
+      if ((hit & (1u << k)) && at_least <= bound) {
+        e = ((__float_as_uint(at_least) >> 17) << 18) | (inner ? (child + (uint32_t)k) << 1 : (ref[k] << 1) | 1u);
         if (tn[k] < best) { best = tn[k]; best_e = e; best_at = sp; }
         R.stack(sp++) = e;
       }

@@ -89,7 +89,7 @@ __global__ void k_instances(const InstanceIn* __restrict__ in, uint32_t n, const
     wo[0].w = x.wide_slack_abs;
     wo[4] = make_float4(__uint_as_float(x.wide_root), __uint_as_float(x.wide_leaf), x.wide_slack, __uint_as_float(x.hull));
     wo[5] = make_float4(__uint_as_float(x.index_offset), __uint_as_float(x.node_offset),
-                        __uint_as_float(kWideRootLeaf), 0.0f);
+                        __uint_as_float(kWideRootLeaf), x.wide_leaves);
   }
   // World bounds of the root box (src/scene/mod.rs:625-658).
   const float4 lo = blas_nodes[2 * (size_t)x.node_offset], hi = blas_nodes[2 * (size_t)x.node_offset + 1];
@@ -202,7 +202,8 @@ __global__ void __launch_bounds__(256) k_tight_bounds(uint32_t n, const float4* 
     }
   }
   out[2 * (size_t)i] = make_float4(l[0], l[1], l[2], slack);
-  out[2 * (size_t)i + 1] = make_float4(u[0], u[1], u[2], 0.0f);
+  const float ex = u[0] - l[0], ey = u[1] - l[1], ez = u[2] - l[2];
+  out[2 * (size_t)i + 1] = make_float4(u[0], u[1], u[2], rec[5].w * (ex * ey + ey * ez + ez * ex));
 }
 
 __global__ void k_light_cdfs(const LightIn* __restrict__ lights, uint32_t n, const float4* __restrict__ prims,

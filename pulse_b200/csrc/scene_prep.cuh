@@ -15,7 +15,9 @@ struct InstanceIn {
   uint32_t triangle_offset, triangle_count, index_offset, node_offset, material_index;
   uint32_t wide_root, wide_leaf;  // root group of the mesh's eight-wide tree, or 0 and its only leaf
   float wide_slack, wide_slack_abs;
-  uint32_t hull, pad[2];  // the mesh's boxes for tight_bounds
+  uint32_t hull;            // the mesh's boxes for tight_bounds
+  float wide_leaves;        // of a mesh without a slack: leaves that a line through it meets
+  uint32_t pad;
 };
 
 // prepare_mesh_instances (src/scene/mod.rs:561-681) per instance: the 160 B
@@ -28,7 +30,8 @@ cudaError_t instances(const InstanceIn* in, uint32_t n, const float4* blas_nodes
 
 // Bounds (two float4) of each of the n instances for the wide traversal: around its
 // mesh's 64 hull boxes transformed, instead of the corners of its root box; and in the first's w
-// the instance's slack (pt_wide.cuh), relative and in world units.  Writes the distances' margins
+// the instance's slack (pt_wide.cuh), relative and in world units, in the second's the area of its bounds
+// times its mesh's wide_leaves.  Writes the distances' margins
 // of its transform into its record.
 cudaError_t tight_bounds(uint32_t n, const float4* instances, float4* inst_wide, const float* bounds9,
                          const float4* hulls, float4* out, cudaStream_t st);

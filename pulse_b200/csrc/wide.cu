@@ -41,6 +41,8 @@ struct LeafSink {
     const float slack = bounds[2 * (size_t)i].w;
     if (slack <= pt::kLeastSlack) return i;
     atomicMax(head + kSlack, __float_as_uint(slack));
+    const float area = bounds[2 * (size_t)i + 1].w;
+    if (area > 0.0f) atomicAdd(reinterpret_cast<float*>(head + kAreas), area);
     return i | pt::kLooseRef;
   }
 };
@@ -229,6 +231,7 @@ __device__ void fit_node(uint32_t i, uint32_t* out, const LeafSink& leaf_of, uin
   if (ni) w[4] |= (loose & ((1u << ni) - 1u)) << pt::kTopLooseShift;
   leaf_of.node_box[2 * (size_t)i] = make_float4(lo[0], lo[1], lo[2], loose ? 1.0f : 0.0f);
   leaf_of.node_box[2 * (size_t)i + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+  if (i == 0) head[kRootArea] = __float_as_uint(half_area(leaf_of.node_box[0], leaf_of.node_box[1]));
   quantize(w, box, used, head);
 }
 
@@ -257,7 +260,7 @@ __global__ void __launch_bounds__(kBlock) k_collapse(const float4* __restrict__ 
     const uint32_t start = __float_as_uint(rlo.w);
     const bool tlas = leaf_of.instance_of != nullptr;
     head[kBad] = 0u;
-    if (tlas) head[kSlack] = 0u;
+    if (tlas) head[kSlack] = head[kAreas] = 0u;
     head[kLevels] = count && tlas ? 1u : 0u;
     head[kRoot] = count && !tlas ? leaf_ref(start, count, head) : 0u;
     queue[0] = 0u;
@@ -373,6 +376,17 @@ __device__ __forceinline__ float triangle_slack(float3 e1, float3 e2, float l1, 
   return kU * k;
 }
 
+__global__ void __launch_bounds__(kBlock) k_leaf_area(const float4* __restrict__ nodes, uint32_t n, uint32_t* head) {
+  float area = 0.0f;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const float4 lo = nodes[2 * (size_t)i], hi = nodes[2 * (size_t)i + 1];
+    if (__float_as_uint(hi.w)) area += half_area(lo, hi);
+    if (i == 0u) head[kRootArea] = __float_as_uint(half_area(lo, hi));
+  }
+  for (int off = 16; off > 0; off >>= 1) area += __shfl_xor_sync(0xffffffffu, area, off);
+  if ((threadIdx.x & 31) == 0) atomicAdd(reinterpret_cast<float*>(head + kAreas), area);
+}
+
 __global__ void __launch_bounds__(kBlock) k_extents(const float4* __restrict__ prims, uint32_t n, uint32_t* head) {
   float rel = 0.0f, abs = 0.0f;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -432,6 +446,13 @@ cudaError_t relocate(const uint32_t* nodes, uint32_t n, uint32_t node_add, uint3
                      cudaStream_t st) {
   if (!n) return cudaSuccess;
   k_relocate<<<(n + kBlock - 1) / kBlock, kBlock, 0, st>>>(nodes, n, node_add, slot_add, out);
+  return cudaGetLastError();
+}
+
+cudaError_t leaf_area(const float4* nodes, uint32_t n_nodes, uint32_t* head, cudaStream_t st) {
+  if (!n_nodes) return cudaSuccess;
+  const uint32_t blocks = (n_nodes + kBlock - 1) / kBlock;
+  k_leaf_area<<<blocks < 1184u ? blocks : 1184u, kBlock, 0, st>>>(nodes, n_nodes, head);
   return cudaGetLastError();
 }
 

@@ -15,6 +15,9 @@ enum Head : uint32_t {
   // distance, and in units of the space.  A mesh's two (extents), or in the first the largest
   // of both of a TLAS's loose instances.
   kSlack, kSlackAbs,
+  // Areas (floats): a mesh's leaf boxes (leaf_area), or a TLAS's instances without a bound times
+  // their meshes' leaves; the root box.
+  kAreas, kRootArea,
   kHeadWords = 8
 };
 
@@ -29,7 +32,7 @@ cudaError_t collapse(const float4* nodes, uint32_t n_nodes, uint4* out, uint32_t
 
 // The same for an instance tree, whose elements' leaf nodes go into the instances'
 // records (pt_wide.cuh) and whose boxes are those of the instances' own bounds (two float4
-// each, the first's w the instance's slack; node_box: scratch of two float4 per node).  meta: the words of a
+// each, the first's w the instance's slack, the second's its share of kAreas; node_box: scratch of two float4 per node).  meta: the words of a
 // bvh::build_direct queued before (kBad and nothing read if it failed), or nullptr.
 cudaError_t collapse_tlas(const float4* nodes, uint32_t n_nodes, const uint32_t* meta, const uint32_t* instance_of,
                           float4* records, const float4* bounds, float4* node_box, uint4* out, uint32_t* queue,
@@ -44,6 +47,10 @@ cudaError_t hull(const uint4* wide_nodes, uint32_t n_wide, const float4* nodes, 
 // slot_add, as they go into the scene's array.
 cudaError_t relocate(const uint32_t* nodes, uint32_t n, uint32_t node_add, uint32_t slot_add, uint32_t* out,
                      cudaStream_t st);
+
+// Adds the areas of the leaf boxes of a tree of n_nodes nodes to head's kAreas, and its root's to
+// kRootArea (zero to begin with).
+cudaError_t leaf_area(const float4* nodes, uint32_t n_nodes, uint32_t* head, cudaStream_t st);
 
 // Raises head's kSlack and kSlackAbs (zero to begin with) to those of n std430 triangles.
 cudaError_t extents(const float4* prims, uint32_t n, uint32_t* head, cudaStream_t st);

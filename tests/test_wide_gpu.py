@@ -549,3 +549,29 @@ def test_surfaces_modelled_twice_equal_the_oracle(ctx, leaf, copies):
         assert np.array_equal(got[a].view(np.uint32), ref[b].view(np.uint32))
     for a, b in (("instance_index", "instance"), ("triangle_index", "triangle")):
         assert np.array_equal(got[a], ref[b])
+
+
+@pytest.mark.parametrize("count", [1, 24, 60])  # loose leaves a line: below the rule's limit, about it, and above
+def test_many_large_triangles_equal_the_oracle(ctx, count):
+    """Instances of a mesh of large triangles, few enough for the wide trees and too many, beside
+    small ones: the rule's routes, through two frames of instances that change between them."""
+    rng = np.random.default_rng(24)
+    big = scenes.displaced_icosphere(2, 0.1, 3, radius=150.0)
+    small = scenes.displaced_icosphere(2, 0.1, 5, radius=8.0)
+    insts = [Instance(0, 0, scenes.trs(rng.uniform(-200, 200, 3), scenes.random_rotation(rng))) for _ in range(count)]
+    insts += [Instance(1, 0, scenes.trs(rng.uniform(-400, 400, 3), scenes.random_rotation(rng))) for _ in range(20)]
+    n = 20000
+    o = rng.uniform(-500, 500, (n, 3))
+    d = rng.uniform(-300, 300, (n, 3)) - o
+    rays = np.concatenate([o, d / np.linalg.norm(d, axis=1, keepdims=True)], 1).astype(np.float32)
+    sc = Scene(ctx)
+    ids = [sc.upload_mesh(m, 20, 8) for m in (big, small)]
+    sc.set_materials(MAT)
+    for now in (insts, insts[count // 2:], insts):
+        sc.set_instances(now, ids)
+        got = sc.trace(rays)
+        ref = oracle.trace(oracle.assemble([big, small], MAT, now, 20, 8), rays)
+        assert np.array_equal(got["t"].view(np.uint32), ref["t"].view(np.uint32))
+        for a, b in (("instance_index", "instance"), ("triangle_index", "triangle")):
+            assert np.array_equal(got[a], ref[b])
+    sc.close()
