@@ -4,7 +4,9 @@
 // node arrays); wide.cu collapses each into nodes of up to eight children with
 // their boxes quantized to 8 bits per plane, rounded outwards (96 bytes against
 // the 448 of the seven binary interior nodes it stands for).  A ray visits
-// about a third of the nodes, each with one set of independent loads.
+// about a third of the nodes, each with one set of independent loads.  (Wide nodes with
+// quantized boxes on a power-of-two grid: Ylitie, Karras and Laine, "Efficient Incoherent Ray
+// Traversal on GPUs Through Compressed Wide BVHs", 2017.)
 //
 // The result is the reference's bit for bit although nodes are visited in
 // another order.  Within one BLAS (o, d object space, t local; the TLAS level
@@ -89,8 +91,9 @@ constexpr uint32_t kLooseRef = 0x80000000u;
 constexpr float kLeastSlack = 1e-4f;
 // Node word 4 of the TLAS from this bit: the interior children that hold a loose instance.
 constexpr uint32_t kTopLooseShift = 24;
-// A slack that culls nothing, and up to which one bounds a hit (wide.cu).
-constexpr float kNoSlackBound = 1e9f, kMostSlack = 0.5f;
+// A slack that culls nothing (boxes lie within 4e9 of a ray's origin), and up to which one bounds
+// a hit (wide.cu).
+constexpr float kNoSlackBound = 1e15f, kMostSlack = 0.5f;
 // Entries up to which children are pushed: 16 for trees of up to 3 levels (the 1080p
 // sphere frame: 9.3 ms, with 24 and the less L1 they leave 9.45), 24 for deeper ones as far as
 // the stack of both levels stays within 36 words, the most with which four blocks fit an SM
