@@ -562,6 +562,12 @@ __device__ __forceinline__ float wide_object_ray(const M4& w2o, float3 wo, float
   return len;
 }
 
+// The margin of distances (wide_gate) that an instance with the given record and object ray adds to
+// that of the ray's origin.
+__device__ __forceinline__ float wide_margin(const M4& w2o, float3 wo, float3 o, float len) {
+  return fmaxf(__fdividef(1.6e-6f * max_abs3(o), len), w2o.c1.w * max_abs3(wo) + w2o.c2.w);
+}
+
 // Leave the BLAS, if in one, and enter the next instance, if one is next.
 __device__ __forceinline__ uint32_t wide_instance(const WideRay& R, const DevScene& S, float3 wo, float3 wd) {
   uint32_t sp = R.u(kwSp);
@@ -583,8 +589,7 @@ __device__ __forceinline__ uint32_t wide_instance(const WideRay& R, const DevSce
   R.setf3(kwOX, o);
   R.setf3(kwDX, d);
   R.setf(kwLen, len);
-  R.setf(kwEps, fmaxf(fmaxf(R.f(kwEps), __fdividef(1.6e-6f * max_abs3(o), len)),
-                      w2o.c1.w * max_abs3(wo) + w2o.c2.w));
+  R.setf(kwEps, fmaxf(R.f(kwEps), wide_margin(w2o, wo, o, len)));
   const float slack = fmaxf(wx.z, __fdividef(w2o.c0.w, len));
   R.setf(kwSlack, slack);
   R.setf(kwCull, (fminf(wide_bound(rec_t, slack), far) + 1e-3f * (1.0f + max_abs3(wo))) * len);
@@ -634,8 +639,11 @@ __device__ __forceinline__ uint32_t wide_verify(const WideRay& R, const DevScene
   const float4* tp = S.tri_bvh + (size_t)slot * 3;
   const float4 t0 = __ldg(tp), t1 = __ldg(tp + 1), t2 = __ldg(tp + 2);
   float3 o, d;
-  const float len = wide_object_ray(load_m4(ip), wo, wd, o, d);
-  const float gate = wide_gate(rec_t, R.f(kwEps)) * 0.999999f;
+  const M4 w2o = load_m4(ip);
+  const float len = wide_object_ray(w2o, wo, wd, o, d);
+  // (the hit's own margin: kwEps may have grown since hits were looked for up to the gate, and a
+  // box entered between the two gates can have let one beyond the first win)
+  const float gate = wide_gate(rec_t, fmaxf(1e-6f * max_abs3(wo), wide_margin(w2o, wo, o, len))) * 0.999999f;
   const float by = decided ? (2.0f * R.f(kwLimit) - R.f(kwFar)) * 0.999999f : gate;
   float t = 0.0f;
   h.u = h.v = 0.0f;

@@ -575,3 +575,37 @@ def test_many_large_triangles_equal_the_oracle(ctx, count):
         for a, b in (("instance_index", "instance"), ("triangle_index", "triangle")):
             assert np.array_equal(got[a], ref[b])
     sc.close()
+
+
+@pytest.mark.parametrize("leaf", [4, 8])
+@pytest.mark.parametrize("turned", [False, True])
+def test_margins_grow_after_the_hit(ctx, turned, leaf):
+    """Rays onto the edges of a cube, almost along them: a face met by a rounding before the box
+    that holds it, the next face's hit within that distance.  Behind the cube's own faces lie the bounds
+    of an instance with far larger coordinates, entered after the hit: its margins are not the hit's."""
+    rng = np.random.default_rng(25)
+    corner = np.array([[0, 0, 0], [0.1, 0, 0], [0, 0.1, 0]])
+    p = np.concatenate([corner - 0.49999, 4.9 - corner]) + 1000.0  # two triangles, little in their box
+    sparse = Mesh(p, np.tile([0.0, 1.0, 0.0], (6, 1)), np.zeros((6, 2)), np.arange(6, dtype=np.uint32))
+    world = scenes.trs((0.1, 0.2, 0.3), scenes.random_rotation(rng)) if turned else np.eye(4)
+    instances = [Instance(0, 0, world), Instance(1, 0, world @ scenes.trs((-1000, -1000, -1000)))]
+    n = 60000
+    axis = rng.integers(0, 3, n)
+    rows = np.arange(n)
+    target = np.full((n, 3), -0.5)
+    target[rows, axis] = rng.uniform(-0.5, 0.5, n)
+    d = np.exp(rng.uniform(np.log(1e-3), np.log(0.3), (n, 3)))
+    d[rows, axis] = rng.choice([-1.0, 1.0], n)
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    o = target - d * np.exp(rng.uniform(np.log(2e-3), np.log(1.0), n))[:, None]
+    o, d = o @ world[:3, :3].T + world[:3, 3], d @ world[:3, :3].T
+    rays = np.concatenate([o, d], 1).astype(np.float32)
+    meshes = [scenes.unit_cube(), sparse]
+    ref = oracle.trace(oracle.assemble(meshes, MAT, instances, 20, leaf), rays)
+    sc = _prepare(ctx, meshes, MAT, instances, leaf)
+    got = sc.trace(rays)
+    sc.close()
+    assert (ref["t"] < 1e29).sum() > n // 4
+    assert np.array_equal(got["t"].view(np.uint32), ref["t"].view(np.uint32))
+    for a, b in (("instance_index", "instance"), ("triangle_index", "triangle")):
+        assert np.array_equal(got[a], ref[b])
