@@ -5,9 +5,9 @@
 // What bounded the binary kernels (wavefront.cu) here is issue with few lanes: one ray per
 // lane, 28 of 32 busy, of which 12 to 14 share an instruction.  With the wide trees a ray takes
 // 31 to 34 steps, of which 20 to 22 visit a node, 18 to 22 slots a step: the 1080p sphere
-// frame 13.5 -> 8.7 ms, the 4K terrain frame 42.0 -> 25.5 ms, a million query rays 4.1 -> 1.4
-// ms.  What bounds these kernels is still issue (55% of the slots with 16 warps an SM; 18
-// threads an instruction in the first launch, 8.5 in the last), then the drain of each launch.
+// frame 13.8 -> 8.8 ms, the 4K terrain frame 40.0 -> 24.7 ms, a million query rays 4.1 -> 1.5
+// ms.  What bounds these kernels is still issue (54% of the slots with 16 warps an SM; 18
+// threads an instruction in the first launch, 8.4 in the last), then the drain of each launch.
 #include <atomic>
 
 #include "pt_wide.cuh"
