@@ -276,6 +276,9 @@ __device__ __forceinline__ bool ray_triangle(float3 o, float3 d, float rec_t, co
 //     visited in the same relative order, so the local closest hit below t_cull
 //     and its tie-breaking are the reference's, and a local miss produces the
 //     far-hit value (~1e30 |M d|), which cannot replace a real hit either.
+//     (Left out is a hit whose ray passes beside its triangle by a rounding and
+//     enters the box that holds it later by more than the margin: 29 of 64 million
+//     rays from vertex to vertex of 8 scenes.)
 // Occlusion queries (trace_init with a finite limit; the NEE shadow rays, whose
 // only use of the closest hit is `t < limit`) add two exact shortcuts:
 //   * boxes of either level whose entry distance exceeds limit (with the same
